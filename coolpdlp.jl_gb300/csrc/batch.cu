@@ -33,6 +33,7 @@
 
 #include "batch.cuh"
 #include "epilogues.cuh"
+#include "resident.cuh"
 #include "solver.cuh"
 
 namespace cpdlp {
@@ -317,6 +318,73 @@ __device__ __forceinline__ void lp_kkt(const BatchArgs<T>& g, const BatchCtl& C,
     Grp<CS>::sync();  // the long-row terms are rewritten by the next pass
 }
 
+// Thread 0, after a block: counts its passes, takes the termination decision
+// (common.jl:218-231) and the restart candidates (pdlp.jl:138-170) from the
+// errors C.e; sets C.status and C.stop and returns the restart flag: 0 none,
+// 2 the restart point's errors are needed first, 3 restart.
+__device__ __forceinline__ int batch_decide(const BatchParams& prm, BatchCtl& C, bool pdlp) {
+    C.passes += prm.check_every;
+    if (pdlp) {
+        C.inner += prm.check_every;
+        C.total += prm.check_every;
+    }
+    C.e_sol = C.e[0];
+    int32_t stt = CPDLP_STILL_RUNNING;
+    const double rel = rel_err(C.e_sol);
+    if (rel <= C.L.reltol) stt = CPDLP_OPTIMAL;
+    else if (C.tl_hit) stt = CPDLP_TIME_LIMIT;
+    else if (C.passes >= C.L.max_passes) stt = CPDLP_ITERATION_LIMIT;
+    // stall: the relative error has not halved over stall_passes passes
+    if (rel < 0.5 * C.best_rel) {
+        C.best_rel = rel;
+        C.mark = C.passes;
+    } else if (stt == CPDLP_STILL_RUNNING && C.L.stall_passes > 0 &&
+               C.passes - C.mark >= C.L.stall_passes) {
+        stt = CPDLP_ITERATION_LIMIT;
+        C.stalled = 1;
+    }
+    int flag = 0;
+    if (stt == CPDLP_STILL_RUNNING && !C.cancelled && pdlp) {
+        const double w = C.omega;
+        if (abs_err(C.e[0], w) < abs_err(C.e[1], w)) { C.from_avg = 0; C.e_cand = C.e[0]; }
+        else { C.from_avg = 1; C.e_cand = C.e[1]; }
+        C.e[2] = (abs_err(C.e[2], w) < abs_err(C.e[3], w)) ? C.e[2] : C.e[3];
+        flag = 2;  // the restart point's errors are needed first
+        if (C.restart_valid)
+            flag = should_restart(prm, abs_err(C.e_cand, w), abs_err(C.e_restart, w),
+                                  abs_err(C.e[2], w), C.inner, C.total) ? 3 : 0;
+    }
+    C.status = stt;
+    C.stop = (stt != CPDLP_STILL_RUNNING) || C.cancelled;
+    return flag;
+}
+
+// One thread of the group, after its solution is written: the LP's result and
+// its done flag, in mapped host memory
+template <class T>
+__device__ __forceinline__ void publish(const BatchArgs<T>& g, const BatchCtl& C, double eta,
+                                        double theta, double omega, double eta_sum) {
+    BatchResult R;
+    R.err = C.e_sol;
+    R.kkt_passes = C.passes;
+    R.outer = C.outer;
+    R.inner = C.inner;
+    R.total = C.total;
+    R.power_iterations = C.power_it;
+    R.eta = eta;
+    R.theta = theta;
+    R.omega = omega;
+    R.eta_sum = eta_sum;
+    R.time_elapsed = (double)(global_ns() - C.t_start) * 1e-9;
+    R.status = C.status;
+    R.restart_from_avg = C.from_avg;
+    R.stalled = C.stalled;
+    R.pad = 0;
+    g.res[C.lp] = R;
+    __threadfence_system();
+    *(volatile int*)(g.done + C.lp) = 1;
+}
+
 // solve(milp, algo) for the LP in C.  Every CTA of the group keeps its own copy
 // of C and updates it identically; rank 0 alone reads the clock and the cancel
 // flag and the others copy those two values from it.
@@ -451,43 +519,7 @@ __device__ __forceinline__ void solve_one(const BatchArgs<T>& g, BatchCtl& C, T*
             }
         }
         // ---- termination (common.jl:218-231) and restart decision (pdlp.jl:138-170)
-        if (tid == 0) {
-            C.passes += g.prm.check_every;
-            if (pdlp) {
-                C.inner += g.prm.check_every;
-                C.total += g.prm.check_every;
-            }
-            C.e_sol = C.e[0];
-            int32_t stt = CPDLP_STILL_RUNNING;
-            if (rel_err(C.e_sol) <= C.L.reltol) stt = CPDLP_OPTIMAL;
-            else if (C.tl_hit) stt = CPDLP_TIME_LIMIT;
-            else if (C.passes >= C.L.max_passes) stt = CPDLP_ITERATION_LIMIT;
-            // stall: the relative error has not halved over stall_passes passes
-            const double rel = rel_err(C.e_sol);
-            if (rel < 0.5 * C.best_rel) {
-                C.best_rel = rel;
-                C.mark = C.passes;
-            } else if (stt == CPDLP_STILL_RUNNING && C.L.stall_passes > 0 &&
-                       C.passes - C.mark >= C.L.stall_passes) {
-                stt = CPDLP_ITERATION_LIMIT;
-                C.stalled = 1;
-            }
-            const int cancelled = C.cancelled;
-            int flag = 0;
-            if (stt == CPDLP_STILL_RUNNING && !cancelled && pdlp) {
-                const double w = C.omega;
-                if (abs_err(C.e[0], w) < abs_err(C.e[1], w)) { C.from_avg = 0; C.e_cand = C.e[0]; }
-                else { C.from_avg = 1; C.e_cand = C.e[1]; }
-                C.e[2] = (abs_err(C.e[2], w) < abs_err(C.e[3], w)) ? C.e[2] : C.e[3];
-                flag = 2;  // the restart point's errors are needed first
-                if (C.restart_valid)
-                    flag = should_restart(g.prm, abs_err(C.e_cand, w), abs_err(C.e_restart, w),
-                                          abs_err(C.e[2], w), C.inner, C.total) ? 3 : 0;
-            }
-            C.status = stt;
-            C.stop = (stt != CPDLP_STILL_RUNNING) || cancelled;
-            C.flag = flag;
-        }
+        if (tid == 0) C.flag = batch_decide(g.prm, C, pdlp);
         __syncthreads();
         int flag = C.flag;
         __syncthreads();
@@ -549,35 +581,15 @@ __device__ __forceinline__ void solve_one(const BatchArgs<T>& g, BatchCtl& C, T*
     for (int i = r0 + gt; i < r1; i += GT) g.out_y[i] = g.D1[i] * (double)g.y[cur][i];
     __threadfence_system();
     Grp<CS>::sync();
-    if (rank == 0 && tid == 0) {
-        BatchResult R;
-        R.err = C.e_sol;
-        R.kkt_passes = C.passes;
-        R.outer = C.outer;
-        R.inner = C.inner;
-        R.total = C.total;
-        R.power_iterations = C.power_it;
-        R.eta = eta;
-        R.theta = g.theta[C.lp];
-        R.omega = omega;
-        R.eta_sum = C.eta_sum;
-        R.time_elapsed = (double)(global_ns() - C.t_start) * 1e-9;
-        R.status = C.status;
-        R.restart_from_avg = C.from_avg;
-        R.stalled = C.stalled;
-        R.pad = 0;
-        g.res[C.lp] = R;
-        __threadfence_system();
-        *(volatile int*)(g.done + C.lp) = 1;
-    }
+    if (rank == 0 && tid == 0) publish(g, C, eta, g.theta[C.lp], omega, C.eta_sum);
 }
 
 // an LP dequeued after a cancellation: not started
-template <class T, int CS>
+template <class T, int CS, int NT = BT>
 __device__ __forceinline__ void skip_one(const BatchArgs<T>& g, const BatchCtl& C) {
-    const int gt = Grp<CS>::rank() * BT + threadIdx.x;
-    for (int j = C.L.col_off + gt; j < C.L.col_off + C.L.n; j += BT * CS) g.out_x[j] = 0.0;
-    for (int i = C.L.row_off + gt; i < C.L.row_off + C.L.m; i += BT * CS) g.out_y[i] = 0.0;
+    const int gt = Grp<CS>::rank() * NT + threadIdx.x;
+    for (int j = C.L.col_off + gt; j < C.L.col_off + C.L.n; j += NT * CS) g.out_x[j] = 0.0;
+    for (int i = C.L.row_off + gt; i < C.L.row_off + C.L.m; i += NT * CS) g.out_y[i] = 0.0;
     __threadfence_system();
     Grp<CS>::sync();
     if (Grp<CS>::rank() == 0 && threadIdx.x == 0) {
@@ -715,6 +727,236 @@ __global__ void __launch_bounds__(BT, batch_min_blocks<T>()) k_batch_pdlp(BatchA
     // every CTA of a group leaves at the same LP; none exits while another
     // may still read its shared memory
     Grp<CS>::sync();
+}
+
+// ---- LPs resident in shared memory (resident.cuh) ------------------------------
+template <class T>
+struct ResArgs {
+    BatchArgs<T> b;
+    ResView<T> v;
+    const ResLP* rlps;
+    const double* x_start;   // power-method start vectors
+};
+
+// KKT errors of (gx, gy) into *out, thread 0 of every CTA
+template <class T, int CS, int NT>
+__device__ __forceinline__ void res_kkt(ResCtx<T, CS, NT>& X, const BatchArgs<T>& b,
+                                        const BatchCtl& C, const T* gx, const T* gy,
+                                        cpdlp_kkt_errors* out, double* sh) {
+    double v[5];
+    X.kkt(gx, gy, b.invD1t + C.L.row_off, b.invD2t + C.L.col_off, v, sh);
+    if (threadIdx.x == 0) {
+        out->primal = sqrt(v[0]);
+        out->primal_scale = C.pscale;
+        out->dual = sqrt(v[2]);
+        out->dual_scale = C.dscale;
+        out->gap = fabs((v[4] + v[1]) + v[3]);
+        out->gap_scale = (1.0 + fabs(v[1] + v[3])) + fabs(v[4]);
+    }
+}
+
+// solve(milp, algo) for the resident LP in C (see solve_one): the power method,
+// then blocks of check_every steps in shared memory; sol, sol_last and the
+// averages go to global memory after a block, for its check, a restart and the
+// solution.
+template <class T, int CS, int NT>
+__device__ __forceinline__ void solve_resident(const ResArgs<T>& g, BatchCtl& C,
+                                               ResCtx<T, CS, NT>& X,
+                                               typename ResCtx<T, CS, NT>::Coefs& tab, double* sh) {
+    const BatchArgs<T>& b = g.b;
+    const int tid = threadIdx.x, rank = X.rank;
+    const int gt = rank * NT + tid;
+    constexpr int GT = NT * CS;
+    const bool pdlp = b.prm.algorithm == CPDLP_ALGO_PDLP;
+    const int m = C.L.m, n = C.L.n, c0 = C.L.col_off, r0 = C.L.row_off;
+    double theta = C.L.theta0;
+    int64_t power_it = 0;
+    if (!(theta >= 0)) {
+        for (int j = tid; j < n; j += NT) X.px[X.invAt[j]] = g.x_start[c0 + j];
+        __syncthreads();
+        const auto P = X.power(0, INT64_MAX, C.L.power_maxiter, C.L.power_tol, C.L.power_rtol, 0.0, sh);
+        theta = P.theta;
+        power_it = P.it;
+    }
+    const double eta = b.prm.invnorm_scaling * (1.0 / sqrt(theta));
+    const T *c = b.c + c0, *lv = b.lv + c0, *uv = b.uv + c0, *lc = b.lc + r0, *uc = b.uc + r0;
+    X.load_bounds(c, lv, uv, lc, uc);
+    double omega;
+    {
+        double q[4] = {0, 0, 0, 0};
+        for (int i = gt; i < m; i += GT) {
+            const double cb = combine((double)lc[i], (double)uc[i]);
+            const double sv = b.invD1[r0 + i] * cb;
+            q[0] += sv * sv;
+            q[1] += cb * cb;
+        }
+        for (int j = gt; j < n; j += GT) {
+            const double cj = (double)c[j];
+            const double sv = b.invD2[c0 + j] * cj;
+            q[2] += sv * sv;
+            q[3] += cj * cj;
+        }
+        res_sum<4, CS, NT / 32>(q, sh);
+        const double cn = sqrt(q[3]), bn = sqrt(q[1]);
+        omega = !pdlp ? 1.0 : (cn > b.prm.zero_tol && bn > b.prm.zero_tol) ? cn / bn : 1.0;
+        if (pdlp && C.L.omega0 > 0) omega = C.L.omega0;
+        if (tid == 0) {
+            C.pscale = 1.0 + sqrt(q[0]);
+            C.dscale = 1.0 + sqrt(q[2]);
+            C.power_it = power_it;
+        }
+    }
+    // initial iterates (see solve_one); the restart point goes to global memory
+    T *gxr = b.xr + c0, *gyr = b.yr + r0;
+    const bool warm_x = C.L.warm && b.x_init, warm_y = C.L.warm && b.y_init;
+    for (int j = gt; j < n; j += GT)
+        gxr[j] = warm_x ? (T)__ddiv_rn(b.x_init[c0 + j], b.D2[c0 + j]) : T(0);
+    for (int i = gt; i < m; i += GT)
+        gyr[i] = warm_y ? (T)__ddiv_rn(b.y_init[r0 + i], b.D1[r0 + i]) : T(0);
+    if (tid == 0) {
+        C.passes = C.outer = C.inner = C.total = 0;
+        C.best_rel = INFINITY;
+        C.mark = 0;
+        C.stalled = 0;
+        C.restart_valid = 0;
+        C.from_avg = 0;
+        C.status = CPDLP_STILL_RUNNING;
+        C.stop = 0;
+        C.omega = omega;
+        tab.es = 0.0;
+    }
+    Grp<CS>::sync();
+    X.load_x(gxr);
+    X.load_xa(gxr);
+    X.load_y(gyr);
+    X.load_ya(gyr);
+    Grp<CS>::sync();
+    const typename ResCtx<T, CS, NT>::Dump d{b.x[0] + c0, b.x[1] + c0, b.xa[0] + c0, b.xa[1] + c0,
+                                             b.y[0] + r0, b.y[1] + r0, b.ya[0] + r0, b.ya[1] + r0};
+    const double tlim_ns = C.L.time_limit * 1e9;
+    while (!C.stop) {
+        X.steps(eta, omega, b.prm.check_every, pdlp, tab, d);
+        // ---- KKT errors of sol, avg, sol_last, avg_last (errors.jl:65-109)
+        const int nv = pdlp ? 4 : 1;
+        for (int p = 0; p < nv; p++)
+            res_kkt(X, b, C, p == 0 ? d.x : p == 1 ? d.xa : p == 2 ? d.xl : d.xal,
+                    p == 0 ? d.y : p == 1 ? d.ya : p == 2 ? d.yl : d.yal, &C.e[p], sh);
+        // ---- the clock and the cancel flag, read once for the group by rank 0
+        if (rank == 0 && tid == 0) {
+            C.tl_hit = (double)(global_ns() - C.t_start) >= tlim_ns ? 1 : 0;
+            C.cancelled = *(volatile const int*)b.cancel;
+        }
+        if constexpr (CS > 1) {
+            Grp<CS>::sync();
+            if (rank != 0 && tid == 0) {
+                const BatchCtl* c0p = Grp<CS>::at(&C, 0);
+                C.tl_hit = c0p->tl_hit;
+                C.cancelled = c0p->cancelled;
+            }
+        }
+        if (tid == 0) C.flag = batch_decide(b.prm, C, pdlp);
+        __syncthreads();
+        int flag = C.flag;
+        __syncthreads();
+        if (flag == 2) {
+            res_kkt(X, b, C, (const T*)gxr, (const T*)gyr, &C.e_restart, sh);
+            if (tid == 0) {
+                C.restart_valid = 1;
+                const double w = C.omega;
+                C.flag = should_restart(b.prm, abs_err(C.e_cand, w), abs_err(C.e_restart, w),
+                                        abs_err(C.e[2], w), C.inner, C.total) ? 3 : 0;
+            }
+            __syncthreads();
+            flag = C.flag;
+            __syncthreads();
+        }
+        if (flag == 3) {
+            // restart! + primal_weight_update! (pdlp.jl:172-196, step_size.jl:58-75)
+            const T* cx = C.from_avg ? d.xa : d.x;
+            const T* cy = C.from_avg ? d.ya : d.y;
+            double q[2] = {0.0, 0.0};
+            for (int j = gt; j < n; j += GT) {
+                const T v = __ldcg(cx + j);
+                const double dd = (double)v - (double)gxr[j];
+                q[0] += dd * dd;
+                gxr[j] = v;
+            }
+            for (int i = gt; i < m; i += GT) {
+                const T v = __ldcg(cy + i);
+                const double dd = (double)v - (double)gyr[i];
+                q[1] += dd * dd;
+                gyr[i] = v;
+            }
+            res_sum<2, CS, NT / 32>(q, sh);
+            const double dx = sqrt(q[0]), dy = sqrt(q[1]), th = b.prm.primal_weight_damping;
+            if (dx > b.prm.zero_tol && dy > b.prm.zero_tol)
+                omega = exp(th * log(dy / dx) + (1.0 - th) * log(omega));
+            if (tid == 0) {
+                C.omega = omega;
+                tab.es = 0.0;
+                C.e_restart = C.e_cand;
+                C.outer += 1;
+                C.inner = 0;
+            }
+            X.load_x(cx);
+            X.load_xa(nullptr);
+            X.load_y(cy);
+            X.load_ya(nullptr);
+        } else if (!C.stop) {
+            X.load_y(d.y);  // the check used the gathered copies
+        }
+        // (after a restart another block always follows, so sol in global
+        // memory need not change)
+        Grp<CS>::sync();
+    }
+    // ---- get_solution (common.jl:233-235): unscaled, double
+    for (int j = gt; j < n; j += GT) b.out_x[c0 + j] = b.D2[c0 + j] * (double)__ldcg(d.x + j);
+    for (int i = gt; i < m; i += GT) b.out_y[r0 + i] = b.D1[r0 + i] * (double)__ldcg(d.y + i);
+    __threadfence_system();
+    Grp<CS>::sync();
+    if (rank == 0 && tid == 0) publish(b, C, eta, theta, omega, tab.es);
+}
+
+// The resident solve kernel: a group per LP of a queue (normally as many
+// groups as LPs, so that the hardware starts the next one as soon as a finished
+// one's shared memory is free).
+template <class T, int CS, int NT>
+__global__ void __launch_bounds__(NT, NT == 256 ? 4 : 2) k_res_pdlp(ResArgs<T> g) {
+    extern __shared__ __align__(16) unsigned char res_smem[];
+    __shared__ double sh[NT / 32 * 8 + 8];
+    __shared__ BatchCtl C;
+    __shared__ typename ResCtx<T, CS, NT>::Coefs tab;
+    const int rank = Grp<CS>::rank();
+    for (int guard = 0; guard <= g.b.count; guard++) {
+        if (rank == 0 && threadIdx.x == 0) {
+            const int q = atomicAdd(g.b.next, 1);
+            C.lp = q < g.b.count ? g.b.order[q] : -1;
+            C.cancelled = C.lp >= 0 ? *(volatile const int*)g.b.cancel : 0;
+        }
+        if constexpr (CS > 1) {
+            Grp<CS>::sync();
+            if (rank != 0 && threadIdx.x == 0) {
+                const BatchCtl* c0p = Grp<CS>::at(&C, 0);
+                C.lp = c0p->lp;
+                C.cancelled = c0p->cancelled;
+            }
+            Grp<CS>::sync();  // rank 0's copy is read before it changes or exits
+        }
+        if (threadIdx.x == 0 && C.lp >= 0) {
+            C.L = g.b.lps[C.lp];
+            C.t_start = global_ns();
+        }
+        __syncthreads();
+        if (C.lp < 0) break;
+        if (C.cancelled) skip_one<T, CS, NT>(g.b, C);
+        else {
+            ResCtx<T, CS, NT> X;
+            X.load(g.rlps[C.lp], g.v, res_smem);
+            solve_resident<T, CS, NT>(g, C, X, tab, sh);
+        }
+        Grp<CS>::sync();
+    }
+    Grp<CS>::sync();  // no CTA exits while another may read or write its shared memory
 }
 
 uint64_t splitmix64_at_host(uint64_t seed, uint64_t counter) {
@@ -858,6 +1100,8 @@ struct Run : RunBase {
     DBuf<int32_t> d_order;
     DBuf<int> d_next;
     DBuf<double> pw_x, pw_Atx, pw_s, pw_start, pw_pA, pw_pAt;  // power-method scratch
+    ResStore<T> res;           // the slices of the resident LPs
+    DBuf<ResLP> d_rlps;
 
     ~Run() override { close(); }
 
@@ -939,9 +1183,28 @@ struct Run : RunBase {
         CK(cudaMemcpyAsync(hpA.data(), P.a_ptr.p, sizeof(int32_t) * (M + 1), cudaMemcpyDeviceToHost, s));
         CK(cudaMemcpyAsync(hpAt.data(), P.at_ptr.p, sizeof(int32_t) * (N + 1), cudaMemcpyDeviceToHost, s));
         CK(cudaStreamSynchronize(s));
+        // LPs that fit a CTA's or a cluster's shared memory go to the resident
+        // kernels (resident.cuh), the others to the tile kernels.  The route
+        // depends on the LP and the value type alone, so its arithmetic does too.
+        std::vector<ResLP> rlps((size_t)count);
+        std::vector<std::vector<int32_t>> rmA((size_t)count), rmAt((size_t)count);
+        std::vector<char> resident((size_t)count, 0);
+        parallel_for(count, [&](int64_t k) {
+            const cpdlp_lp& L = all[lps[k].id].v;
+            ResLP& r = rlps[(size_t)k];
+            r = ResLP{};
+            r.row_off = (int32_t)row_off[k];
+            r.col_off = (int32_t)col_off[k];
+            resident[(size_t)k] = res_plan(hpA.data() + row_off[k], hpAt.data() + col_off[k], L.m, L.n,
+                                           L.nnz, (int)sizeof(T), false, r, rmA[(size_t)k],
+                                           rmAt[(size_t)k]) > 0;
+        });
+        const std::vector<LaunchClass> classes = stage_resident(rlps, rmA, rmAt, resident, nz_off, P);
         std::vector<int32_t> aT, aL, aI, atT, atL, atI;
-        build_tile_plan(hpA, (int32_t)M, items, planA, s, &row_off, &aT, &aL, &aI, 32 * BATCH_RPL);
-        build_tile_plan(hpAt, (int32_t)N, items, planAt, s, &col_off, &atT, &atL, &atI, 32 * BATCH_RPL);
+        build_tile_plan(hpA, (int32_t)M, items, planA, s, &row_off, &aT, &aL, &aI, 32 * BATCH_RPL,
+                        &resident);
+        build_tile_plan(hpAt, (int32_t)N, items, planAt, s, &col_off, &atT, &atL, &atI, 32 * BATCH_RPL,
+                        &resident);
         partA.alloc((size_t)std::max(planA.npieces, 1));
         partAt.alloc((size_t)std::max(planAt.npieces, 1));
         // per-LP descriptors and the largest-first queue order
@@ -973,9 +1236,13 @@ struct Run : RunBase {
             d.theta0 = lps[k].theta0;
             d.omega0 = lps[k].omega0;
         }
-        std::vector<int32_t> order((size_t)count);
-        std::iota(order.begin(), order.end(), 0);
-        std::stable_sort(order.begin(), order.end(), [&](int32_t a, int32_t b) {
+        std::vector<int32_t> order;   // the tile kernels' queue
+        for (int64_t k = 0; k < count; k++)
+            if (!resident[(size_t)k]) order.push_back((int32_t)k);
+        const int64_t ntile = (int64_t)order.size();
+        // then the resident kernels' queues, one after another
+        for (const LaunchClass& cl : classes) order.insert(order.end(), cl.lps.begin(), cl.lps.end());
+        std::stable_sort(order.begin(), order.begin() + ntile, [&](int32_t a, int32_t b) {
             return nz_off[a + 1] - nz_off[a] > nz_off[b + 1] - nz_off[b];
         });
         // largest first: the first nbig LPs of the order go to the cluster kernel
@@ -984,7 +1251,7 @@ struct Run : RunBase {
         const int64_t cmin = phase == 2 ? PHASE_CLUSTER_MIN_NNZ : CLUSTER_MIN_NNZ;
         int64_t nbig = 0;
         if (nclusters > 0 && nclusters_p > 0)
-            while (nbig < count && nz_off[order[nbig] + 1] - nz_off[order[nbig]] >= cmin) nbig++;
+            while (nbig < ntile && nz_off[order[nbig] + 1] - nz_off[order[nbig]] >= cmin) nbig++;
         // power-method start vectors: the single-LP generator, per LP from counter
         // 0, so every LP's vector is a prefix of one vector (computed once)
         int64_t nmax = 0;
@@ -1019,7 +1286,7 @@ struct Run : RunBase {
         d_piters.alloc((size_t)std::max<int64_t>(count, 1));
         longA.alloc((size_t)std::max(planA.nlong, 1) * 2);
         longAt.alloc((size_t)std::max(planAt.nlong, 1) * 3);
-        d_next.alloc(4);
+        d_next.alloc(4 + classes.size());
         if (any_warm) {
             d_x0.alloc(nz);
             d_y0.alloc(mz);
@@ -1028,7 +1295,7 @@ struct Run : RunBase {
         }
         CK(cudaMemcpyAsync(d_desc.p, desc.data(), sizeof(BatchLP) * desc.size(), cudaMemcpyHostToDevice, s));
         CK(cudaMemcpyAsync(d_order.p, order.data(), sizeof(int32_t) * order.size(), cudaMemcpyHostToDevice, s));
-        CK(cudaMemsetAsync(d_next.p, 0, 4 * sizeof(int), s));
+        CK(cudaMemsetAsync(d_next.p, 0, d_next.n * sizeof(int), s));
         // power method: FP64 vectors; the cluster-sized LPs on s2, the others on s
         pw_x.alloc(nz); pw_Atx.alloc(nz); pw_s.alloc(mz); pw_start.alloc(nz);
         pw_pA.alloc((size_t)std::max(planA.npieces, 1));
@@ -1054,12 +1321,12 @@ struct Run : RunBase {
             ccfg.gridDim = dim3((unsigned)(nc * CLUSTER_CTAS));
             CK(cudaLaunchKernelEx(&ccfg, pkc, pb));
         }
-        if (count > nbig) {
+        if (ntile > nbig) {
             PowerArgs<T> ps1 = pg;
             ps1.order = d_order.p + nbig;
-            ps1.count = (int32_t)(count - nbig);
+            ps1.count = (int32_t)(ntile - nbig);
             ps1.next = d_next.p + 1;
-            int64_t pgrid = std::min<int64_t>(count - nbig, (int64_t)std::max(per_sm_p, 1) * rh.num_sms);
+            int64_t pgrid = std::min<int64_t>(ntile - nbig, (int64_t)std::max(per_sm_p, 1) * rh.num_sms);
             if (max_ctas > 0) pgrid = std::min(pgrid, max_ctas);
             pgrid = std::max<int64_t>(pgrid, 1);
             pk<<<(unsigned)pgrid, BT, 0, s>>>(ps1);
@@ -1102,17 +1369,163 @@ struct Run : RunBase {
             CK(cudaLaunchKernelEx(&ccfg, kclu, gb));  // after s2's power method
             CK(cudaEventRecord(ev2, s2));
         }
-        if (count > nbig) {
+        launch_resident(g, classes, ntile, max_ctas);
+        if (ntile > nbig) {
             g.order = d_order.p + nbig;
-            g.count = (int32_t)(count - nbig);
-            grid = std::max<int64_t>(std::min<int64_t>(grid, count - nbig), 1);
+            g.count = (int32_t)(ntile - nbig);
+            grid = std::max<int64_t>(std::min<int64_t>(grid, ntile - nbig), 1);
             kern<<<(unsigned)grid, BT, 0, s>>>(g);
             CK_LAUNCH();
         }
         if (nbig > 0) CK(cudaStreamWaitEvent(s, ev2, 0));
+        for (cudaEvent_t e : class_ev) CK(cudaStreamWaitEvent(s, e, 0));
         CK(cudaEventRecord(ev, s));
     }
+
+    // ---- resident LPs --------------------------------------------------------
+    // LPs of one cluster size and shared-memory class: one launch on a stream of
+    // its own, the largest first.  Up to 52 KB a CTA (four resident per SM) the
+    // CTAs have 256 threads, above that 512 (two per SM up to 108 KB).
+    struct LaunchClass {
+        int cs, threads;
+        uint32_t smem;              // of its largest LP
+        std::vector<int32_t> lps;
+    };
+    std::vector<LaunchClass> stage_resident(std::vector<ResLP>& r, std::vector<std::vector<int32_t>>& mA,
+                                            std::vector<std::vector<int32_t>>& mAt,
+                                            const std::vector<char>& resident,
+                                            const std::vector<int64_t>& nz_off, ProblemT<T>& P) {
+        std::vector<LaunchClass> out;
+        std::vector<int32_t> ids;
+        for (size_t k = 0; k < r.size(); k++)
+            if (resident[k]) ids.push_back((int32_t)k);
+        if (ids.empty()) return out;
+        cudaStream_t s = rh.stream;
+        int64_t eA = 0, eAt = 0, max_rows = 0;
+        std::vector<int32_t> metaA, metaAt;
+        std::vector<ResLP> build;
+        for (int32_t k : ids) {
+            ResLP& q = r[(size_t)k];
+            q.eA = eA;
+            q.eAt = eAt;
+            q.mA = (int32_t)metaA.size();
+            q.mAt = (int32_t)metaAt.size();
+            eA += 32 * (int64_t)mA[(size_t)k][(size_t)q.cs];
+            eAt += 32 * (int64_t)mAt[(size_t)k][(size_t)q.cs];
+            metaA.insert(metaA.end(), mA[(size_t)k].begin(), mA[(size_t)k].end());
+            metaAt.insert(metaAt.end(), mAt[(size_t)k].begin(), mAt[(size_t)k].end());
+            max_rows = std::max<int64_t>(max_rows, std::max(q.m, q.n));
+            build.push_back(q);
+        }
+        const size_t M = (size_t)std::max<int64_t>(P.m, 1), N = (size_t)std::max<int64_t>(P.n, 1);
+        res.idxA.alloc((size_t)eA);
+        res.idxAt.alloc((size_t)eAt);
+        res.valA.alloc((size_t)eA);
+        res.valAt.alloc((size_t)eAt);
+        res.metaA.alloc(metaA.size());
+        res.metaAt.alloc(metaAt.size());
+        res.ordA.alloc(M);
+        res.ordAt.alloc(N);
+        res.invA.alloc(M);
+        res.invAt.alloc(N);
+        res.lenA.alloc(M);
+        res.lenAt.alloc(N);
+        // kernels index the descriptors by LP; the build takes the resident ones
+        DBuf<ResLP> d_build(build.size());
+        d_rlps.alloc(r.size());
+        CK(cudaMemcpyAsync(res.metaA.p, metaA.data(), sizeof(int32_t) * metaA.size(), cudaMemcpyHostToDevice, s));
+        CK(cudaMemcpyAsync(res.metaAt.p, metaAt.data(), sizeof(int32_t) * metaAt.size(), cudaMemcpyHostToDevice, s));
+        CK(cudaMemcpyAsync(d_rlps.p, r.data(), sizeof(ResLP) * r.size(), cudaMemcpyHostToDevice, s));
+        CK(cudaMemcpyAsync(d_build.p, build.data(), sizeof(ResLP) * build.size(), cudaMemcpyHostToDevice, s));
+        res_build<T>(res, d_build.p, (int)build.size(), P.a_ptr.p, P.a_idx.p, P.a_val.p, P.at_ptr.p,
+                     P.at_idx.p, P.at_val.p, max_rows, s);
+        // classes, largest shared memory first
+        std::stable_sort(ids.begin(), ids.end(), [&](int32_t a, int32_t b) {
+            return nz_off[a + 1] - nz_off[a] > nz_off[b + 1] - nz_off[b];
+        });
+        for (int cs = RES_MAX_CS; cs >= 1; cs /= 2)
+            for (int band = 2; band >= 0; band--) {
+                LaunchClass c{cs, band == 0 ? 256 : 512, 0, {}};
+                for (int32_t k : ids) {
+                    const ResLP& q = r[(size_t)k];
+                    if (q.cs != cs) continue;
+                    const uint32_t t = res_layout<T>(q).total;
+                    if (band != (t > 108 * 1024 ? 2 : t > 52 * 1024 ? 1 : 0)) continue;
+                    c.lps.push_back(k);
+                    c.smem = std::max(c.smem, t);
+                }
+                if (!c.lps.empty()) out.push_back(std::move(c));
+            }
+        return out;
+    }
+
+    template <int CS, int NT>
+    void launch_class(const ResArgs<T>& a, const LaunchClass& c, int64_t max_ctas, cudaStream_t s) {
+        auto kern = k_res_pdlp<T, CS, NT>;
+        CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RES_MAX_SMEM));
+        int64_t groups = (int64_t)c.lps.size();
+        if (max_ctas > 0) groups = std::min<int64_t>(groups, std::max<int64_t>(max_ctas / CS, 1));
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = CS;
+        attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = 1;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)(groups * CS));
+        cfg.blockDim = dim3(NT);
+        cfg.dynamicSmemBytes = c.smem;
+        cfg.stream = s;
+        cfg.attrs = attr;
+        cfg.numAttrs = CS > 1 ? 1 : 0;
+        CK(cudaLaunchKernelEx(&cfg, kern, a));
+    }
+
+    std::vector<cudaStream_t> class_s;
+    std::vector<cudaEvent_t> class_ev;
+    // the classes' kernels, each on its own stream after everything queued on s
+    void launch_resident(const BatchArgs<T>& g, const std::vector<LaunchClass>& classes, int64_t first,
+                         int64_t max_ctas) {
+        if (classes.empty()) return;
+        cudaStream_t s = rh.stream;
+        class_ev.resize(classes.size(), nullptr);
+        class_s.resize(classes.size(), nullptr);
+        cudaEvent_t ready = nullptr;
+        CK(cudaEventCreateWithFlags(&ready, cudaEventDisableTiming));
+        struct Drop { cudaEvent_t e; ~Drop() { cudaEventDestroy(e); } } drop{ready};
+        CK(cudaEventRecord(ready, s));
+        for (size_t k = 0; k < classes.size(); k++) {
+            const LaunchClass& c = classes[k];
+            CK(cudaStreamCreateWithFlags(&class_s[k], cudaStreamNonBlocking));
+            CK(cudaEventCreateWithFlags(&class_ev[k], cudaEventDisableTiming));
+            CK(cudaStreamWaitEvent(class_s[k], ready, 0));
+            ResArgs<T> a;
+            a.b = g;
+            a.b.order = d_order.p + first;
+            a.b.count = (int32_t)c.lps.size();
+            a.b.next = d_next.p + 4 + k;
+            a.v = res_view(res);
+            a.rlps = d_rlps.p;
+            a.x_start = pw_start.p;
+            first += (int64_t)c.lps.size();
+            const bool wide = c.threads == 512;
+            if (c.cs == 1) wide ? launch_class<1, 512>(a, c, max_ctas, class_s[k]) : launch_class<1, 256>(a, c, max_ctas, class_s[k]);
+            else if (c.cs == 2) wide ? launch_class<2, 512>(a, c, max_ctas, class_s[k]) : launch_class<2, 256>(a, c, max_ctas, class_s[k]);
+            else if (c.cs == 4) wide ? launch_class<4, 512>(a, c, max_ctas, class_s[k]) : launch_class<4, 256>(a, c, max_ctas, class_s[k]);
+            else wide ? launch_class<8, 512>(a, c, max_ctas, class_s[k]) : launch_class<8, 256>(a, c, max_ctas, class_s[k]);
+            CK(cudaEventRecord(class_ev[k], class_s[k]));
+        }
+    }
+
     void release_device() override {
+        for (cudaEvent_t e : class_ev)
+            if (e) cudaEventDestroy(e);
+        for (cudaStream_t t : class_s)
+            if (t) {
+                cudaStreamSynchronize(t);
+                cudaStreamDestroy(t);
+            }
+        class_ev.clear();
+        class_s.clear();
         AllocScope scope(rh.stream);
         PB.reset();
         for (int b = 0; b < 2; b++) { bx[b].release(); by[b].release(); bxa[b].release(); bya[b].release(); }
@@ -1121,6 +1534,8 @@ struct Run : RunBase {
         d_order.release(); d_theta.release(); d_piters.release(); d_next.release();
         pw_x.release(); pw_Atx.release(); pw_s.release(); pw_start.release();
         pw_pA.release(); pw_pAt.release();
+        res.release();
+        d_rlps.release();
         planA = TilePlan();
         planAt = TilePlan();
     }

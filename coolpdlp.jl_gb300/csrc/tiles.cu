@@ -22,7 +22,8 @@ int choose_items(int64_t nnz, int64_t rows, int requested_tile_nnz) {
 void build_tile_plan(const std::vector<int32_t>& ptr, int32_t rows, int items, TilePlan& plan,
                      cudaStream_t s, const std::vector<int64_t>* seg_rows,
                      std::vector<int32_t>* seg_tasks, std::vector<int32_t>* seg_ltasks,
-                     std::vector<int32_t>* seg_lids, int max_rows) {
+                     std::vector<int32_t>* seg_lids, int max_rows,
+                     const std::vector<char>* seg_skip) {
     if (max_rows < 32 || max_rows > MAX_TILE_ROWS || max_rows % 32 != 0)
         fail(CPDLP_ERR_ARGUMENT, "tile row cap must be a multiple of 32 up to 128");
     plan.rows = rows;
@@ -51,6 +52,7 @@ void build_tile_plan(const std::vector<int32_t>& ptr, int32_t rows, int items, T
         if (seg_tasks) (*seg_tasks)[k] = (int32_t)shorts.size();
         if (seg_ltasks) (*seg_ltasks)[k] = (int32_t)longs.size();
         if (seg_lids) (*seg_lids)[k] = (int32_t)plan.long_rows.size();
+        if (seg_skip && (*seg_skip)[k]) continue;
         const int32_t end = (int32_t)segs[k + 1];
         int32_t r = (int32_t)segs[k];
         while (r < end) {

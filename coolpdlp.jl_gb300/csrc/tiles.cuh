@@ -59,6 +59,7 @@ struct TilePlan {
 // With seg_rows (segment start rows, last = rows) no tile crosses a segment
 // start, and seg_tasks / seg_ltasks / seg_lids receive, per segment, the first
 // short task, long task and long-row id (one extra final entry = totals).
+// Segments with seg_skip[k] != 0 get no tasks.
 // max_rows caps the rows of a short tile (a multiple of 32, at most
 // MAX_TILE_ROWS): kernels built for max_rows / 32 rows per lane.  With the
 // default cap, a matrix with rows of LONG_ROW+1 .. TILE nonzeros (which short
@@ -68,7 +69,8 @@ void build_tile_plan(const std::vector<int32_t>& ptr, int32_t rows, int items, T
                      cudaStream_t s, const std::vector<int64_t>* seg_rows = nullptr,
                      std::vector<int32_t>* seg_tasks = nullptr,
                      std::vector<int32_t>* seg_ltasks = nullptr,
-                     std::vector<int32_t>* seg_lids = nullptr, int max_rows = MAX_TILE_ROWS);
+                     std::vector<int32_t>* seg_lids = nullptr, int max_rows = MAX_TILE_ROWS,
+                     const std::vector<char>* seg_skip = nullptr);
 
 // Picks nonzeros-per-lane from the size and mean row length (autotuner default).
 int choose_items(int64_t nnz, int64_t rows, int requested_tile_nnz);
