@@ -740,11 +740,11 @@ struct ResArgs {
 
 // KKT errors of (gx, gy) into *out, thread 0 of every CTA
 template <class T, int CS, int NT>
-__device__ __forceinline__ void res_kkt(ResCtx<T, CS, NT>& X, const BatchArgs<T>& b,
-                                        const BatchCtl& C, const T* gx, const T* gy,
-                                        cpdlp_kkt_errors* out, double* sh) {
+__device__ __forceinline__ void res_kkt(ResGeo& G, const BatchArgs<T>& b, const BatchCtl& C,
+                                        const T* gx, const T* gy, cpdlp_kkt_errors* out, double* sh,
+                                        int& phase) {
     double v[5];
-    X.kkt(gx, gy, b.invD1t + C.L.row_off, b.invD2t + C.L.col_off, v, sh);
+    res_kkt_sums<T, CS, NT>(G, gx, gy, b.invD1t + C.L.row_off, b.invD2t + C.L.col_off, v, sh, phase);
     if (threadIdx.x == 0) {
         out->primal = sqrt(v[0]);
         out->primal_scale = C.pscale;
@@ -755,32 +755,36 @@ __device__ __forceinline__ void res_kkt(ResCtx<T, CS, NT>& X, const BatchArgs<T>
     }
 }
 
-// solve(milp, algo) for the resident LP in C (see solve_one): the power method,
-// then blocks of check_every steps in shared memory; sol, sol_last and the
-// averages go to global memory after a block, for its check, a restart and the
-// solution.
+// solve(milp, algo) for the resident LP in C and G (see solve_one): the power
+// method, then blocks of check_every steps in shared memory; sol, sol_last and
+// the averages go to global memory after a block, for its check, a restart and
+// the solution.
 template <class T, int CS, int NT>
-__device__ __forceinline__ void solve_resident(const ResArgs<T>& g, BatchCtl& C,
-                                               ResCtx<T, CS, NT>& X,
-                                               typename ResCtx<T, CS, NT>::Coefs& tab, double* sh) {
+__device__ __forceinline__ void solve_resident(const ResArgs<T>& g, BatchCtl& C, ResGeo& G,
+                                               ResCoefs<T>& tab, double* sh, ResWait& W,
+                                               unsigned& parity) {
     const BatchArgs<T>& b = g.b;
-    const int tid = threadIdx.x, rank = X.rank;
+    const int tid = threadIdx.x, rank = G.rank;
     const int gt = rank * NT + tid;
     constexpr int GT = NT * CS;
+    int phase = 0;
     const bool pdlp = b.prm.algorithm == CPDLP_ALGO_PDLP;
     const int m = C.L.m, n = C.L.n, c0 = C.L.col_off, r0 = C.L.row_off;
     double theta = C.L.theta0;
     int64_t power_it = 0;
     if (!(theta >= 0)) {
-        for (int j = tid; j < n; j += NT) X.px[X.invAt[j]] = g.x_start[c0 + j];
+        double* px = &sm_at<double>(G.px);
+        for (int j = tid; j < n; j += NT) px[G.invAt[j]] = g.x_start[c0 + j];
         __syncthreads();
-        const auto P = X.power(0, INT64_MAX, C.L.power_maxiter, C.L.power_tol, C.L.power_rtol, 0.0, sh);
+        ResPower P;
+        res_power<T, CS, NT>(G, 0, INT64_MAX, C.L.power_maxiter, C.L.power_tol, C.L.power_rtol, 0.0, P,
+                             sh, phase, W, parity);
         theta = P.theta;
         power_it = P.it;
     }
     const double eta = b.prm.invnorm_scaling * (1.0 / sqrt(theta));
     const T *c = b.c + c0, *lv = b.lv + c0, *uv = b.uv + c0, *lc = b.lc + r0, *uc = b.uc + r0;
-    X.load_bounds(c, lv, uv, lc, uc);
+    res_bounds<T, CS, NT>(G, c, lv, uv, lc, uc);
     double omega;
     {
         double q[4] = {0, 0, 0, 0};
@@ -796,7 +800,7 @@ __device__ __forceinline__ void solve_resident(const ResArgs<T>& g, BatchCtl& C,
             q[2] += sv * sv;
             q[3] += cj * cj;
         }
-        res_sum<4, CS, NT / 32>(q, sh);
+        res_sum<4, CS, NT / 32>(q, sh, phase);
         const double cn = sqrt(q[3]), bn = sqrt(q[1]);
         omega = !pdlp ? 1.0 : (cn > b.prm.zero_tol && bn > b.prm.zero_tol) ? cn / bn : 1.0;
         if (pdlp && C.L.omega0 > 0) omega = C.L.omega0;
@@ -826,25 +830,23 @@ __device__ __forceinline__ void solve_resident(const ResArgs<T>& g, BatchCtl& C,
         tab.es = 0.0;
     }
     Grp<CS>::sync();
-    X.load_x(gxr);
-    X.load_xa(gxr);
-    X.load_y(gyr);
-    X.load_ya(gyr);
+    res_load_iterate<T, CS, NT>(G, gxr, gxr, gyr, gyr);
     Grp<CS>::sync();
-    const typename ResCtx<T, CS, NT>::Dump d{b.x[0] + c0, b.x[1] + c0, b.xa[0] + c0, b.xa[1] + c0,
+    const ResDump<T> d{b.x[0] + c0, b.x[1] + c0, b.xa[0] + c0, b.xa[1] + c0,
                                              b.y[0] + r0, b.y[1] + r0, b.ya[0] + r0, b.ya[1] + r0};
     const double tlim_ns = C.L.time_limit * 1e9;
     while (!C.stop) {
-        X.steps(eta, omega, b.prm.check_every, pdlp, tab, d);
+        res_steps<T, CS, NT>(G, eta, omega, b.prm.check_every, pdlp, tab, d, W, parity);
         // ---- KKT errors of sol, avg, sol_last, avg_last (errors.jl:65-109)
         const int nv = pdlp ? 4 : 1;
         for (int p = 0; p < nv; p++)
-            res_kkt(X, b, C, p == 0 ? d.x : p == 1 ? d.xa : p == 2 ? d.xl : d.xal,
-                    p == 0 ? d.y : p == 1 ? d.ya : p == 2 ? d.yl : d.yal, &C.e[p], sh);
+            res_kkt<T, CS, NT>(G, b, C, p == 0 ? d.x : p == 1 ? d.xa : p == 2 ? d.xl : d.xal,
+                               p == 0 ? d.y : p == 1 ? d.ya : p == 2 ? d.yl : d.yal, &C.e[p], sh,
+                               phase);
         // ---- the clock and the cancel flag, read once for the group by rank 0
         if (rank == 0 && tid == 0) {
             C.tl_hit = (double)(global_ns() - C.t_start) >= tlim_ns ? 1 : 0;
-            C.cancelled = *(volatile const int*)b.cancel;
+            C.cancelled = *(volatile const int*)b.cancel || W.failed;
         }
         if constexpr (CS > 1) {
             Grp<CS>::sync();
@@ -859,7 +861,7 @@ __device__ __forceinline__ void solve_resident(const ResArgs<T>& g, BatchCtl& C,
         int flag = C.flag;
         __syncthreads();
         if (flag == 2) {
-            res_kkt(X, b, C, (const T*)gxr, (const T*)gyr, &C.e_restart, sh);
+            res_kkt<T, CS, NT>(G, b, C, gxr, gyr, &C.e_restart, sh, phase);
             if (tid == 0) {
                 C.restart_valid = 1;
                 const double w = C.omega;
@@ -887,7 +889,7 @@ __device__ __forceinline__ void solve_resident(const ResArgs<T>& g, BatchCtl& C,
                 q[1] += dd * dd;
                 gyr[i] = v;
             }
-            res_sum<2, CS, NT / 32>(q, sh);
+            res_sum<2, CS, NT / 32>(q, sh, phase);
             const double dx = sqrt(q[0]), dy = sqrt(q[1]), th = b.prm.primal_weight_damping;
             if (dx > b.prm.zero_tol && dy > b.prm.zero_tol)
                 omega = exp(th * log(dy / dx) + (1.0 - th) * log(omega));
@@ -898,12 +900,9 @@ __device__ __forceinline__ void solve_resident(const ResArgs<T>& g, BatchCtl& C,
                 C.outer += 1;
                 C.inner = 0;
             }
-            X.load_x(cx);
-            X.load_xa(nullptr);
-            X.load_y(cy);
-            X.load_ya(nullptr);
+            res_load_iterate<T, CS, NT>(G, cx, nullptr, cy, nullptr);
         } else if (!C.stop) {
-            X.load_y(d.y);  // the check used the gathered copies
+            res_load_y<T, NT>(G, d.y);  // the check used the gathered copies
         }
         // (after a restart another block always follows, so sol in global
         // memory need not change)
@@ -914,7 +913,8 @@ __device__ __forceinline__ void solve_resident(const ResArgs<T>& g, BatchCtl& C,
     for (int i = gt; i < m; i += GT) b.out_y[r0 + i] = b.D1[r0 + i] * (double)__ldcg(d.y + i);
     __threadfence_system();
     Grp<CS>::sync();
-    if (rank == 0 && tid == 0) publish(b, C, eta, theta, omega, tab.es);
+    // (a wait that ran out leaves the done flag unset: the host reports an error)
+    if (rank == 0 && tid == 0 && !W.failed) publish(b, C, eta, theta, omega, tab.es);
 }
 
 // The resident solve kernel: a group per LP of a queue (normally as many
@@ -922,10 +922,13 @@ __device__ __forceinline__ void solve_resident(const ResArgs<T>& g, BatchCtl& C,
 // one's shared memory is free).
 template <class T, int CS, int NT>
 __global__ void __launch_bounds__(NT, NT == 256 ? 4 : 2) k_res_pdlp(ResArgs<T> g) {
-    extern __shared__ __align__(16) unsigned char res_smem[];
-    __shared__ double sh[NT / 32 * 8 + 8];
+    __shared__ double sh[res_sh<CS, NT / 32>()];
     __shared__ BatchCtl C;
-    __shared__ typename ResCtx<T, CS, NT>::Coefs tab;
+    __shared__ ResCoefs<T> tab;
+    __shared__ ResGeo G;
+    __shared__ ResWait W;
+    unsigned parity = 0;
+    if (threadIdx.x == 0) res_wait_init(W);
     const int rank = Grp<CS>::rank();
     for (int guard = 0; guard <= g.b.count; guard++) {
         if (rank == 0 && threadIdx.x == 0) {
@@ -950,9 +953,8 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 4 : 2) k_res_pdlp(ResArgs<T> g
         if (C.lp < 0) break;
         if (C.cancelled) skip_one<T, CS, NT>(g.b, C);
         else {
-            ResCtx<T, CS, NT> X;
-            X.load(g.rlps[C.lp], g.v, res_smem);
-            solve_resident<T, CS, NT>(g, C, X, tab, sh);
+            res_load<T, CS, NT>(G, g.rlps[C.lp], g.v);
+            solve_resident<T, CS, NT>(g, C, G, tab, sh, W, parity);
         }
         Grp<CS>::sync();
     }

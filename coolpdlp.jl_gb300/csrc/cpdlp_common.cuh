@@ -97,6 +97,10 @@ struct DBuf {
 // scalar semantics shared by host and device (src/utils/linalg.jl:1-53)
 // Base.max/min on floats: NaN propagates and -0.0 < +0.0.
 // ---------------------------------------------------------------------------
+// On the device: FP32 is one instruction (max.NaN orders -0 below +0 too).
+// FP64 compares bit patterns as integers, because a comparison on GB300's FP64
+// pipe (1.9 lanes a clock and SM) costs as much as an addition and a projection
+// onto a box has six: they were 6 of a primal row's 14 FP64 operations.
 template <class T>
 __host__ __device__ __forceinline__ T jl_max(T x, T y) {
     bool sx = signbit(x), sy = signbit(y);
@@ -108,6 +112,62 @@ __host__ __device__ __forceinline__ T jl_min(T x, T y) {
     bool sx = signbit(x), sy = signbit(y);
     if ((y < x) || (sy > sx)) return (x != x) ? x : y;
     return (y != y) ? y : x;
+}
+#ifdef __CUDACC__
+// order-preserving integer of a double (-0 just below +0; NaNs outside the infinities)
+__device__ __forceinline__ long long f64_key(double x) {
+    const long long b = __double_as_longlong(x);
+    return b ^ (long long)((unsigned long long)(b >> 63) >> 1);
+}
+__device__ __forceinline__ bool f64_is_nan(double x) {
+    return (__double_as_longlong(x) & 0x7fffffffffffffffll) > 0x7ff0000000000000ll;
+}
+#endif
+template <>
+__host__ __device__ __forceinline__ float jl_max<float>(float x, float y) {
+#ifdef __CUDA_ARCH__
+    float r;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(x), "f"(y));
+    return r;
+#else
+    bool sx = std::signbit(x), sy = std::signbit(y);
+    if ((y > x) || (sy < sx)) return (x != x) ? x : y;
+    return (y != y) ? y : x;
+#endif
+}
+template <>
+__host__ __device__ __forceinline__ float jl_min<float>(float x, float y) {
+#ifdef __CUDA_ARCH__
+    float r;
+    asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(x), "f"(y));
+    return r;
+#else
+    bool sx = std::signbit(x), sy = std::signbit(y);
+    if ((y < x) || (sy > sx)) return (x != x) ? x : y;
+    return (y != y) ? y : x;
+#endif
+}
+template <>
+__host__ __device__ __forceinline__ double jl_max<double>(double x, double y) {
+#ifdef __CUDA_ARCH__
+    const double r = f64_key(y) > f64_key(x) ? y : x;
+    return f64_is_nan(x) ? x : f64_is_nan(y) ? y : r;
+#else
+    bool sx = std::signbit(x), sy = std::signbit(y);
+    if ((y > x) || (sy < sx)) return (x != x) ? x : y;
+    return (y != y) ? y : x;
+#endif
+}
+template <>
+__host__ __device__ __forceinline__ double jl_min<double>(double x, double y) {
+#ifdef __CUDA_ARCH__
+    const double r = f64_key(y) < f64_key(x) ? y : x;
+    return f64_is_nan(x) ? x : f64_is_nan(y) ? y : r;
+#else
+    bool sx = std::signbit(x), sy = std::signbit(y);
+    if ((y < x) || (sy > sx)) return (x != x) ? x : y;
+    return (y != y) ? y : x;
+#endif
 }
 template <class T>
 __host__ __device__ __forceinline__ T proj_box(T x, T l, T u) { return jl_min(u, jl_max(l, x)); }
@@ -138,6 +198,11 @@ __device__ __forceinline__ double add_rn(double a, double b) { return __dadd_rn(
 __device__ __forceinline__ float add_rn(float a, float b) { return __fadd_rn(a, b); }
 __device__ __forceinline__ double sub_rn(double a, double b) { return __dsub_rn(a, b); }
 __device__ __forceinline__ float sub_rn(float a, float b) { return __fsub_rn(a, b); }
+
+// 2x - y: doubling is exact, so one fused operation rounds like the product
+// and the difference do
+__device__ __forceinline__ double extrapolate(double x, double y) { return __fma_rn(2.0, x, -y); }
+__device__ __forceinline__ float extrapolate(float x, float y) { return __fmaf_rn(2.0f, x, -y); }
 
 // Scalar loads as volatile PTX: volatile asm statements keep their relative
 // order, so loads meant to be in flight together (prefetches) are issued

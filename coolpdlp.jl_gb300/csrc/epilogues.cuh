@@ -97,7 +97,7 @@ struct PrimalEpi {
         if (SCALED) s = mul_rn(q.d, s);
         const T xp = proj_box(sub_rn(q.x, mul_rn(k.tau, sub_rn(q.c, s))), q.lv, q.uv);
         __stcs(xn + j, xp);
-        const T xb = sub_rn(mul_rn(T(2), xp), q.x);
+        const T xb = extrapolate(xp, q.x);
         xbar[j] = SCALED ? mul_rn(q.d, xb) : xb;
         if (avg) __stcs(xa_new + j, add_rn(mul_rn(xp, k.a), mul_rn(q.xa, k.b)));
     }

@@ -25,6 +25,7 @@ __global__ void __launch_bounds__(256)
     int32_t* ord = (t ? ordAt : ordA) + off;
     uint16_t* inv = (t ? invAt : invA) + off;
     uint8_t* lo = (t ? lenAt : lenA) + off;
+    const int loc = res_local(rows, L.cs);
     for (int k = threadIdx.x; k <= LONG_ROW; k += blockDim.x) hist[k] = 0;
     __syncthreads();
     for (int r = threadIdx.x; r < rows; r += blockDim.x) {
@@ -55,8 +56,11 @@ __global__ void __launch_bounds__(256)
         if (in && rank == 0) hist[n] += __popc(peers);
         __syncwarp();
         if (in) {
+            // place `at` is row at % 32 of slice at / 32, which is slice
+            // (at / 32) / cs of rank (at / 32) % cs; a rank's slices are a block
+            const int s = at >> 5;
             ord[at] = r;
-            inv[r] = (uint16_t)at;
+            inv[r] = (uint16_t)(((s % L.cs) * loc + s / L.cs) * 32 + (at & 31));
             lo[at] = (uint8_t)n;
         }
     }
@@ -144,7 +148,10 @@ int res_plan(const int32_t* ptrA, const int32_t* ptrAt, int64_t m, int64_t n, in
     if (single && nnz >= RES_SINGLE_CLUSTER_NNZ) cs = RES_MAX_CS;
     r.m = (int32_t)m;
     r.n = (int32_t)n;
-    for (; cs <= RES_MAX_CS; cs *= 2) {
+    // every rank needs a slice of both matrices: the parts it sends tell the
+    // others that it is done with what it received (see ResWait)
+    while (cs > 1 && cs > std::min(res_slices(r.m), res_slices(r.n))) cs /= 2;
+    for (; cs <= RES_MAX_CS && (cs == 1 || cs <= std::min(res_slices(r.m), res_slices(r.n))); cs *= 2) {
         r.cs = cs;
         // a lower bound first: the unpadded entries
         if ((double)nnz * 2.0 * (2 + sv) > (double)RES_MAX_SMEM * cs) continue;

@@ -33,9 +33,9 @@
 
 namespace cpdlp {
 
-constexpr int RES_MAX_DIM = 65535;
+constexpr int RES_MAX_DIM = 65000;      // padded to whole slices per rank: 16-bit indices
 constexpr int RES_MAX_CS = 8;            // portable cluster size
-constexpr uint32_t RES_MAX_SMEM = 222 * 1024;  // dynamic shared memory of a CTA
+constexpr uint32_t RES_MAX_SMEM = 212 * 1024;  // dynamic shared memory of a CTA
 constexpr int RES_COEF = 128;            // averaging coefficients computed at a time
 // LPs with at least this many nonzeros take a whole cluster: in a batch with
 // FP64 iterates, and alone with either type
@@ -97,16 +97,17 @@ __host__ __device__ inline ResLayout res_layout(const ResLP& r) {
     };
     o.valA = take((uint32_t)r.capA * 32u * (uint32_t)sizeof(T));
     o.valAt = take((uint32_t)r.capAt * 32u * (uint32_t)sizeof(T));
-    // step: y (m) | xbar (n) whole, x xa c lv uv of the own columns, ya lc uc
-    // of the own rows; power method (FP64): x (n) | Ax (m) whole, A'Ax own
-    const uint32_t step = (((uint32_t)(r.m + r.n) + 7u) / 4u * 4u + 32u * (5u * lc + 3u * lr)) *
-                          (uint32_t)sizeof(T);
-    const uint32_t power = ((uint32_t)(r.m + r.n) + 4u + 32u * lc) * 8u;
+    // step: y | xbar whole (each rank's slices in a block of its own), x xa c lv
+    // uv of the own columns, ya lc uc of the own rows; power method (FP64):
+    // x | Ax whole, A'Ax own
+    const uint32_t whole = 32u * (uint32_t)r.cs * (lr + lc);
+    const uint32_t step = (whole + 32u * (5u * lc + 3u * lr)) * (uint32_t)sizeof(T);
+    const uint32_t power = (whole + 32u * lc) * 8u;
     o.vec = take(step > power ? step : power);
     o.idxA = take((uint32_t)r.capA * 64u);
     o.idxAt = take((uint32_t)r.capAt * 64u);
-    o.offA = take((lr + 1u) * 2u);
-    o.offAt = take((lc + 1u) * 2u);
+    o.offA = take(lr * 4u);
+    o.offAt = take(lc * 4u);
     o.lenA = take(lr * 32u);
     o.lenAt = take(lc * 32u);
     o.total = p;
@@ -131,447 +132,683 @@ void res_build(ResStore<T>& st, const ResLP* lps_dev, int count, const int32_t* 
                const T* at_val, int64_t max_rows, cudaStream_t s);
 
 // ---------------------------------------------------------------------------
-// device side
+// device side.  Everything of the LP is addressed by byte offsets into the
+// dynamic shared memory (32-bit shared-memory instructions, one register an
+// address).  The geometry lives in shared memory too, and steps, checks and
+// the power method are functions of their own (not inlined), so that each has
+// the registers to itself: inlined into one kernel of 64 registers they spilled
+// 900 bytes and a step of a 60-row FP32 LP took 2.8 us.
 // ---------------------------------------------------------------------------
+extern __shared__ __align__(16) unsigned char res_smem[];
+
+template <class V>
+__device__ __forceinline__ V& sm_at(uint32_t off) {
+    return *reinterpret_cast<V*>(res_smem + off);
+}
 template <int CS>
 __device__ __forceinline__ int res_rank() {
     if constexpr (CS == 1) return 0;
     else return (int)cooperative_groups::this_cluster().block_rank();
 }
+// the two halves of a group barrier: work between them that touches only the
+// thread's own data overlaps the wait (one CTA: all of it in the second half)
+template <int CS>
+__device__ __forceinline__ void res_arrive() {
+    if constexpr (CS > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+template <int CS>
+__device__ __forceinline__ void res_wait() {
+    if constexpr (CS > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    else __syncthreads();
+}
 template <int CS>
 __device__ __forceinline__ void res_sync() {
-    if constexpr (CS == 1) __syncthreads();
-    else cooperative_groups::this_cluster().sync();
+    res_arrive<CS>();
+    res_wait<CS>();
 }
-// stores v at the same place of every CTA's shared memory
-template <int CS, class T>
-__device__ __forceinline__ void res_put(T* p, T v) {
-    if constexpr (CS == 1) *p = v;
-    else {
+__device__ __forceinline__ uint32_t smem_addr(const void* p) {
+    return (uint32_t)__cvta_generic_to_shared(p);
+}
+__device__ __forceinline__ uint32_t map_rank(uint32_t a, int rank) {
+    uint32_t b;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(b) : "r"(a), "r"(rank));
+    return b;
+}
+// stores v at the same place of every CTA's shared memory (ordered by the
+// group barrier that follows)
+template <int CS>
+__device__ __forceinline__ void res_put(double* p, double v, int rank) {
+    *p = v;
+    if constexpr (CS > 1) {
+        const uint32_t a = smem_addr(p);
 #pragma unroll
-        for (int q = 0; q < CS; q++) *cooperative_groups::this_cluster().map_shared_rank(p, q) = v;
+        for (int q = 0; q < CS; q++)
+            if (q != rank)
+                asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(map_rank(a, q)), "d"(v) : "memory");
     }
 }
 
-// one row of a slice: entries at ip/vp + 32 k, k < w (the slice's width); the
-// row's own length is len <= w, its padding has index 0
-template <class V, class T>
-__device__ __forceinline__ T slice_sum(const uint16_t* ip, const V* vp, int w, int len,
-                                       const T* vec) {
-    T s = T(0);
-    int k = 0;
-#pragma unroll 1
-    for (; k + 4 <= w; k += 4) {
-        T p[4];
+// ---- exchange of a gathered vector -------------------------------------------
+// Every CTA holds the whole vector, each rank's slices in a block of its own.
+// A warp that finished a slice stores it locally and sends its 128 or 256
+// bytes to every other CTA with 16-byte asynchronous stores that count
+// themselves on the receiver's mbarrier; a receiver waits until all bytes of
+// the other ranks are there.  Against plain remote stores and a cluster
+// barrier (whose release waits for the stores' acknowledgements) a half-step
+// on 8 CTAs loses 0.5 us of waiting.
+// No second barrier protects the readers of the vector: a rank sends its part
+// of y after it gathered the whole xbar for it, so a CTA that has all of y
+// knows that every CTA is done with xbar, and the other way round.  This, and
+// that no CTA's barrier sees bytes of a later phase, needs every rank to send
+// some of both vectors: res_plan gives each at least one slice of A and of A'.
+struct ResWait {
+    uint64_t bar[2];   // mbarriers: 0 for y (and Ax), 1 for xbar (and x)
+    int failed;        // a wait ran out (never, unless the kernel is wrong)
+};
+// one warp sends slice block p[0..32) (whole in local shared memory)
+template <int CS, class V>
+__device__ __forceinline__ void res_send(const V* p, uint64_t* bar, int rank) {
+    if constexpr (CS > 1) {
+        __syncwarp();
+        constexpr int CH = 32 * (int)sizeof(V) / 16;  // 16-byte chunks of a slice
+        const int lane = threadIdx.x & 31;
+        const uint32_t a = smem_addr(p), mb = smem_addr(bar);
 #pragma unroll
-        for (int u = 0; u < 4; u++) p[u] = mul_rn((T)vp[(k + u) * 32], vec[ip[(k + u) * 32]]);
+        for (int k = 0; k < CH * CS; k += 32) {
+            const int q = (k + lane) / CH, c = (k + lane) % CH;
+            if (q < CS && q != rank) {
+                const int4 v = reinterpret_cast<const int4*>(p)[c];
+                asm volatile(
+                    "st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(
+                        map_rank(a + 16u * (uint32_t)c, q)),
+                    "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w), "r"(map_rank(mb, q))
+                    : "memory");
+            }
+        }
+    }
+}
+// waits for `bytes` of the other ranks; parity: the barrier's phases so far,
+// modulo 2 (advanced).  Also a CTA barrier.
+template <int CS>
+__device__ __forceinline__ void res_receive(ResWait& W, int which, uint32_t bytes, unsigned& parity) {
+    __syncthreads();
+    if constexpr (CS > 1) {
+        const uint32_t mb = smem_addr(&W.bar[which]);
+        if (threadIdx.x == 0)
+            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(mb), "r"(bytes)
+                         : "memory");
+        const unsigned par = (parity >> which) & 1u;
+        uint32_t ok = 0;
+        for (int tries = 0; tries < (1 << 20); tries++) {
+            asm volatile(
+                "{\n\t.reg .pred p;\n\t"
+                "mbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+                "selp.u32 %0, 1, 0, p;\n\t}"
+                : "=r"(ok)
+                : "r"(mb), "r"(par)
+                : "memory");
+            if (ok || *(volatile int*)&W.failed) break;
+        }
+        if (!ok) W.failed = 1;
+        parity ^= 1u << which;
+    }
+}
+// before the first exchange (thread 0 of every CTA, then a group barrier)
+__device__ __forceinline__ void res_wait_init(ResWait& W) {
+    for (int k = 0; k < 2; k++)
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&W.bar[k])) : "memory");
+    W.failed = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+}
+
+// One row of a slice: entries at ip/vp + 32 k, k < w (the slice's width, uniform
+// over the warp); the row's own length is len <= w.  Its padding (index 0, value
+// 0) adds -0, which changes nothing, and costs no branch.
+// FP32: up to eight entries' loads are in flight together (straight code for
+// each remainder: guards around each entry's loads took 1.6 times as long); the
+// sum rounds each product and each addition like the tile engine.
+template <int N, class V>
+__device__ __forceinline__ float slice_chunk(const uint16_t* ip, const V* vp, int len,
+                                             const float* vec, float s) {
+    float p[N];
 #pragma unroll
-        for (int u = 0; u < 4; u++)
-            if (k + u < len) s = add_rn(s, p[u]);
-    }
-#pragma unroll 1
-    for (; k < w; k++) {
-        const T p = mul_rn((T)vp[k * 32], vec[ip[k * 32]]);
-        if (k < len) s = add_rn(s, p);
-    }
+    for (int u = 0; u < N; u++) p[u] = mul_rn(vp[u * 32], vec[ip[u * 32]]);
+#pragma unroll
+    for (int u = 0; u < N; u++) s = add_rn(s, u < len ? p[u] : -0.0f);
     return s;
 }
+template <class V>
+__device__ __forceinline__ float slice_sum(const uint16_t* ip, const V* vp, int w, int len,
+                                           const float* vec) {
+    float s = 0.0f;
+#pragma unroll 1
+    for (; w > 8; w -= 8, len -= 8, ip += 256, vp += 256) s = slice_chunk<8>(ip, vp, len, vec, s);
+    switch (w) {
+        case 8: return slice_chunk<8>(ip, vp, len, vec, s);
+        case 7: return slice_chunk<7>(ip, vp, len, vec, s);
+        case 6: return slice_chunk<6>(ip, vp, len, vec, s);
+        case 5: return slice_chunk<5>(ip, vp, len, vec, s);
+        case 4: return slice_chunk<4>(ip, vp, len, vec, s);
+        case 3: return slice_chunk<3>(ip, vp, len, vec, s);
+        case 2: return slice_chunk<2>(ip, vp, len, vec, s);
+        case 1: return slice_chunk<1>(ip, vp, len, vec, s);
+        default: return s;
+    }
+}
+// FP64: fused operations (one rounding where the product and the sum have two)
+// in column order, two entries' loads ahead.  A GB300 sub-partition starts one
+// FP64 instruction of a warp every 63 cycles (76 with all four busy), dependent
+// or not, so their number per sub-partition is what a step costs; a second
+// chain for every other entry only added one.
+template <class V>
+__device__ __forceinline__ double slice_sum(const uint16_t* ip, const V* vp, int w, int len,
+                                            const double* vec) {
+    double s = 0.0;
+    if (w & 1) {
+        s = __fma_rn((double)vp[0], len > 0 ? vec[ip[0]] : -0.0, -0.0);
+        ip += 32;
+        vp += 32;
+        w--;
+        len--;
+    }
+    if (w == 0) return s;
+    V v0 = vp[0], v1 = vp[32];
+    double g0 = vec[ip[0]], g1 = vec[ip[32]];
+#pragma unroll 1
+    for (;;) {
+        const double a0 = (double)v0, a1 = (double)v1, b0 = len > 0 ? g0 : -0.0,
+                     b1 = len > 1 ? g1 : -0.0;
+        w -= 2;
+        if (w > 0) {
+            ip += 64;
+            vp += 64;
+            len -= 2;
+            v0 = vp[0];
+            v1 = vp[32];
+            g0 = vec[ip[0]];
+            g1 = vec[ip[32]];
+        }
+        s = __fma_rn(a0, b0, s);
+        s = __fma_rn(a1, b1, s);
+        if (w <= 0) return s;
+    }
+}
+// a*b + c: rounded twice (FP32, as the tile kernels) or once (FP64)
+__device__ __forceinline__ float mul_add(float a, float b, float c) { return add_rn(mul_rn(a, b), c); }
+__device__ __forceinline__ double mul_add(double a, double b, double c) { return __fma_rn(a, b, c); }
 
-// Sums Q <= 8 values per thread over the group; every thread gets the sums.
-// A warp's first three exchanges halve the number of values a lane carries
-// (9 additions a lane instead of 5 Q: FP64 additions are what this costs),
-// then warps and ranks are added in order.  sh: NW * 8 + 8 doubles.
+constexpr int RES_SUMS = 5;  // most values of one sum
+// Sums Q <= RES_SUMS values per thread over the group; every thread gets the
+// sums.  FP64 additions are what this costs (64 cycles each, one after the
+// other), so few of them are in a row: a warp's first exchanges halve the
+// number of values a lane carries (9 additions a lane for 5 values instead of
+// 25), every warp stores its sums into every CTA, and after one group barrier
+// warp q of each CTA adds value q of all warps of the group with a tree.  The
+// order depends on the group's shape alone.
+// sh: res_sh<CS, NW>() doubles; `phase` alternates the halves, so that a fast
+// CTA's next sums do not meet a slow one's reads.
+template <int CS, int NW>
+constexpr int res_sh() { return 2 * RES_SUMS * CS * NW + 8; }
 template <int Q, int CS, int NW>
-__device__ __forceinline__ void res_sum(double (&v)[Q], double* sh) {
+__device__ __forceinline__ void res_sum(double (&v)[Q], double* sh, int& phase) {
+    static_assert(Q <= RES_SUMS && Q <= NW, "a warp per value");
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    double a[8];
+    constexpr int P = CS * NW;  // warps of the group
+    double* slot = sh + 8 + phase * (RES_SUMS * P);
+    phase ^= 1;
+    double d;
+    int which;
+    if constexpr (Q <= 4) {
+        double a[4], c[2];
 #pragma unroll
-    for (int q = 0; q < 8; q++) a[q] = q < Q ? v[q < Q ? q : 0] : 0.0;
-    double b[4], c[2], d;
-    {
-        const bool h = lane & 16;
+        for (int q = 0; q < 4; q++) a[q] = q < Q ? v[q < Q ? q : 0] : 0.0;
+        const bool h = lane & 16, h2 = lane & 8;
+#pragma unroll
+        for (int q = 0; q < 2; q++) {
+            const double send = h ? a[q] : a[q + 2], keep = h ? a[q + 2] : a[q];
+            c[q] = keep + __shfl_xor_sync(FULL_MASK, send, 16);
+        }
+        const double send = h2 ? c[0] : c[1], keep = h2 ? c[1] : c[0];
+        d = keep + __shfl_xor_sync(FULL_MASK, send, 8);
+        d += __shfl_xor_sync(FULL_MASK, d, 4);
+        which = (h ? 2 : 0) + (h2 ? 1 : 0);
+    } else {
+        double a[8], b[4], c[2];
+#pragma unroll
+        for (int q = 0; q < 8; q++) a[q] = q < Q ? v[q < Q ? q : 0] : 0.0;
+        const bool h = lane & 16, h2 = lane & 8, h3 = lane & 4;
 #pragma unroll
         for (int q = 0; q < 4; q++) {
             const double send = h ? a[q] : a[q + 4], keep = h ? a[q + 4] : a[q];
             b[q] = keep + __shfl_xor_sync(FULL_MASK, send, 16);
         }
-    }
-    {
-        const bool h = lane & 8;
 #pragma unroll
         for (int q = 0; q < 2; q++) {
-            const double send = h ? b[q] : b[q + 2], keep = h ? b[q + 2] : b[q];
+            const double send = h2 ? b[q] : b[q + 2], keep = h2 ? b[q + 2] : b[q];
             c[q] = keep + __shfl_xor_sync(FULL_MASK, send, 8);
         }
-    }
-    {
-        const bool h = lane & 4;
-        const double send = h ? c[0] : c[1], keep = h ? c[1] : c[0];
+        const double send = h3 ? c[0] : c[1], keep = h3 ? c[1] : c[0];
         d = keep + __shfl_xor_sync(FULL_MASK, send, 4);
+        which = (h ? 4 : 0) + (h2 ? 2 : 0) + (h3 ? 1 : 0);
     }
     d += __shfl_xor_sync(FULL_MASK, d, 2);
     d += __shfl_xor_sync(FULL_MASK, d, 1);
-    // lane bits 4, 3, 2 chose values +4, +2, +1
-    if ((lane & 3) == 0) sh[w * 8 + ((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1)] = d;
-    __syncthreads();
-    if (threadIdx.x < Q) {
-        double s = 0.0;
-        for (int ww = 0; ww < NW; ww++) s += sh[ww * 8 + threadIdx.x];
-        sh[NW * 8 + threadIdx.x] = s;
-    }
+    const int rank = res_rank<CS>();
+    if ((lane & (Q <= 4 ? 7 : 3)) == 0 && which < Q)
+        res_put<CS>(slot + which * P + rank * NW + w, d, rank);
+    __syncwarp();
     res_sync<CS>();
+    if (w < Q) {
+        double s = 0.0;
 #pragma unroll
-    for (int q = 0; q < Q; q++) {
-        if constexpr (CS == 1) v[q] = sh[NW * 8 + q];
-        else {
-            double s = cooperative_groups::this_cluster().map_shared_rank(sh, 0)[NW * 8 + q];
-            for (int r = 1; r < CS; r++)
-                s += cooperative_groups::this_cluster().map_shared_rank(sh, r)[NW * 8 + q];
-            v[q] = s;
+        for (int k = 0; k < (P + 31) / 32; k++)
+            if (k * 32 + lane < P) s = k ? s + slot[w * P + k * 32 + lane] : slot[w * P + lane];
+#pragma unroll
+        for (int o = (P < 32 ? P : 32) / 2; o > 0; o >>= 1) s += __shfl_xor_sync(FULL_MASK, s, o);
+        if (lane == 0) sh[w] = s;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < Q; q++) v[q] = sh[q];
+    // sh[0..7] are rewritten only after the next call's group barrier
+}
+
+// the resident LP as one CTA of its group sees it (in shared memory)
+struct ResGeo {
+    ResLP R;
+    int rank;
+    int LA, LAt;                  // own slices of A's and A''s rows
+    int baseA, baseAt;            // place of the own block in a gathered vector
+    uint32_t remA, remAt;         // rows in the other ranks' slices (with padding)
+    ResLayout o;
+    uint32_t y, xb;               // gathered vectors, whole
+    uint32_t x, xa, c, lv, uv;    // own columns
+    uint32_t ya, lc, uc;          // own rows
+    uint32_t px, ps, pax;         // the power method's vectors
+    const int32_t *ordA, *ordAt;  // global: slice row -> row of the LP
+    const uint16_t *invA, *invAt;
+};
+// averaging coefficients of the next steps and the weight sum (shared memory)
+template <class T>
+struct ResCoefs {
+    T a[RES_COEF], b[RES_COEF];
+    double es;
+};
+// where the last step of a block leaves sol, sol_last and the averages
+template <class T>
+struct ResDump {
+    T *x, *xl, *xa, *xal, *y, *yl, *ya, *yal;
+};
+struct ResPower {
+    double theta, residual;
+    int64_t it;
+    bool stop;
+};
+
+// f(l, r) for each own slice l of this warp and this lane's row r of it
+template <int CS, int NT, class F>
+__device__ __forceinline__ void res_rows(int slices, int rank, int rows, F&& f) {
+    const int lane = threadIdx.x & 31;
+    for (int l = threadIdx.x >> 5; l < slices; l += NT / 32) {
+        const int r = (l * CS + rank) * 32 + lane;
+        if (r < rows) f(l * 32 + lane, r);
+    }
+}
+
+template <class T, int CS, int NT>
+__device__ void res_load_side(const ResGeo& G, const int32_t* meta, int rows, int L,
+                              const uint16_t* gi, const T* gv, const uint8_t* gl, uint32_t sv,
+                              uint32_t si, uint32_t so, uint32_t sl) {
+    const int rank = G.rank;
+    const int32_t start = meta[rank], units = meta[rank + 1] - start;
+    const int ns = res_slices(rows);
+    int list = CS + 1;  // this rank's offsets follow those of the lower ranks
+    for (int q = 0; q < rank; q++) list += (ns - q + CS - 1) / CS + 1;
+    // 32 entries are 64 bytes of indices and 128 or 256 bytes of values
+    const int4* a = reinterpret_cast<const int4*>(gi + (int64_t)start * 32);
+    const int4* b = reinterpret_cast<const int4*>(gv + (int64_t)start * 32);
+    for (int k = threadIdx.x; k < units * 4; k += NT) (&sm_at<int4>(si))[k] = __ldg(a + k);
+    for (int k = threadIdx.x; k < units * (int)(2 * sizeof(T)); k += NT)
+        (&sm_at<int4>(sv))[k] = __ldg(b + k);
+    // offset (units of 32 entries) and width of each slice in one word
+    for (int k = threadIdx.x; k < L; k += NT)
+        (&sm_at<uint32_t>(so))[k] = (uint32_t)meta[list + k] << 8 | (uint32_t)(meta[list + k + 1] - meta[list + k]);
+    for (int k = threadIdx.x; k < L * 32; k += NT) {
+        const int r = ((k >> 5) * CS + rank) * 32 + (k & 31);
+        (&sm_at<uint8_t>(sl))[k] = r < rows ? gl[r] : 0;
+    }
+}
+// the geometry and the matrices of LP r; ends with a CTA barrier
+template <class T, int CS, int NT>
+__device__ __noinline__ void res_load(ResGeo& G, const ResLP& r, const ResView<T>& g) {
+    if (threadIdx.x == 0) {
+        G.R = r;
+        G.rank = res_rank<CS>();
+        G.LA = (res_slices(r.m) - G.rank + CS - 1) / CS;
+        G.LAt = (res_slices(r.n) - G.rank + CS - 1) / CS;
+        G.o = res_layout<T>(r);
+        const uint32_t S = sizeof(T), cols = 32u * S * (uint32_t)res_local(r.n, CS),
+                       rows = 32u * S * (uint32_t)res_local(r.m, CS);
+        G.baseA = G.rank * res_local(r.m, CS) * 32;
+        G.baseAt = G.rank * res_local(r.n, CS) * 32;
+        G.remA = 32u * (uint32_t)(res_slices(r.m) - G.LA);
+        G.remAt = 32u * (uint32_t)(res_slices(r.n) - G.LAt);
+        G.y = G.o.vec;
+        G.xb = G.y + CS * rows;
+        G.x = G.xb + CS * cols;
+        G.xa = G.x + cols;
+        G.c = G.xa + cols;
+        G.lv = G.c + cols;
+        G.uv = G.lv + cols;
+        G.ya = G.uv + cols;
+        G.lc = G.ya + rows;
+        G.uc = G.lc + rows;
+        G.px = G.o.vec;
+        G.ps = G.px + CS * 256u * (uint32_t)res_local(r.n, CS);
+        G.pax = G.ps + CS * 256u * (uint32_t)res_local(r.m, CS);
+        G.ordA = g.ordA + r.row_off;
+        G.ordAt = g.ordAt + r.col_off;
+        G.invA = g.invA + r.row_off;
+        G.invAt = g.invAt + r.col_off;
+    }
+    __syncthreads();
+    res_load_side<T, CS, NT>(G, g.metaA + r.mA, r.m, G.LA, g.idxA + r.eA, g.valA + r.eA,
+                             g.lenA + r.row_off, G.o.valA, G.o.idxA, G.o.offA, G.o.lenA);
+    res_load_side<T, CS, NT>(G, g.metaAt + r.mAt, r.n, G.LAt, g.idxAt + r.eAt, g.valAt + r.eAt,
+                             g.lenAt + r.col_off, G.o.valAt, G.o.idxAt, G.o.offAt, G.o.lenAt);
+    __syncthreads();
+}
+// costs and bounds of the own rows and columns (global vectors of the LP)
+template <class T, int CS, int NT>
+__device__ __noinline__ void res_bounds(const ResGeo& G, const T* gc, const T* glv, const T* guv,
+                                        const T* glc, const T* guc) {
+    res_rows<CS, NT>(G.LAt, G.rank, G.R.n, [&](int k, int r) {
+        const int j = G.ordAt[r];
+        (&sm_at<T>(G.c))[k] = gc[j];
+        (&sm_at<T>(G.lv))[k] = glv[j];
+        (&sm_at<T>(G.uv))[k] = guv[j];
+    });
+    res_rows<CS, NT>(G.LA, G.rank, G.R.m, [&](int k, int r) {
+        const int i = G.ordA[r];
+        (&sm_at<T>(G.lc))[k] = glc[i];
+        (&sm_at<T>(G.uc))[k] = guc[i];
+    });
+}
+// whole vectors of the LP (global, the LP's order) into the gathered copies
+template <class T, int NT>
+__device__ __forceinline__ void res_load_y(const ResGeo& G, const T* gy) {
+    T* y = &sm_at<T>(G.y);
+    for (int i = threadIdx.x; i < G.R.m; i += NT) y[G.invA[i]] = __ldcg(gy + i);
+}
+template <class T, int NT>
+__device__ __forceinline__ void res_load_xb(const ResGeo& G, const T* gx) {
+    T* xb = &sm_at<T>(G.xb);
+    for (int j = threadIdx.x; j < G.R.n; j += NT) xb[G.invAt[j]] = __ldcg(gx + j);
+}
+// sol and the average (null: zero) of the own rows and columns, and y whole
+template <class T, int CS, int NT>
+__device__ __noinline__ void res_load_iterate(const ResGeo& G, const T* gx, const T* gxa,
+                                              const T* gy, const T* gya) {
+    res_rows<CS, NT>(G.LAt, G.rank, G.R.n, [&](int k, int r) {
+        (&sm_at<T>(G.x))[k] = __ldcg(gx + G.ordAt[r]);
+        (&sm_at<T>(G.xa))[k] = gxa ? __ldcg(gxa + G.ordAt[r]) : T(0);
+    });
+    res_rows<CS, NT>(G.LA, G.rank, G.R.m, [&](int k, int r) {
+        (&sm_at<T>(G.ya))[k] = gya ? __ldcg(gya + G.ordA[r]) : T(0);
+    });
+    res_load_y<T, NT>(G, gy);
+}
+
+// `count` steps (pdlp.jl:96-136); FP32: the arithmetic of PrimalEpi and
+// DualEpi, FP64: the same with fused operations.  tab.es: the weight sum,
+// advanced (averaging only).  The last step also writes both iterates and both
+// averages to d; ends with a group barrier.
+template <class T, int CS, int NT>
+__device__ __noinline__ void res_steps(const ResGeo& G, double eta, double omega, int count,
+                                       bool avg, ResCoefs<T>& tab, const ResDump<T>& d, ResWait& W,
+                                       unsigned& parity_io) {
+    constexpr int NW = NT / 32;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, rank = G.rank;
+    const int LA = G.LA, LAt = G.LAt, m = G.R.m, n = G.R.n;
+    const T *valA = &sm_at<T>(G.o.valA) + lane, *valAt = &sm_at<T>(G.o.valAt) + lane;
+    const uint16_t *idxA = &sm_at<uint16_t>(G.o.idxA) + lane, *idxAt = &sm_at<uint16_t>(G.o.idxAt) + lane;
+    const uint32_t *offA = &sm_at<uint32_t>(G.o.offA), *offAt = &sm_at<uint32_t>(G.o.offAt);
+    const uint8_t *lenA = &sm_at<uint8_t>(G.o.lenA) + lane, *lenAt = &sm_at<uint8_t>(G.o.lenAt) + lane;
+    const T *y = &sm_at<T>(G.y), *xb = &sm_at<T>(G.xb);
+    T *yown = &sm_at<T>(G.y) + G.baseA, *xbown = &sm_at<T>(G.xb) + G.baseAt;
+    T *x = &sm_at<T>(G.x) + lane, *xa = &sm_at<T>(G.xa) + lane, *ya = &sm_at<T>(G.ya) + lane;
+    const T *c = &sm_at<T>(G.c) + lane, *lv = &sm_at<T>(G.lv) + lane, *uv = &sm_at<T>(G.uv) + lane;
+    const T *lc = &sm_at<T>(G.lc) + lane, *uc = &sm_at<T>(G.uc) + lane;
+    unsigned parity = parity_io;
+    const double sg = eta * omega;
+    const T tau = (T)(eta / omega), sigma = (T)sg, inv_sigma = (T)(1.0 / sg);
+    for (int k0 = 0; k0 < count; k0 += RES_COEF) {
+        const int nk = min(count - k0, RES_COEF);
+        if (avg) {
+            // eta/(eta+es), es/(eta+es) of all nk steps at once, es growing by
+            // eta a step (a chain of additions, like the host's): a division
+            // a step by one thread would be longer than the step
+            __syncthreads();
+            const double es = tab.es;
+            __syncthreads();
+            for (int t = threadIdx.x; t < nk; t += NT) {
+                double e = es;
+                for (int q = 0; q < t; q++) e += eta;
+                tab.a[t] = (T)(eta / (eta + e));
+                tab.b[t] = (T)(e / (eta + e));
+                if (t == nk - 1) tab.es = e + eta;
+            }
+            __syncthreads();
+        }
+#pragma unroll 1
+        for (int st = 0; st < nk; st++) {
+            const bool last = k0 + st == count - 1;
+#pragma unroll 1
+            for (int l = w; l < LAt; l += NW) {
+                const int k = l * 32, r = (l * CS + rank) * 32 + lane;
+                const uint32_t o = offAt[l];
+                const T xo = x[k], cj = c[k], lo = lv[k], up = uv[k];
+                const T s = slice_sum(idxAt + (o >> 8) * 32, valAt + (o >> 8) * 32, (int)(o & 255u),
+                                      lenAt[k], y);
+                const T xp = proj_box(mul_add(-tau, sub_rn(cj, s), xo), lo, up);
+                xbown[k + lane] = extrapolate(xp, xo);
+                x[k] = xp;
+                res_send<CS>(xbown + k, &W.bar[1], rank);
+                if (last && r < n) {
+                    d.x[G.ordAt[r]] = xp;
+                    d.xl[G.ordAt[r]] = xo;
+                }
+            }
+            // the averages are formed while the others' parts arrive
+            if (avg) {
+                const T a = tab.a[st], b = tab.b[st];
+#pragma unroll 1
+                for (int l = w; l < LAt; l += NW) {
+                    const int k = l * 32, r = (l * CS + rank) * 32 + lane;
+                    const T xao = xa[k], xan = mul_add(x[k], a, mul_rn(xao, b));
+                    xa[k] = xan;
+                    if (last && r < n) {
+                        d.xa[G.ordAt[r]] = xan;
+                        d.xal[G.ordAt[r]] = xao;
+                    }
+                }
+            }
+            res_receive<CS>(W, 1, G.remAt * (uint32_t)sizeof(T), parity);
+#pragma unroll 1
+            for (int l = w; l < LA; l += NW) {
+                const int k = l * 32, r = (l * CS + rank) * 32 + lane;
+                const uint32_t o = offA[l];
+                const T yo = yown[k + lane], lo = lc[k], up = uc[k];
+                const T s = slice_sum(idxA + (o >> 8) * 32, valA + (o >> 8) * 32, (int)(o & 255u),
+                                      lenA[k], xb);
+                const T t2 = mul_add(-sigma, s, yo);
+                const T t4 = mul_add(inv_sigma, yo, -s);
+                const T yp = mul_add(-sigma, proj_box(t4, -up, -lo), t2);
+                yown[k + lane] = yp;
+                res_send<CS>(yown + k, &W.bar[0], rank);
+                if (last && r < m) {
+                    d.y[G.ordA[r]] = yp;
+                    d.yl[G.ordA[r]] = yo;
+                }
+            }
+            if (avg) {
+                const T a = tab.a[st], b = tab.b[st];
+#pragma unroll 1
+                for (int l = w; l < LA; l += NW) {
+                    const int k = l * 32, r = (l * CS + rank) * 32 + lane;
+                    const T yao = ya[k], yan = mul_add(yown[k + lane], a, mul_rn(yao, b));
+                    ya[k] = yan;
+                    if (last && r < m) {
+                        d.ya[G.ordA[r]] = yan;
+                        d.yal[G.ordA[r]] = yao;
+                    }
+                }
+            }
+            res_receive<CS>(W, 0, G.remA * (uint32_t)sizeof(T), parity);
         }
     }
+    parity_io = parity;
+    // a check reads what the other CTAs dumped, and overwrites y and xbar
     res_sync<CS>();
 }
 
-// the resident LP as one CTA of its group sees it
+// FP64 sums of the KKT terms of one iterate (gx, gy): v = {primal^2, row
+// objective, dual^2, column objective, c'x}; overwrites the gathered copies
+// y and xb
 template <class T, int CS, int NT>
-struct ResCtx {
-    static constexpr int NW = NT / 32;
-    ResLP R;
-    int rank, lane, w;
-    int LA, LAt;                  // own slices of A's and A''s rows
-    int locA, locAt;              // slices of the fullest rank (vector strides)
-    const T *valA, *valAt;
-    const uint16_t *idxA, *idxAt, *offA, *offAt;
-    const uint8_t *lenA, *lenAt;
-    T *y, *xb;                    // gathered vectors, whole
-    T *x, *xa, *c, *lv, *uv;      // own columns
-    T *ya, *lc, *uc;              // own rows
-    double *px, *ps, *pax;        // the power method's vectors
-    const int32_t *ordA, *ordAt;  // global: slice row -> row of the LP
-    const uint16_t *invA, *invAt;
-
-    // reads the matrices into shared memory; ends with a CTA barrier
-    __device__ void load(const ResLP& r, const ResView<T>& g, unsigned char* sm) {
-        R = r;
-        rank = res_rank<CS>();
-        lane = threadIdx.x & 31;
-        w = threadIdx.x >> 5;
-        const ResLayout o = res_layout<T>(r);
-        locA = res_local(r.m, CS);
-        locAt = res_local(r.n, CS);
-        LA = (res_slices(r.m) - rank + CS - 1) / CS;
-        LAt = (res_slices(r.n) - rank + CS - 1) / CS;
-        one(g.metaA + r.mA, r.m, LA, g.idxA + r.eA, g.valA + r.eA, g.lenA + r.row_off,
-            sm + o.valA, sm + o.idxA, sm + o.offA, sm + o.lenA);
-        one(g.metaAt + r.mAt, r.n, LAt, g.idxAt + r.eAt, g.valAt + r.eAt, g.lenAt + r.col_off,
-            sm + o.valAt, sm + o.idxAt, sm + o.offAt, sm + o.lenAt);
-        valA = reinterpret_cast<const T*>(sm + o.valA);
-        valAt = reinterpret_cast<const T*>(sm + o.valAt);
-        idxA = reinterpret_cast<const uint16_t*>(sm + o.idxA);
-        idxAt = reinterpret_cast<const uint16_t*>(sm + o.idxAt);
-        offA = reinterpret_cast<const uint16_t*>(sm + o.offA);
-        offAt = reinterpret_cast<const uint16_t*>(sm + o.offAt);
-        lenA = sm + o.lenA;
-        lenAt = sm + o.lenAt;
-        T* v = reinterpret_cast<T*>(sm + o.vec);
-        y = v;
-        xb = v + (r.m + 3) / 4 * 4;
-        x = v + (r.m + r.n + 7) / 4 * 4;
-        xa = x + 32 * locAt;
-        c = xa + 32 * locAt;
-        lv = c + 32 * locAt;
-        uv = lv + 32 * locAt;
-        ya = uv + 32 * locAt;
-        lc = ya + 32 * locA;
-        uc = lc + 32 * locA;
-        px = reinterpret_cast<double*>(sm + o.vec);
-        ps = px + (r.n + 1) / 2 * 2;
-        pax = ps + (r.m + 1) / 2 * 2;
-        ordA = g.ordA + r.row_off;
-        ordAt = g.ordAt + r.col_off;
-        invA = g.invA + r.row_off;
-        invAt = g.invAt + r.col_off;
-        __syncthreads();
-    }
-    __device__ void one(const int32_t* meta, int rows, int L, const uint16_t* gi, const T* gv,
-                        const uint8_t* gl, unsigned char* sv, unsigned char* si,
-                        unsigned char* so, unsigned char* sl) {
-        const int32_t start = meta[rank], units = meta[rank + 1] - start;
-        const int ns = res_slices(rows);
-        int list = CS + 1;  // this rank's offsets follow those of the lower ranks
-        for (int q = 0; q < rank; q++) list += (ns - q + CS - 1) / CS + 1;
-        // 32 entries are 64 bytes of indices and 128 or 256 bytes of values
-        const int4* a = reinterpret_cast<const int4*>(gi + (int64_t)start * 32);
-        const int4* b = reinterpret_cast<const int4*>(gv + (int64_t)start * 32);
-        for (int k = threadIdx.x; k < units * 4; k += NT) reinterpret_cast<int4*>(si)[k] = __ldg(a + k);
-        for (int k = threadIdx.x; k < units * (int)(2 * sizeof(T)); k += NT)
-            reinterpret_cast<int4*>(sv)[k] = __ldg(b + k);
-        for (int k = threadIdx.x; k <= L; k += NT)
-            reinterpret_cast<uint16_t*>(so)[k] = (uint16_t)meta[list + k];
-        for (int k = threadIdx.x; k < L * 32; k += NT) {
-            const int r = ((k >> 5) * CS + rank) * 32 + (k & 31);
-            sl[k] = r < rows ? gl[r] : 0;
-        }
-    }
-
-    // own slice l of a matrix: its rows are r = row(l)
-    __device__ __forceinline__ int row(int l) const { return (l * CS + rank) * 32 + lane; }
-    template <class VT>
-    __device__ __forceinline__ VT sumA(int l, const VT* vec) const {
-        const int o = offA[l];
-        return slice_sum(idxA + o * 32 + lane, valA + o * 32 + lane, offA[l + 1] - o,
-                         lenA[l * 32 + lane], vec);
-    }
-    template <class VT>
-    __device__ __forceinline__ VT sumAt(int l, const VT* vec) const {
-        const int o = offAt[l];
-        return slice_sum(idxAt + o * 32 + lane, valAt + o * 32 + lane, offAt[l + 1] - o,
-                         lenAt[l * 32 + lane], vec);
-    }
-
-    // costs and bounds of the own rows and columns (global vectors of the LP)
-    __device__ void load_bounds(const T* gc, const T* glv, const T* guv, const T* glc, const T* guc) {
-        for (int l = w; l < LAt; l += NW) {
-            const int r = row(l);
-            if (r < R.n) {
-                const int j = ordAt[r];
-                c[l * 32 + lane] = gc[j];
-                lv[l * 32 + lane] = glv[j];
-                uv[l * 32 + lane] = guv[j];
-            }
-        }
-        for (int l = w; l < LA; l += NW) {
-            const int r = row(l);
-            if (r < R.m) {
-                const int i = ordA[r];
-                lc[l * 32 + lane] = glc[i];
-                uc[l * 32 + lane] = guc[i];
-            }
-        }
-    }
-    // whole vectors of the LP into the gathered copies
-    __device__ void load_y(const T* gy) {
-        for (int i = threadIdx.x; i < R.m; i += NT) y[invA[i]] = __ldcg(gy + i);
-    }
-    __device__ void load_xb(const T* gx) {
-        for (int j = threadIdx.x; j < R.n; j += NT) xb[invAt[j]] = __ldcg(gx + j);
-    }
-    __device__ void load_x(const T* gx) {
-        for (int l = w; l < LAt; l += NW) {
-            const int r = row(l);
-            if (r < R.n) x[l * 32 + lane] = __ldcg(gx + ordAt[r]);
-        }
-    }
-    __device__ void load_xa(const T* gx) {
-        for (int l = w; l < LAt; l += NW) {
-            const int r = row(l);
-            if (r < R.n) xa[l * 32 + lane] = gx ? __ldcg(gx + ordAt[r]) : T(0);
-        }
-    }
-    __device__ void load_ya(const T* gy) {
-        for (int l = w; l < LA; l += NW) {
-            const int r = row(l);
-            if (r < R.m) ya[l * 32 + lane] = gy ? __ldcg(gy + ordA[r]) : T(0);
-        }
-    }
-
-    // where the last step of a block leaves sol, sol_last and the averages
-    struct Dump {
-        T *x, *xl, *xa, *xal, *y, *yl, *ya, *yal;
-    };
-
-    // One step! (pdlp.jl:96-136), the arithmetic of PrimalEpi and DualEpi.
-    // `last`: also write both iterates and both averages to d.
-    __device__ __forceinline__ void step(T tau, T sigma, T inv_sigma, T a, T b, bool avg, bool last,
-                                         const Dump& d) {
-        for (int l = w; l < LAt; l += NW) {
-            const T s = sumAt(l, y);
-            const int r = row(l), k = l * 32 + lane;
-            if (r < R.n) {
-                const T xo = x[k];
-                const T xp = proj_box(sub_rn(xo, mul_rn(tau, sub_rn(c[k], s))), lv[k], uv[k]);
-                res_put<CS>(xb + r, sub_rn(mul_rn(T(2), xp), xo));
-                x[k] = xp;
-                T xao = T(0), xan = T(0);
-                if (avg) {
-                    xao = xa[k];
-                    xan = add_rn(mul_rn(xp, a), mul_rn(xao, b));
-                    xa[k] = xan;
-                }
-                if (last) {
-                    const int j = ordAt[r];
-                    d.x[j] = xp;
-                    d.xl[j] = xo;
-                    if (avg) {
-                        d.xa[j] = xan;
-                        d.xal[j] = xao;
-                    }
-                }
-            }
-        }
-        res_sync<CS>();
-        for (int l = w; l < LA; l += NW) {
-            const T s = sumA(l, xb);
-            const int r = row(l), k = l * 32 + lane;
-            if (r < R.m) {
-                const T yo = y[r];
-                const T t2 = sub_rn(yo, mul_rn(sigma, s));
-                const T t4 = sub_rn(mul_rn(inv_sigma, yo), s);
-                const T yp = sub_rn(t2, mul_rn(sigma, proj_box(t4, -uc[k], -lc[k])));
-                res_put<CS>(y + r, yp);
-                T yao = T(0), yan = T(0);
-                if (avg) {
-                    yao = ya[k];
-                    yan = add_rn(mul_rn(yp, a), mul_rn(yao, b));
-                    ya[k] = yan;
-                }
-                if (last) {
-                    const int i = ordA[r];
-                    d.y[i] = yp;
-                    d.yl[i] = yo;
-                    if (avg) {
-                        d.ya[i] = yan;
-                        d.yal[i] = yao;
-                    }
-                }
-            }
-        }
-        res_sync<CS>();
-    }
-
-    // averaging coefficients of the next `count` <= RES_COEF steps from the
-    // weight sum tab.es (pdlp.jl:126-136): eta/(eta+es), es/(eta+es), es growing
-    // by eta a step (a chain of additions, like the host's).  Computed ahead for
-    // all steps at once: an FP64 division a step by one thread, as the step
-    // loop over global memory has it, would be longer than the step.
-    struct Coefs {
-        T a[RES_COEF], b[RES_COEF];
-        double es;
-    };
-    __device__ void coefs(double eta, int count, Coefs& tab) {
-        __syncthreads();
-        const double es = tab.es;
-        __syncthreads();
-        for (int t = threadIdx.x; t < count; t += NT) {
-            double e = es;
-            for (int q = 0; q < t; q++) e += eta;
-            tab.a[t] = (T)(eta / (eta + e));
-            tab.b[t] = (T)(e / (eta + e));
-            if (t == count - 1) tab.es = e + eta;
-        }
-        __syncthreads();
-    }
-
-    // `count` steps; tab.es: the weight sum, advanced (averaging only)
-    __device__ void steps(double eta, double omega, int count, bool avg, Coefs& tab, const Dump& d) {
-        const double sg = eta * omega;
-        const T tau = (T)(eta / omega), sigma = (T)sg, inv_sigma = (T)(1.0 / sg);
-        for (int k0 = 0; k0 < count; k0 += RES_COEF) {
-            const int nk = min(count - k0, RES_COEF);
-            if (avg) coefs(eta, nk, tab);
-            for (int k = 0; k < nk; k++)
-                step(tau, sigma, inv_sigma, avg ? tab.a[k] : T(0), avg ? tab.b[k] : T(0), avg,
-                     k0 + k == count - 1, d);
-        }
-    }
-
-    // FP64 sums of the KKT terms of one iterate (gx, gy), v = {primal^2,
-    // row objective, dual^2, column objective, c'x}; overwrites the gathered
-    // copies y and xb
-    __device__ void kkt(const T* gx, const T* gy, const T* invD1, const T* invD2, double (&v)[5],
-                        double* sh) {
-        load_xb(gx);
-        load_y(gy);
-        __syncthreads();
-#pragma unroll
-        for (int q = 0; q < 5; q++) v[q] = 0.0;
-        for (int l = w; l < LA; l += NW) {
-            const T s = sumA(l, xb);
-            const int r = row(l), k = l * 32 + lane;
-            if (r < R.m) {
-                const T lo = lc[k], up = uc[k], yy = y[r];
-                const double dd = (double)mul_rn(invD1[ordA[r]], sub_rn(s, proj_box(s, lo, up)));
+__device__ __noinline__ void res_kkt_sums(const ResGeo& G, const T* gx, const T* gy, const T* invD1,
+                                          const T* invD2, double (&out)[5], double* sh, int& phase) {
+    const int lane = threadIdx.x & 31;
+    res_load_xb<T, NT>(G, gx);
+    res_load_y<T, NT>(G, gy);
+    __syncthreads();
+    const T *y = &sm_at<T>(G.y), *xb = &sm_at<T>(G.xb);
+    double v[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+    {
+        const T *val = &sm_at<T>(G.o.valA) + lane, *lc = &sm_at<T>(G.lc) + lane, *uc = &sm_at<T>(G.uc) + lane;
+        const uint16_t* idx = &sm_at<uint16_t>(G.o.idxA) + lane;
+        const uint32_t* off = &sm_at<uint32_t>(G.o.offA);
+        const uint8_t* len = &sm_at<uint8_t>(G.o.lenA) + lane;
+        for (int l = threadIdx.x >> 5; l < G.LA; l += NT / 32) {
+            const int k = l * 32, r = (l * CS + G.rank) * 32 + lane;
+            const uint32_t o = off[l];
+            const T s = slice_sum(idx + (o >> 8) * 32, val + (o >> 8) * 32, (int)(o & 255u), len[k], xb);
+            if (r < G.R.m) {
+                const T lo = lc[k], up = uc[k], yy = y[G.baseA + k + lane];
+                const double dd = (double)mul_rn(invD1[G.ordA[r]], sub_rn(s, proj_box(s, lo, up)));
                 v[0] += __dmul_rn(dd, dd);
                 v[1] += (double)sub_rn(safeprod_left(up, pos_part(-yy)), safeprod_left(lo, neg_part(-yy)));
             }
         }
-        for (int l = w; l < LAt; l += NW) {
-            const T s = sumAt(l, y);
-            const int r = row(l), k = l * 32 + lane;
-            if (r < R.n) {
+    }
+    {
+        const T *val = &sm_at<T>(G.o.valAt) + lane, *lv = &sm_at<T>(G.lv) + lane,
+                *uv = &sm_at<T>(G.uv) + lane, *c = &sm_at<T>(G.c) + lane;
+        const uint16_t* idx = &sm_at<uint16_t>(G.o.idxAt) + lane;
+        const uint32_t* off = &sm_at<uint32_t>(G.o.offAt);
+        const uint8_t* len = &sm_at<uint8_t>(G.o.lenAt) + lane;
+        for (int l = threadIdx.x >> 5; l < G.LAt; l += NT / 32) {
+            const int k = l * 32, r = (l * CS + G.rank) * 32 + lane;
+            const uint32_t o = off[l];
+            const T s = slice_sum(idx + (o >> 8) * 32, val + (o >> 8) * 32, (int)(o & 255u), len[k], y);
+            if (r < G.R.n) {
                 const T cj = c[k], lo = lv[k], up = uv[k];
                 const T gg = sub_rn(cj, s);
                 const T rr = proj_multiplier(gg, lo, up);
-                const double dd = (double)mul_rn(invD2[ordAt[r]], sub_rn(gg, rr));
+                const double dd = (double)mul_rn(invD2[G.ordAt[r]], sub_rn(gg, rr));
                 v[2] += __dmul_rn(dd, dd);
                 v[3] += (double)sub_rn(safeprod_left(up, pos_part(-rr)), safeprod_left(lo, neg_part(-rr)));
-                v[4] += (double)mul_rn(cj, xb[r]);
+                v[4] += (double)mul_rn(cj, xb[G.baseAt + k + lane]);
             }
         }
-        res_sum<5, CS, NW>(v, sh);
     }
+    __syncwarp();
+    res_sum<5, CS, NT / 32>(v, sh, phase);
+#pragma unroll
+    for (int q = 0; q < 5; q++) out[q] = v[q];
+}
 
-    // powm! iterations (linalg.jl:86-96) in FP64 over the stored values, from
-    // the vector px (already loaded): stops after an iteration whose residual
-    // is at most tol or rtol * theta, or after iteration `last`.
-    // The residual of an iteration needs its theta, so its norm is summed with
-    // the next iteration's theta (one exchange an iteration); the extra
-    // iteration's own theta is dropped.  it0: iterations already run.
-    struct Power {
-        double theta, residual;
-        int64_t it;
-        bool stop;
-    };
-    __device__ Power power(int64_t it0, int64_t max_here, int64_t maxiter, double tol, double rtol,
-                           double theta_prev, double* sh) {
-        Power P{theta_prev, INFINITY, it0, false};
-        double r2 = 0.0;       // own part of the last iteration's residual^2
-        bool pending = false;  // an iteration's residual is not summed yet
-        for (;;) {
-            // Ax, then A'Ax with the sums of theta, |A'Ax|^2 and the residual
-            for (int l = w; l < LA; l += NW) {
-                const double s = sumA(l, px);
-                const int r = row(l);
-                if (r < R.m) res_put<CS>(ps + r, s);
-            }
-            res_sync<CS>();
-            double v[3] = {0.0, 0.0, r2};
-            for (int l = w; l < LAt; l += NW) {
-                const double s = sumAt(l, ps);
-                const int r = row(l);
-                if (r < R.n) {
-                    pax[l * 32 + lane] = s;
-                    v[0] += px[r] * s;
-                    v[1] += s * s;
-                }
-            }
-            res_sum<3, CS, NW>(v, sh);
-            if (pending) {
-                P.residual = sqrt(v[2]);
-                P.it++;
-                if (P.it > maxiter || P.residual <= tol || (rtol > 0 && P.residual <= rtol * P.theta)) {
-                    P.stop = true;
-                    return P;
-                }
-                if (P.it - it0 >= max_here) return P;
-            }
-            const double theta = v[0], inv = 1.0 / sqrt(v[1]);
-            P.theta = theta;
-            r2 = 0.0;
-            for (int l = w; l < LAt; l += NW) {
-                const int r = row(l);
-                if (r < R.n) {
-                    const double ax = pax[l * 32 + lane];
-                    const double rr = add_rn(mul_rn(-theta, px[r]), ax);
-                    r2 += rr * rr;
-                    res_put<CS>(px + r, mul_rn(ax, inv));
-                }
-            }
-            pending = true;
-            res_sync<CS>();
+// powm! iterations (linalg.jl:86-96) in FP64 over the stored values, from the
+// vector px (loaded whole into every CTA): stops after an iteration whose
+// residual is at most tol or rtol * theta, after iteration maxiter + 1 or after
+// max_here iterations of this call.  The residual of an iteration needs its
+// theta, so its norm is summed with the next iteration's theta (one exchange
+// an iteration); the extra iteration's own theta is dropped.  it0 iterations
+// ran before, the last with theta_prev.
+template <class T, int CS, int NT>
+__device__ __noinline__ void res_power(const ResGeo& G, int64_t it0, int64_t max_here,
+                                       int64_t maxiter, double tol, double rtol, double theta_prev,
+                                       ResPower& P, double* sh, int& phase, ResWait& W,
+                                       unsigned& parity_io) {
+    constexpr int NW = NT / 32;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, rank = G.rank;
+    const int LA = G.LA, LAt = G.LAt, n = G.R.n;
+    const T *valA = &sm_at<T>(G.o.valA) + lane, *valAt = &sm_at<T>(G.o.valAt) + lane;
+    const uint16_t *idxA = &sm_at<uint16_t>(G.o.idxA) + lane, *idxAt = &sm_at<uint16_t>(G.o.idxAt) + lane;
+    const uint32_t *offA = &sm_at<uint32_t>(G.o.offA), *offAt = &sm_at<uint32_t>(G.o.offAt);
+    const uint8_t *lenA = &sm_at<uint8_t>(G.o.lenA) + lane, *lenAt = &sm_at<uint8_t>(G.o.lenAt) + lane;
+    const double *px = &sm_at<double>(G.px), *ps = &sm_at<double>(G.ps);
+    double *pxown = &sm_at<double>(G.px) + G.baseAt, *psown = &sm_at<double>(G.ps) + G.baseA;
+    double* pax = &sm_at<double>(G.pax) + lane;
+    unsigned parity = parity_io;
+    double theta = theta_prev, residual = INFINITY;
+    int64_t it = it0;
+    bool stop = false;
+    double r2 = 0.0;       // own part of the last iteration's residual^2
+    bool pending = false;  // an iteration's residual is not summed yet
+    for (;;) {
+#pragma unroll 1
+        for (int l = w; l < LA; l += NW) {
+            const uint32_t o = offA[l];
+            psown[l * 32 + lane] = slice_sum(idxA + (o >> 8) * 32, valA + (o >> 8) * 32,
+                                             (int)(o & 255u), lenA[l * 32], px);
+            res_send<CS>(psown + l * 32, &W.bar[0], rank);
         }
+        res_receive<CS>(W, 0, G.remA * 8u, parity);
+        double v[3] = {0.0, 0.0, r2};
+#pragma unroll 1
+        for (int l = w; l < LAt; l += NW) {
+            const int r = (l * CS + rank) * 32 + lane;
+            const uint32_t o = offAt[l];
+            const double s = slice_sum(idxAt + (o >> 8) * 32, valAt + (o >> 8) * 32,
+                                       (int)(o & 255u), lenAt[l * 32], ps);
+            pax[l * 32] = s;
+            if (r < n) {
+                v[0] += pxown[l * 32 + lane] * s;
+                v[1] += s * s;
+            }
+        }
+        __syncwarp();
+        res_sum<3, CS, NW>(v, sh, phase);
+        if (pending) {
+            residual = sqrt(v[2]);
+            it++;
+            stop = it > maxiter || residual <= tol || (rtol > 0 && residual <= rtol * theta);
+            if (stop || it - it0 >= max_here || (CS > 1 && W.failed)) break;
+        }
+        theta = v[0];
+        const double inv = 1.0 / sqrt(v[1]);
+        r2 = 0.0;
+#pragma unroll 1
+        for (int l = w; l < LAt; l += NW) {
+            const int r = (l * CS + rank) * 32 + lane;
+            const double ax = pax[l * 32];
+            if (r < n) {
+                const double rr = __fma_rn(-theta, pxown[l * 32 + lane], ax);
+                r2 += rr * rr;
+            }
+            pxown[l * 32 + lane] = mul_rn(ax, inv);
+            res_send<CS>(pxown + l * 32, &W.bar[1], rank);
+        }
+        pending = true;
+        res_receive<CS>(W, 1, G.remAt * 8u, parity);
     }
-};
+    P.theta = theta;
+    P.residual = residual;
+    P.it = it;
+    P.stop = stop;
+    parity_io = parity;
+    res_sync<CS>();
+}
 
 }  // namespace cpdlp
