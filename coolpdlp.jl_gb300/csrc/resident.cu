@@ -143,6 +143,7 @@ int res_plan(const int32_t* ptrA, const int32_t* ptrAt, int64_t m, int64_t n, in
     if (m < 1 || n < 1 || nnz < 1 || m > RES_MAX_DIM || n > RES_MAX_DIM) return 0;
     // FP64 steps are bounded by the SM's FP64 pipe, so even small LPs are
     // spread over a cluster; FP32 ones only when they need its shared memory
+    if (single && sv == 8 && nnz > RES_SINGLE_F64_NNZ) return 0;
     int cs = 1;
     if (sv == 8 && nnz >= RES_F64_CLUSTER_NNZ) cs = RES_MAX_CS;
     if (single && nnz >= RES_SINGLE_CLUSTER_NNZ) cs = RES_MAX_CS;

@@ -1004,6 +1004,9 @@ ProblemBase* make_problem(Handle& h, const cpdlp_lp* lp, const cpdlp_params* prm
         }
     }
     mark("formats, autotuner, density order");
+    // a small LP runs its blocks on the resident kernels: with the library's own
+    // choice of engine (no ELL, no pinned tile size) and valued storage
+    if (!pm1 && mt != CPDLP_FMT_ELL && prm->tile_nnz == 0) res_single_build<T>(*P, hp2, hp1, s);
     // the CSR plans (also kept for an ELL side: the tuner and the exports use them),
     // the two on two host threads (each a sequential pass over its rows)
     {
@@ -1137,6 +1140,31 @@ double spectral_norm_T(Handle& h, ProblemT<V>& P, const cpdlp_params* prm, int64
     const CsrView<Pm1, double> At1{P.at_ptr.p, P.at_idx.p, nullptr, P.planAt.tasks.p,
                                    P.planAt.ntasks, P.planAt.ltasks.p, P.planAt.nltasks,
                                    P.planAt.counters.p, pAt.p};
+    if (P.rlp.cs > 0) {
+        // a launch runs many iterations; the host looks at the deadline between
+        // launches (1,024 iterations take a few milliseconds)
+        void* block = h.host_get(sizeof(double) * 8);
+        double* out = static_cast<double*>(block);
+        struct Put {
+            Handle& h; void* block; cudaStream_t s;
+            ~Put() { cudaStreamSynchronize(s); h.host_put(block); }
+        } put{h, block, s};
+        double* dout = nullptr;
+        CK(cudaHostGetDevicePointer((void**)&dout, out, 0));
+        int64_t it = 0;
+        double theta = 0.0;
+        for (;;) {
+            out[4] = 0.0;
+            res_single_power<V>(P, x.p, it, 1024, maxiter, tol, rtol, theta, dout, s);
+            CK(cudaStreamSynchronize(s));
+            if (out[4] != 0.0) fail(CPDLP_ERR_CUDA, "resident power method: a wait ran out");
+            theta = out[0];
+            it = (int64_t)out[2];
+            if (out[3] != 0.0 || now_seconds() >= deadline) break;
+        }
+        if (iters_out) *iters_out = it;
+        return std::sqrt(theta);
+    }
     DBuf<double> xs((size_t)(P.pm1 && n > 0 ? n : 1));
     if (P.pm1 && n > 0) {
         k_mul_vec<double><<<grid_for(n, 256), 256, 0, s>>>(x.p, P.D2.p, xs.p, n);
@@ -1340,8 +1368,41 @@ struct StateT : StateBase {
         cudaGraphDestroy(g);
     }
 
-    // `len` steps as one graph launch (len == check_every).
-    void run_block(int len) {
+    // the KKT sums of the last resident block's iterates (kkt_multi reads them
+    // instead of evaluating): how many, 0 when none are ready
+    int res_nv = 0;
+    double* res_out() { return h->pinned_area(sizeof(double) * 64) + 32; }
+
+    // `len` steps in one resident launch, with the KKT sums of nv iterates
+    void run_resident(int len, int nv) {
+        const int o = cur, nw = (len & 1) ? cur ^ 1 : cur, la = nw ^ 1;
+        ResBlock<T> b{};
+        b.x = x[o].p; b.xa = xa[o].p; b.y = y[o].p; b.ya = ya[o].p;
+        b.to.x = x[nw].p; b.to.xl = x[la].p; b.to.xa = xa[nw].p; b.to.xal = xa[la].p;
+        b.to.y = y[nw].p; b.to.yl = y[la].p; b.to.ya = ya[nw].p; b.to.yal = ya[la].p;
+        b.eta = eta; b.omega = omega; b.eta_sum = eta_sum;
+        b.steps = len;
+        b.avg = pdlp() ? 1 : 0;
+        b.nv = nv;
+        b.out = res_out();
+        res_out()[20] = 0.0;
+        res_single_block<T>(*PT, b, h->stream);
+        launches += 1;
+        res_nv = nv;
+        if (pdlp())
+            for (int k = 0; k < len; k++) eta_sum += eta;
+        cur = nw;
+        advance_counters(len);
+    }
+
+    // `len` steps: one resident launch (nv: the iterates whose KKT errors the
+    // check after it wants), or one graph launch (len == check_every).
+    void run_block(int len, int nv = 0) {
+        res_nv = 0;
+        if (PT->rlp.cs > 0 && !yoff) {
+            run_resident(len, kkt_hook ? 0 : nv);
+            return;
+        }
         cudaStream_t s = h->stream;
         if (len != graph_len) {
             for (auto& g : graph)
@@ -1380,6 +1441,7 @@ struct StateT : StateBase {
     }
 
     void step(int64_t count) override {
+        res_out()[20] = 0.0;
         const int ce = prm.check_every > 0 ? prm.check_every : 100;
         while (count >= ce) {
             run_block(ce);
@@ -1387,6 +1449,7 @@ struct StateT : StateBase {
         }
         while (count-- > 0) run_single();
         CK(cudaStreamSynchronize(h->stream));
+        if (PT->rlp.cs > 0 && res_out()[20] != 0.0) fail(CPDLP_ERR_CUDA, "resident block: a wait ran out");
     }
 
     // KKT errors (errors.jl:65-109) of NV (1 or 4) (x, y) pairs in ONE
@@ -1462,6 +1525,15 @@ struct StateT : StateBase {
         }
         ProblemT<T>& P = *PT;
         cudaStream_t s = h->stream;
+        if (res_nv == NV && xs[0] == x[cur].p) {
+            // evaluated by the block that produced the iterates
+            res_nv = 0;
+            CK(cudaStreamSynchronize(s));
+            const double* v = res_out();
+            if (v[20] != 0.0) fail(CPDLP_ERR_CUDA, "resident block: a wait ran out");
+            for (int p = 0; p < NV; p++, v += 5) errors_from(v[0], v[1], v[2], v[3], v[4], out[p]);
+            return;
+        }
         enqueue_kkt<NV>(xs, ys);
         reduce_partials(P.red_rows.p, NV == 4 ? P.rows_A_kkt4 : P.rows_A_kkt, 2 * NV,
                         P.red_out.p, s);
@@ -1472,17 +1544,18 @@ struct StateT : StateBase {
         CK(cudaMemcpyAsync(pin, P.red_out.p, sizeof(double) * 5 * NV, cudaMemcpyDeviceToHost, s));
         CK(cudaStreamSynchronize(s));
         for (int p = 0; p < NV; p++) {
-            const double pr2 = pin[2 * p], pc = pin[2 * p + 1];
-            const double du2 = pin[2 * NV + 3 * p], pv = pin[2 * NV + 3 * p + 1],
-                         cx = pin[2 * NV + 3 * p + 2];
-            cpdlp_kkt_errors& e = out[p];
-            e.primal = std::sqrt(pr2);
-            e.primal_scale = P.primal_scale;
-            e.dual = std::sqrt(du2);
-            e.dual_scale = P.dual_scale;
-            e.gap = std::fabs((cx + pc) + pv);
-            e.gap_scale = (1.0 + std::fabs(pc + pv)) + std::fabs(cx);
+            const double* col = pin + 2 * NV + 3 * p;
+            errors_from(pin[2 * p], pin[2 * p + 1], col[0], col[1], col[2], out[p]);
         }
+    }
+    void errors_from(double pr2, double pc, double du2, double pv, double cx,
+                     cpdlp_kkt_errors& e) const {
+        e.primal = std::sqrt(pr2);
+        e.primal_scale = PT->primal_scale;
+        e.dual = std::sqrt(du2);
+        e.dual_scale = PT->dual_scale;
+        e.gap = std::fabs((cx + pc) + pv);
+        e.gap_scale = (1.0 + std::fabs(pc + pv)) + std::fabs(cx);
     }
 
     void vec_of(int which, const T*& vx, const T*& vy) {
@@ -1684,7 +1757,7 @@ struct StateT : StateBase {
         if (!pdlp()) {
             for (;;) {
                 if (blocks >= max_blocks) return status;
-                run_block(ce);
+                run_block(ce, 1);
                 blocks++;
                 cpdlp_kkt_errors e;
                 kkt(CPDLP_VEC_SOL, &e);
@@ -1700,7 +1773,7 @@ struct StateT : StateBase {
         // restart check; on termination the outer loop checks once more.
         for (;;) {
             if (blocks >= max_blocks) return status;
-            run_block(ce);
+            run_block(ce, 4);
             blocks++;
             cpdlp_kkt_errors e4[4];
             const T* const xs[4] = {x[cur].p, xa[cur].p, x[cur ^ 1].p, xa[cur ^ 1].p};

@@ -4,6 +4,7 @@
 #include <type_traits>
 
 #include "cpdlp_common.cuh"
+#include "resident_plan.cuh"
 #include "sparse_build.cuh"
 #include "tiles.cuh"
 
@@ -81,6 +82,9 @@ struct ProblemT : ProblemBase {
     // value arrays are empty, and the products apply d1 / d2 (as T)
     bool pm1 = false;
     DBuf<T> d1t, d2t;
+    // a small LP's slices for the resident kernels (rlp.cs = 0: not resident)
+    ResStore<T> res;
+    ResLP rlp{};
     // 1 ./ D1 and 1 ./ D2 in T for the KKT terms (FP32 problems keep a copy;
     // FP64 problems use invD1 / invD2 themselves)
     DBuf<T> invD1t, invD2t;
@@ -93,6 +97,35 @@ struct ProblemT : ProblemBase {
         else return invD2t.p;
     }
 };
+
+// One LP on the resident kernels (resident_single.cu).  res_single_build
+// decides and fills P.res (hpA, hpAt: the row pointers on the host).
+template <class T>
+void res_single_build(ProblemT<T>& P, const std::vector<int32_t>& hpA,
+                      const std::vector<int32_t>& hpAt, cudaStream_t s);
+// A block of steps from (x, y) and the averages (P's order); the last step
+// leaves both iterates and both averages at `to` (which may be the buffers read).
+// nv = 1 or 4: then also the KKT sums of sol, or of sol, avg, sol_last and
+// avg_last, 5 values each (primal^2, row objective, dual^2, column objective,
+// c'x), to `out`; out[20] != 0: the kernel gave up a wait.  out: page-locked.
+template <class T>
+struct ResBlock {
+    const T *x, *xa, *y, *ya;
+    struct {
+        T *x, *xl, *xa, *xal, *y, *yl, *ya, *yal;
+    } to;
+    double eta, omega, eta_sum;
+    int steps, avg, nv;
+    double* out;
+};
+template <class T>
+void res_single_block(const ProblemT<T>& P, const ResBlock<T>& b, cudaStream_t s);
+// powm! iterations on x (n doubles, P's order, in place), at most max_here:
+// out[0..3] = theta, residual, iterations so far, stopped; out[4]: gave up.
+template <class T>
+void res_single_power(const ProblemT<T>& P, double* x, int64_t it0, int64_t max_here,
+                      int64_t maxiter, double tol, double rtol, double theta_prev, double* out,
+                      cudaStream_t s);
 
 struct StateBase {
     virtual ~StateBase() = default;
