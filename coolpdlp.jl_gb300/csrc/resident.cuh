@@ -246,21 +246,27 @@ constexpr int RES_SUMS = 5;  // most values of one sum
 // number of values a lane carries (9 additions a lane for 5 values instead of
 // 25), every warp stores its sums into every CTA, and after one group barrier
 // warp q of each CTA adds value q of all warps of the group with a tree.  The
-// order depends on the group's shape alone.
+// order depends on the group's shape alone.  `busy` is false for a warp whose
+// values are all zero (it does no additions: 16 warps' trees take 0.9 us of the
+// SM's FP64 pipe).  finish(q, sum), by one lane of warp q, gives what the
+// threads receive in place of the sum: what every thread would compute alike
+// costs the pipe once per warp (a square root and a division by 16 warps 3.6 us).
 // sh: res_sh<CS, NW>() doubles; `phase` alternates the halves, so that a fast
 // CTA's next sums do not meet a slow one's reads.
 template <int CS, int NW>
 constexpr int res_sh() { return 2 * RES_SUMS * CS * NW + 8; }
-template <int Q, int CS, int NW>
-__device__ __forceinline__ void res_sum(double (&v)[Q], double* sh, int& phase) {
+template <int Q, int CS, int NW, class F>
+__device__ __forceinline__ void res_sum(double (&v)[Q], double* sh, int& phase, bool busy,
+                                        F&& finish) {
     static_assert(Q <= RES_SUMS && Q <= NW, "a warp per value");
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     constexpr int P = CS * NW;  // warps of the group
     double* slot = sh + 8 + phase * (RES_SUMS * P);
     phase ^= 1;
-    double d;
-    int which;
-    if constexpr (Q <= 4) {
+    double d = 0.0;
+    int which = lane / (Q <= 4 ? 8 : 4);
+    if (!busy) {
+    } else if constexpr (Q <= 4) {
         double a[4], c[2];
 #pragma unroll
         for (int q = 0; q < 4; q++) a[q] = q < Q ? v[q < Q ? q : 0] : 0.0;
@@ -273,7 +279,6 @@ __device__ __forceinline__ void res_sum(double (&v)[Q], double* sh, int& phase) 
         const double send = h2 ? c[0] : c[1], keep = h2 ? c[1] : c[0];
         d = keep + __shfl_xor_sync(FULL_MASK, send, 8);
         d += __shfl_xor_sync(FULL_MASK, d, 4);
-        which = (h ? 2 : 0) + (h2 ? 1 : 0);
     } else {
         double a[8], b[4], c[2];
 #pragma unroll
@@ -291,10 +296,11 @@ __device__ __forceinline__ void res_sum(double (&v)[Q], double* sh, int& phase) 
         }
         const double send = h3 ? c[0] : c[1], keep = h3 ? c[1] : c[0];
         d = keep + __shfl_xor_sync(FULL_MASK, send, 4);
-        which = (h ? 4 : 0) + (h2 ? 2 : 0) + (h3 ? 1 : 0);
     }
-    d += __shfl_xor_sync(FULL_MASK, d, 2);
-    d += __shfl_xor_sync(FULL_MASK, d, 1);
+    if (busy) {
+        d += __shfl_xor_sync(FULL_MASK, d, 2);
+        d += __shfl_xor_sync(FULL_MASK, d, 1);
+    }
     const int rank = res_rank<CS>();
     if ((lane & (Q <= 4 ? 7 : 3)) == 0 && which < Q)
         res_put<CS>(slot + which * P + rank * NW + w, d, rank);
@@ -307,12 +313,17 @@ __device__ __forceinline__ void res_sum(double (&v)[Q], double* sh, int& phase) 
             if (k * 32 + lane < P) s = k ? s + slot[w * P + k * 32 + lane] : slot[w * P + lane];
 #pragma unroll
         for (int o = (P < 32 ? P : 32) / 2; o > 0; o >>= 1) s += __shfl_xor_sync(FULL_MASK, s, o);
-        if (lane == 0) sh[w] = s;
+        if (lane == 0) sh[w] = finish(w, s);
     }
     __syncthreads();
 #pragma unroll
     for (int q = 0; q < Q; q++) v[q] = sh[q];
     // sh[0..7] are rewritten only after the next call's group barrier
+}
+
+template <int Q, int CS, int NW>
+__device__ __forceinline__ void res_sum(double (&v)[Q], double* sh, int& phase, bool busy = true) {
+    res_sum<Q, CS, NW>(v, sh, phase, busy, [](int, double s) { return s; });
 }
 
 // the resident LP as one CTA of its group sees it (in shared memory)
@@ -334,6 +345,7 @@ struct ResGeo {
 template <class T>
 struct ResCoefs {
     T a[RES_COEF], b[RES_COEF];
+    T k[3];  // tau, sigma, 1 / sigma
     double es;
 };
 // where the last step of a block leaves sol, sol_last and the averages
@@ -482,17 +494,16 @@ __device__ __noinline__ void res_steps(const ResGeo& G, double eta, double omega
     const T *c = &sm_at<T>(G.c) + lane, *lv = &sm_at<T>(G.lv) + lane, *uv = &sm_at<T>(G.uv) + lane;
     const T *lc = &sm_at<T>(G.lc) + lane, *uc = &sm_at<T>(G.uc) + lane;
     unsigned parity = parity_io;
-    const double sg = eta * omega;
-    const T tau = (T)(eta / omega), sigma = (T)sg, inv_sigma = (T)(1.0 / sg);
+    T tau = T(0), sigma = T(0), inv_sigma = T(0);
     for (int k0 = 0; k0 < count; k0 += RES_COEF) {
         const int nk = min(count - k0, RES_COEF);
-        if (avg) {
-            // eta/(eta+es), es/(eta+es) of all nk steps at once, es growing by
-            // eta a step (a chain of additions, like the host's): a division
-            // a step by one thread would be longer than the step
-            __syncthreads();
-            const double es = tab.es;
-            __syncthreads();
+        // the step sizes, and eta/(eta+es), es/(eta+es) of all nk steps at once,
+        // es growing by eta a step (a chain of additions, like the host's): a
+        // division a step by one thread would be longer than the step
+        __syncthreads();
+        const double es = tab.es;
+        __syncthreads();
+        if (avg)
             for (int t = threadIdx.x; t < nk; t += NT) {
                 double e = es;
                 for (int q = 0; q < t; q++) e += eta;
@@ -500,8 +511,16 @@ __device__ __noinline__ void res_steps(const ResGeo& G, double eta, double omega
                 tab.b[t] = (T)(e / (eta + e));
                 if (t == nk - 1) tab.es = e + eta;
             }
-            __syncthreads();
+        if (threadIdx.x == NT - 32) {
+            const double sg = eta * omega;
+            tab.k[0] = (T)(eta / omega);
+            tab.k[1] = (T)sg;
+            tab.k[2] = (T)(1.0 / sg);
         }
+        __syncthreads();
+        tau = tab.k[0];
+        sigma = tab.k[1];
+        inv_sigma = tab.k[2];
 #pragma unroll 1
         for (int st = 0; st < nk; st++) {
             const bool last = k0 + st == count - 1;
@@ -625,7 +644,7 @@ __device__ __noinline__ void res_kkt_sums(const ResGeo& G, const T* gx, const T*
         }
     }
     __syncwarp();
-    res_sum<5, CS, NT / 32>(v, sh, phase);
+    res_sum<5, CS, NT / 32>(v, sh, phase, (int)(threadIdx.x >> 5) < max(G.LA, G.LAt));
 #pragma unroll
     for (int q = 0; q < 5; q++) out[q] = v[q];
 }
@@ -676,20 +695,28 @@ __device__ __noinline__ void res_power(const ResGeo& G, int64_t it0, int64_t max
                                        (int)(o & 255u), lenAt[l * 32], ps);
             pax[l * 32] = s;
             if (r < n) {
-                v[0] += pxown[l * 32 + lane] * s;
-                v[1] += s * s;
+                v[0] = __fma_rn(pxown[l * 32 + lane], s, v[0]);
+                v[1] = __fma_rn(s, s, v[1]);
             }
         }
         __syncwarp();
-        res_sum<3, CS, NW>(v, sh, phase);
+        // theta, 1 / |A'Ax| and the previous iteration's residual (negative when
+        // it ends the iteration)
+        res_sum<3, CS, NW>(v, sh, phase, w < LAt, [&](int q, double s) {
+            if (q == 0) return s;
+            if (q == 1) return rsqrt(s);
+            const double res = sqrt(s);
+            return res <= tol || (rtol > 0 && res <= rtol * theta) ? -1.0 - res : res;
+        });
         if (pending) {
-            residual = sqrt(v[2]);
+            const bool small = __double_as_longlong(v[2]) < 0;
+            residual = v[2];
             it++;
-            stop = it > maxiter || residual <= tol || (rtol > 0 && residual <= rtol * theta);
+            stop = it > maxiter || small;
             if (stop || it - it0 >= max_here || (CS > 1 && W.failed)) break;
         }
         theta = v[0];
-        const double inv = 1.0 / sqrt(v[1]);
+        const double inv = v[1];
         r2 = 0.0;
 #pragma unroll 1
         for (int l = w; l < LAt; l += NW) {
@@ -697,7 +724,7 @@ __device__ __noinline__ void res_power(const ResGeo& G, int64_t it0, int64_t max
             const double ax = pax[l * 32];
             if (r < n) {
                 const double rr = __fma_rn(-theta, pxown[l * 32 + lane], ax);
-                r2 += rr * rr;
+                r2 = __fma_rn(rr, rr, r2);
             }
             pxown[l * 32 + lane] = mul_rn(ax, inv);
             res_send<CS>(pxown + l * 32, &W.bar[1], rank);
@@ -705,6 +732,7 @@ __device__ __noinline__ void res_power(const ResGeo& G, int64_t it0, int64_t max
         pending = true;
         res_receive<CS>(W, 1, G.remAt * 8u, parity);
     }
+    if (__double_as_longlong(residual) < 0) residual = -1.0 - residual;
     P.theta = theta;
     P.residual = residual;
     P.it = it;
