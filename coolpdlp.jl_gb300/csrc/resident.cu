@@ -141,11 +141,12 @@ bool res_meta(const int32_t* ptr, int rows, int cs, std::vector<int32_t>& meta, 
 int res_plan(const int32_t* ptrA, const int32_t* ptrAt, int64_t m, int64_t n, int64_t nnz, int sv,
              bool single, ResLP& r, std::vector<int32_t>& metaA, std::vector<int32_t>& metaAt) {
     if (m < 1 || n < 1 || nnz < 1 || m > RES_MAX_DIM || n > RES_MAX_DIM) return 0;
-    // FP64 steps are bounded by the SM's FP64 pipe, so even small LPs are
-    // spread over a cluster; FP32 ones only when they need its shared memory
+    // FP64 steps are bounded by the SMs' FP64 pipes, so even small LPs are
+    // spread over a cluster
     if (single && sv == 8 && nnz > RES_SINGLE_F64_NNZ) return 0;
     int cs = 1;
     if (sv == 8 && nnz >= RES_F64_CLUSTER_NNZ) cs = RES_MAX_CS;
+    if (sv == 4 && nnz >= RES_F32_CLUSTER_NNZ) cs = 4;
     if (single && nnz >= RES_SINGLE_CLUSTER_NNZ) cs = RES_MAX_CS;
     r.m = (int32_t)m;
     r.n = (int32_t)n;

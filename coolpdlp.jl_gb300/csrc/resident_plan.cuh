@@ -16,9 +16,12 @@ constexpr int RES_COEF = 128;            // averaging coefficients computed at a
 // LPs with at least this many nonzeros take a whole cluster.  FP64 (in a batch
 // or alone): a step of 1,978 nonzeros takes 3.9 us on one CTA and 3.1 us on 8,
 // 575 nonzeros 2.5 and 3.0 us.  FP32 alone: 8,000 nonzeros 2.7 and 1.5 us, 1,978
-// nonzeros 1.14 and 1.27 us; in a batch FP32 LPs take the smallest group that
-// holds them (2,048 LPs: 550 ms, 571 ms with groups of 4 from 3,000 nonzeros).
+// nonzeros 1.14 and 1.27 us.  FP32 in a batch: groups of 4 from 3,000 nonzeros
+// (10,000 nonzeros: 1.6 us a step against 3.1 us alone on an SM; the slowest LPs
+// of a batch end sooner, and 2,048 LPs together take 571 instead of 550 ms;
+// groups of 8 from there 679 ms).
 constexpr int64_t RES_F64_CLUSTER_NNZ = 1500;
+constexpr int64_t RES_F32_CLUSTER_NNZ = 3000;
 constexpr int64_t RES_SINGLE_CLUSTER_NNZ = 3000;
 // a single LP with FP64 iterates is resident up to this many nonzeros: above,
 // the FP64 pipes of the whole chip beat those of eight SMs
