@@ -199,6 +199,10 @@ __device__ __forceinline__ float add_rn(float a, float b) { return __fadd_rn(a, 
 __device__ __forceinline__ double sub_rn(double a, double b) { return __dsub_rn(a, b); }
 __device__ __forceinline__ float sub_rn(float a, float b) { return __fsub_rn(a, b); }
 
+// a*b + c: rounded twice in FP32 (as the reference's sequence of operations),
+// once in FP64, where the number of operations is what steps cost
+__device__ __forceinline__ float mul_add(float a, float b, float c) { return add_rn(mul_rn(a, b), c); }
+__device__ __forceinline__ double mul_add(double a, double b, double c) { return __fma_rn(a, b, c); }
 // 2x - y: doubling is exact, so one fused operation rounds like the product
 // and the difference do
 __device__ __forceinline__ double extrapolate(double x, double y) { return __fma_rn(2.0, x, -y); }

@@ -95,11 +95,11 @@ struct PrimalEpi {
     __device__ __forceinline__ void row(int, int j, T s, const Pre& q, Acc&) {
         const StepCoef<T>& k = coef.get();
         if (SCALED) s = mul_rn(q.d, s);
-        const T xp = proj_box(sub_rn(q.x, mul_rn(k.tau, sub_rn(q.c, s))), q.lv, q.uv);
+        const T xp = proj_box(mul_add(-k.tau, sub_rn(q.c, s), q.x), q.lv, q.uv);
         __stcs(xn + j, xp);
         const T xb = extrapolate(xp, q.x);
         xbar[j] = SCALED ? mul_rn(q.d, xb) : xb;
-        if (avg) __stcs(xa_new + j, add_rn(mul_rn(xp, k.a), mul_rn(q.xa, k.b)));
+        if (avg) __stcs(xa_new + j, mul_add(xp, k.a, mul_rn(q.xa, k.b)));
     }
     __device__ void row_long(int p, int j, T s, int, Acc& a) { row(p, j, s, pre_global(j), a); }
     __device__ void finish(Acc&) {}
@@ -147,14 +147,14 @@ struct DualEpi {
             const double pr = proj_box(t4, -(double)q.uc, -(double)q.lc);
             yp = (T)__dsub_rn(__dsub_rn((double)q.y, __dmul_rn(sg, sd)), __dmul_rn(sg, pr));
         } else {
-            const T t2 = sub_rn(q.y, mul_rn(sigma, s));
-            const T t4 = sub_rn(mul_rn(k.inv_sigma, q.y), s);
+            const T t2 = mul_add(-sigma, s, q.y);
+            const T t4 = mul_add(k.inv_sigma, q.y, -s);
             const T pr = proj_box(t4, -q.uc, -q.lc);
-            yp = sub_rn(t2, mul_rn(sigma, pr));
+            yp = mul_add(-sigma, pr, t2);
         }
         yn[i] = yp;
         if (SCALED) ysn[i] = mul_rn(q.d, yp);
-        if (avg) __stcs(ya_new + i, add_rn(mul_rn(yp, k.a), mul_rn(q.ya, k.b)));
+        if (avg) __stcs(ya_new + i, mul_add(yp, k.a, mul_rn(q.ya, k.b)));
     }
     __device__ void row_long(int p, int i, T s, int, Acc& a) { row(p, i, s, pre_global(i), a); }
     __device__ void finish(Acc&) {}

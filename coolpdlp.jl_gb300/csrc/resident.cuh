@@ -235,10 +235,6 @@ __device__ __forceinline__ double slice_sum(const uint16_t* ip, const V* vp, int
         if (w <= 0) return s;
     }
 }
-// a*b + c: rounded twice (FP32, as the tile kernels) or once (FP64)
-__device__ __forceinline__ float mul_add(float a, float b, float c) { return add_rn(mul_rn(a, b), c); }
-__device__ __forceinline__ double mul_add(double a, double b, double c) { return __fma_rn(a, b, c); }
-
 constexpr int RES_SUMS = 5;  // most values of one sum
 // Sums Q <= RES_SUMS values per thread over the group; every thread gets the
 // sums.  FP64 additions are what this costs (64 cycles each, one after the

@@ -1,0 +1,210 @@
+// sell.cuh -- the sliced-ELL step engine: one lane per row, 32 rows a slice.
+//
+// The tile engine (tiles.cuh) computes products nonzero by nonzero, stages them
+// in shared memory and sums them row by row: two phases, the second with as
+// many lanes as a tile has rows.  Here a lane walks its own row: the row's
+// entries are stored column-major in its slice, padded to the slice's longest
+// row, so a warp's loads are 128 (indices) and 128 or 256 bytes (values) wide,
+// nothing is staged, and the chain is offset -> entries -> gathers -> sum.
+// Measured (power-law LP, density order): FP64 6M nonzeros primal step 0.0887 ->
+// 0.0376 ms, dual 0.0729 -> 0.0505 ms; FP32 24M nonzeros primal 0.1164 -> 0.0933
+// ms, dual 0.1115 -> 0.1096 ms (a quarter of its entries are in long rows).
+// It suits the two places where the tile engine is not bound by memory:
+//  * FP64 on GB300, whose pipe retires 1.9 lane operations a clock and SM and
+//    charges idle lanes like busy ones: products and sums become one fused
+//    operation an entry with (nearly) all lanes in use;
+//  * small and medium LPs, where a step is the latency of that chain.
+// Rows are sorted by length inside windows of SELL_WINDOW rows (a permutation
+// kept per slice row, unless it is the identity, as in density order), so that
+// the padding stays small.  Rows longer than LONG_ROW are cut into pieces of
+// the tile plan's size and reduced by one warp each, like the tile engine's
+// long rows; every row sum rounds like the tile engine's in FP32.
+#pragma once
+
+#include "tiles.cuh"
+
+namespace cpdlp {
+
+constexpr int SELL_WINDOW = 256;
+constexpr uint8_t SELL_SKIP = 255;  // no row, or a row that the long pieces take
+
+template <class T>
+struct SellSide {
+    bool on = false;
+    int32_t nslices = 0, nltasks = 0, npieces = 0, tile = 512;
+    int64_t entries = 0;          // with padding
+    int64_t long_nnz = 0;         // nonzeros of the rows that the pieces take
+    DBuf<int32_t> off;            // per slice, units of 32 entries
+    DBuf<uint8_t> len;            // per slice row
+    DBuf<int32_t> perm;           // slice row -> row; empty: the identity
+    DBuf<int32_t> idx;
+    DBuf<T> val;
+    DBuf<int4> ltasks;            // {row, -(piece + 1), id, slot}
+    DBuf<int32_t> counters;
+    DBuf<T> partials;
+    void release() { *this = SellSide(); }
+};
+
+template <class T>
+struct SellView {
+    const int32_t* __restrict__ off;
+    const uint8_t* __restrict__ len;
+    const int32_t* __restrict__ perm;
+    const int32_t* __restrict__ idx;
+    const T* __restrict__ val;
+    const int4* __restrict__ ltasks;
+    int32_t* counters;
+    T* partials;
+    int32_t nslices, nltasks, tile;
+    const int32_t* __restrict__ ptr;   // the CSR, for the long rows
+    const int32_t* __restrict__ cidx;
+    const T* __restrict__ cval;
+};
+
+// The slices of a CSR (device; hp: its row pointer on the host); tile: the
+// piece size of long rows.  Leaves S.on false; S.entries tells the padding.
+template <class T>
+void build_sell(SellSide<T>& S, const std::vector<int32_t>& hp, const int32_t* ptr,
+                const int32_t* idx, const T* val, int64_t rows, int tile, cudaStream_t s);
+
+template <class T>
+SellView<T> sell_view(const SellSide<T>& S, const int32_t* ptr, const int32_t* idx, const T* val) {
+    return SellView<T>{S.off.p, S.len.p, S.perm.p, S.idx.p, S.val.p, S.ltasks.p, S.counters.p,
+                       S.partials.p, S.nslices, S.nltasks, S.tile, ptr, idx, val};
+}
+
+__device__ __forceinline__ int ld_cs(const int32_t* p) {
+    int v;
+    asm volatile("ld.global.cs.s32 %0, [%1];" : "=r"(v) : "l"(p));
+    return v;
+}
+// N entries of a row from place p (stride 32): all loads, then all gathers, are
+// in flight together; entries beyond the row's length add -0 (its padding has
+// value 0 and index 0)
+template <int N, class T>
+__device__ __forceinline__ T sell_chunk(const int32_t* ip, const T* vp, int len,
+                                        const T* __restrict__ x, T s) {
+    int c[N];
+    T v[N], g[N];
+#pragma unroll
+    for (int u = 0; u < N; u++) c[u] = ld_cs(ip + u * 32);
+#pragma unroll
+    for (int u = 0; u < N; u++) v[u] = ld_stream(vp + u * 32);
+#pragma unroll
+    for (int u = 0; u < N; u++) g[u] = gather<false>(x + c[u]);
+#pragma unroll
+    for (int u = 0; u < N; u++) {
+        if constexpr (sizeof(T) == 8) s = __fma_rn(v[u], u < len ? g[u] : T(-0.0), s);
+        else {
+            const T p = mul_rn(v[u], g[u]);
+            s = add_rn(s, u < len ? p : T(-0.0));
+        }
+    }
+    return s;
+}
+template <class T>
+__device__ __forceinline__ T sell_row(const int32_t* ip, const T* vp, int w, int len,
+                                      const T* __restrict__ x) {
+    T s = T(0);
+#pragma unroll 1
+    for (; w > 8; w -= 8, len -= 8, ip += 256, vp += 256) s = sell_chunk<8>(ip, vp, len, x, s);
+    switch (w) {
+        case 8: return sell_chunk<8>(ip, vp, len, x, s);
+        case 7: return sell_chunk<7>(ip, vp, len, x, s);
+        case 6: return sell_chunk<6>(ip, vp, len, x, s);
+        case 5: return sell_chunk<5>(ip, vp, len, x, s);
+        case 4: return sell_chunk<4>(ip, vp, len, x, s);
+        case 3: return sell_chunk<3>(ip, vp, len, x, s);
+        case 2: return sell_chunk<2>(ip, vp, len, x, s);
+        case 1: return sell_chunk<1>(ip, vp, len, x, s);
+        default: return s;
+    }
+}
+
+// one piece of a row longer than LONG_ROW (long_piece in tiles.cuh, with the
+// piece size at run time and four entries' loads in flight)
+template <class T, class Epi>
+__device__ __forceinline__ void sell_piece(const SellView<T>& S, const T* __restrict__ x, Epi& epi,
+                                           typename Epi::Acc& acc, int4 t, int lane) {
+    const int row = t.x, piece = -t.y - 1, lid = t.z, slot = t.w;
+    const int rb = ld_keep(S.ptr + row), re = ld_keep(S.ptr + row + 1);
+    const int npieces = (re - rb + S.tile - 1) / S.tile;
+    const int a = rb + piece * S.tile, b = min(a + S.tile, re);
+    T s = T(0);
+    for (int e = a + lane; e < b; e += 128) {
+        int c[4];
+        T v[4], g[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) c[u] = e + 32 * u < b ? ld_cs(S.cidx + e + 32 * u) : 0;
+#pragma unroll
+        for (int u = 0; u < 4; u++) v[u] = e + 32 * u < b ? ld_stream(S.cval + e + 32 * u) : T(0);
+#pragma unroll
+        for (int u = 0; u < 4; u++) g[u] = gather<false>(x + c[u]);
+#pragma unroll
+        for (int u = 0; u < 4; u++)
+            if (e + 32 * u < b) {
+                if constexpr (sizeof(T) == 8) s = __fma_rn(v[u], g[u], s);
+                else s = add_rn(s, mul_rn(v[u], g[u]));
+            }
+    }
+    s = warp_sum_tree(s);
+    if (npieces == 1) {
+        if (lane == 0) epi.row_long(0, row, s, lid, acc);
+        return;
+    }
+    int done = 0;
+    if (lane == 0) {
+        S.partials[slot + piece] = s;
+        __threadfence();
+        done = atomicAdd(&S.counters[lid], 1);
+    }
+    done = __shfl_sync(FULL_MASK, done, 0);
+    if (done == npieces - 1 && lane == 0) {
+        __threadfence();
+        T tot = T(0);
+        for (int q = 0; q < npieces; q++) tot = add_rn(tot, __ldcg(S.partials + slot + q));
+        epi.row_long(0, row, tot, lid, acc);
+        S.counters[lid] = 0;
+    }
+}
+
+// the long pieces first (they take longest), then a warp per slice
+template <int WARPS, class T, class Epi>
+__global__ void __launch_bounds__(WARPS * 32)
+    k_sell(const SellView<T> S, const T* __restrict__ x, Epi epi) {
+    const int lane = threadIdx.x & 31;
+    const int task = blockIdx.x * WARPS + (threadIdx.x >> 5);
+    typename Epi::Acc acc;
+    epi.init(acc);
+    if (task < S.nltasks) {
+        sell_piece(S, x, epi, acc, S.ltasks[task], lane);
+    } else if (task - S.nltasks < S.nslices) {
+        const int s = task - S.nltasks, k = s * 32 + lane;
+        const int o = ld_keep(S.off + s), w = ld_keep(S.off + s + 1) - o;
+        const int len = S.len[k];
+        const int r = S.perm ? ld_keep(S.perm + k) : k;
+        const bool in = len != SELL_SKIP;
+        typename Epi::Pre pre{};
+        if (in) pre = epi.pre_global(r);
+        const T sum = sell_row(S.idx + (int64_t)o * 32 + lane, S.val + (int64_t)o * 32 + lane, w,
+                               in ? len : 0, x);
+        if (in) epi.row(0, r, sum, pre, acc);
+    }
+    epi.finish(acc);
+}
+
+// Eight warps a block; two when the whole grid is small, so that it covers all
+// SMs (an FP64 block of eight warps keeps one SM's FP64 pipe busy while others
+// are idle).
+template <class T, class Epi>
+void launch_sell(const SellView<T>& S, const T* x, const Epi& epi, cudaStream_t s) {
+    const int64_t tasks = (int64_t)S.nslices + S.nltasks;
+    if (tasks == 0 || tiles_dry_run()) return;
+    if (tasks < 152 * 16)
+        k_sell<2, T, Epi><<<(unsigned)((tasks + 1) / 2), 64, 0, s>>>(S, x, epi);
+    else
+        k_sell<8, T, Epi><<<(unsigned)((tasks + 7) / 8), 256, 0, s>>>(S, x, epi);
+    CK_LAUNCH();
+}
+
+}  // namespace cpdlp

@@ -421,6 +421,15 @@ EllView<V, VT> ell_view(const ProblemT<T>& P, int side, const int32_t* ptr) {
 template <int W = TILE_WARPS, int NVEC, class V, class VT, class Epi, class T>
 void launch_side(const ProblemT<T>& P, int side, const CsrView<V, VT>& view,
                  const VecSet<VT, NVEC>& xs, const Epi& epi, cudaStream_t s) {
+    // epilogues without block reductions over the problem's own values: the
+    // sliced engine, where the problem has it
+    if constexpr (std::is_same<typename Epi::Acc, NoAcc>::value && std::is_same<V, T>::value &&
+                  std::is_same<VT, T>::value && NVEC == 1) {
+        if (P.sell[side].on) {
+            launch_sell(sell_view<T>(P.sell[side], view.ptr, view.idx, view.val), xs.v[0], epi, s);
+            return;
+        }
+    }
     if (P.fmt[side] == CPDLP_FMT_ELL)
         launch_ell<W>(ell_view<V, VT>(P, side, view.ptr), xs, epi, s);
     else
@@ -477,6 +486,7 @@ void build_ell(Handle& h, ProblemT<T>& P, int side, const std::vector<int32_t>& 
 // candidate is at least 3% faster.  Decisions are cached per matrix shape and
 // requested format for the process.  With ELL chosen the slabs stay in P.
 constexpr int64_t AUTOTUNE_MIN_NNZ = 1 << 21;
+constexpr int FMT_SELL = -1;  // the tuner's name for the sliced engine (internal)
 // ELL is a candidate when its slabs hold at most this many times the nonzeros
 constexpr int64_t ELL_MAX_PADDING = 3;
 
@@ -559,6 +569,66 @@ SideChoice tune_side(Handle& h, ProblemT<T>& P, int side, const std::vector<int3
     std::lock_guard<std::mutex> lock(mu);
     cache[key] = best;
     return best;
+}
+
+// the slices may hold this many times the nonzeros; FP32 without the
+// autotuner: the share of the nonzeros in rows longer than LONG_ROW
+constexpr double SELL_MAX_PADDING = 1.5;
+constexpr double SELL_MAX_LONG_F32 = 0.05;
+
+// The sliced engine against the tile plan the autotuner chose for this side:
+// kept when its step kernel is 3% faster; decided once per matrix shape.
+template <class T, class Launch>
+void tune_sell(Handle& h, ProblemT<T>& P, int side, const std::vector<int32_t>& hp, int items,
+               Launch&& launch) {
+    if (P.fmt[side] != CPDLP_FMT_CSR) return;
+    static std::mutex mu;
+    static std::map<std::tuple<int64_t, int64_t, int64_t, int, int, int, int, bool>, bool> cache;
+    const int64_t rows = side_rows(P, side), cols = side_rows(P, 1 - side);
+    const auto key = std::make_tuple(rows, cols, P.nnz, (int)sizeof(T), h.device, side, items, P.ordered);
+    int decided = -1;
+    {
+        std::lock_guard<std::mutex> lock(mu);
+        auto it = cache.find(key);
+        if (it != cache.end()) decided = it->second ? 1 : 0;
+    }
+    if (decided == 0) return;
+    cudaStream_t s = h.stream;
+    SellSide<T>& S = P.sell[side];
+    build_sell<T>(S, hp, side == 0 ? P.a_ptr.p : P.at_ptr.p, side == 0 ? P.a_idx.p : P.at_idx.p,
+                  side == 0 ? P.a_val.p : P.at_val.p, rows, 32 * items, s);
+    bool keep = (double)S.entries <= SELL_MAX_PADDING * (double)P.nnz;
+    if (decided < 0 && keep) {
+        struct Events {
+            cudaEvent_t e[2] = {};
+            ~Events() { for (cudaEvent_t x : e) if (x) cudaEventDestroy(x); }
+        } ev;
+        for (cudaEvent_t& e : ev.e) CK(cudaEventCreate(&e));
+        TilePlan plan;
+        build_tile_plan(hp, (int32_t)rows, items, plan, s);
+        DBuf<T> part((size_t)std::max(plan.npieces, 1));
+        auto timed = [&](int fmt) {
+            launch(fmt, plan, part.p);
+            CK(cudaEventRecord(ev.e[0], s));
+            for (int r = 0; r < 4; r++) launch(fmt, plan, part.p);
+            CK(cudaEventRecord(ev.e[1], s));
+            CK(cudaEventSynchronize(ev.e[1]));
+            float ms = 0.f;
+            CK(cudaEventElapsedTime(&ms, ev.e[0], ev.e[1]));
+            return ms;
+        };
+        const float tiles = timed(CPDLP_FMT_CSR), slices = timed(FMT_SELL);
+        keep = slices < 0.97f * tiles;
+        if (trace_level() > 0)
+            fprintf(stderr, "[cpdlp setup]   side %d: tiles %.4f ms, slices %.4f ms (%.3f entries a nonzero)\n",
+                    side, tiles / 4, slices / 4, (double)S.entries / (double)std::max<int64_t>(P.nnz, 1));
+    }
+    if (decided < 0) {
+        std::lock_guard<std::mutex> lock(mu);
+        cache[key] = keep;
+    }
+    S.on = keep;
+    if (!keep) S.release();
 }
 
 // device reduction of (rows x q) partials into host doubles
@@ -912,7 +982,8 @@ ProblemBase* make_problem(Handle& h, const cpdlp_lp* lp, const cpdlp_params* prm
                 const CsrView<T, T> V{Q->at_ptr.p, Q->at_idx.p, Q->at_val.p, pl.tasks.p, pl.ntasks,
                                       pl.ltasks.p, pl.nltasks, pl.counters.p, part};
                 PrimalEpi<T> pe{vx.p, Q->c.p, Q->lv.p, Q->uv.p, vxn.p, vxb.p, vxa.p, vxa2.p, {cf.p}, 1};
-                if (fmt == CPDLP_FMT_ELL) launch_ell<TILE_WARPS>(ell_view<T, T>(*Q, 1, Q->at_ptr.p), VecSet<T, 1>{{vy.p}}, pe, s);
+                if (fmt == FMT_SELL) launch_sell(sell_view<T>(Q->sell[1], V.ptr, V.idx, V.val), vy.p, pe, s);
+                else if (fmt == CPDLP_FMT_ELL) launch_ell<TILE_WARPS>(ell_view<T, T>(*Q, 1, Q->at_ptr.p), VecSet<T, 1>{{vy.p}}, pe, s);
                 else launch_tiles<1>(pl, V, VecSet<T, 1>{{vy.p}}, pe, s);
             }
         };
@@ -928,7 +999,8 @@ ProblemBase* make_problem(Handle& h, const cpdlp_lp* lp, const cpdlp_params* prm
                 const CsrView<T, T> V{Q->a_ptr.p, Q->a_idx.p, Q->a_val.p, pl.tasks.p, pl.ntasks,
                                       pl.ltasks.p, pl.nltasks, pl.counters.p, part};
                 DualEpi<T> de{vy.p, Q->lc.p, Q->uc.p, vyn.p, vya.p, vya2.p, {cf.p}, 1};
-                if (fmt == CPDLP_FMT_ELL) launch_ell<TILE_WARPS>(ell_view<T, T>(*Q, 0, Q->a_ptr.p), VecSet<T, 1>{{vxb.p}}, de, s);
+                if (fmt == FMT_SELL) launch_sell(sell_view<T>(Q->sell[0], V.ptr, V.idx, V.val), vxb.p, de, s);
+                else if (fmt == CPDLP_FMT_ELL) launch_ell<TILE_WARPS>(ell_view<T, T>(*Q, 0, Q->a_ptr.p), VecSet<T, 1>{{vxb.p}}, de, s);
                 else launch_tiles<1>(pl, V, VecSet<T, 1>{{vxb.p}}, de, s);
             }
         };
@@ -1002,11 +1074,32 @@ ProblemBase* make_problem(Handle& h, const cpdlp_lp* lp, const cpdlp_params* prm
             cudaEventDestroy(e0);
             cudaEventDestroy(e1);
         }
+        // the sliced engine as a candidate on each side that stayed with CSR
+        if (!pm1) {
+            tune_sell<T>(h, *P, 1, hp1, items_At, launch_At);
+            tune_sell<T>(h, *P, 0, hp2, items_A, launch_A);
+        }
     }
     mark("formats, autotuner, density order");
-    // a small LP runs its blocks on the resident kernels: with the library's own
-    // choice of engine (no ELL, no pinned tile size) and valued storage
-    if (!pm1 && mt != CPDLP_FMT_ELL && prm->tile_nnz == 0) res_single_build<T>(*P, hp2, hp1, s);
+    // below the autotuner's sizes, with the library's own choice of engine (no
+    // ELL, no pinned tile size) and valued storage: a small LP runs its blocks on
+    // the resident kernels, others step on the sliced engine, where its padding
+    // is small and, in FP32, few entries are in long rows (us a step, tiles and
+    // slices: FP64 flow 63,000 nonzeros 8.9, 5.5, random 1,000,000 42.7, 20.2,
+    // power-law 240,000 with a quarter in long rows 17.1, 14.7; FP32 random
+    // 1,000,000 15.7, 14.2, 200,000 9.3, 7.8, power-law 240,000 10.1, 10.9)
+    if (!tune && !pm1 && mt != CPDLP_FMT_ELL && prm->tile_nnz == 0) {
+        res_single_build<T>(*P, hp2, hp1, s);
+        for (int side = 0; side < 2 && P->rlp.cs == 0 && nnz > 0; side++) {
+            SellSide<T>& S = P->sell[side];
+            build_sell<T>(S, side == 0 ? hp2 : hp1, side == 0 ? P->a_ptr.p : P->at_ptr.p,
+                          side == 0 ? P->a_idx.p : P->at_idx.p, side == 0 ? P->a_val.p : P->at_val.p,
+                          side_rows(*P, side), 32 * (side == 0 ? items_A : items_At), s);
+            S.on = (double)S.entries <= SELL_MAX_PADDING * (double)nnz &&
+                   (sizeof(T) == 8 || (double)S.long_nnz <= SELL_MAX_LONG_F32 * (double)nnz);
+            if (!S.on) S.release();
+        }
+    }
     // the CSR plans (also kept for an ELL side: the tuner and the exports use them),
     // the two on two host threads (each a sequential pass over its rows)
     {

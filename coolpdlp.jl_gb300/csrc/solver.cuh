@@ -5,6 +5,7 @@
 
 #include "cpdlp_common.cuh"
 #include "resident_plan.cuh"
+#include "sell.cuh"
 #include "sparse_build.cuh"
 #include "tiles.cuh"
 
@@ -82,6 +83,8 @@ struct ProblemT : ProblemBase {
     // value arrays are empty, and the products apply d1 / d2 (as T)
     bool pm1 = false;
     DBuf<T> d1t, d2t;
+    // the step engine's slices of each matrix ([0]: rows of A, [1]: rows of A')
+    SellSide<T> sell[2];
     // a small LP's slices for the resident kernels (rlp.cs = 0: not resident)
     ResStore<T> res;
     ResLP rlp{};
