@@ -12,6 +12,7 @@
 // in the index (~col for -1) and has no value slab.
 #pragma once
 
+#include "sell.cuh"
 #include "tiles.cuh"
 
 namespace cpdlp {
@@ -24,48 +25,37 @@ struct EllView {
     int64_t rows;
 };
 
-// one row: sum_k val[k] * x[idx[k]] in k order, four entries' loads and
-// gathers issued together
-template <class V, class T>
-__device__ __forceinline__ T ell_row(const EllView<V, T>& A, int64_t r, int len,
-                                     const T* __restrict__ xv) {
-    T sum = T(0);
-    int k = 0;
-    for (; k + 4 <= len; k += 4) {
-        int c[4];
-        T v[4], g[4];
-#pragma unroll
-        for (int u = 0; u < 4; u++) {
-            c[u] = __ldcs(A.idx + r + (int64_t)(k + u) * A.rows);
-            if constexpr (!is_pm1<V>::value) v[u] = load1v<V, T>(A.val + r + (int64_t)(k + u) * A.rows);
-        }
-#pragma unroll
-        for (int u = 0; u < 4; u++) g[u] = gather<false>(xv + (is_pm1<V>::value ? pm1_col(c[u]) : c[u]));
-#pragma unroll
-        for (int u = 0; u < 4; u++)
-            sum = add_rn(sum, is_pm1<V>::value ? pm1_apply(c[u], g[u]) : mul_rn(v[u], g[u]));
-    }
-    for (; k < len; k++) {
-        const int c = __ldcs(A.idx + r + (int64_t)k * A.rows);
-        const T g = gather<false>(xv + (is_pm1<V>::value ? pm1_col(c) : c));
-        if constexpr (is_pm1<V>::value) sum = add_rn(sum, pm1_apply(c, g));
-        else sum = add_rn(sum, mul_rn(load1v<V, T>(A.val + r + (int64_t)k * A.rows), g));
-    }
-    return sum;
-}
-
+// A row's entries are summed in column order (row_sum: up to eight entries'
+// loads, then their gathers, are in flight together; the warp runs to its
+// longest row, the padding of the others is stored).  The flow LP's columns of
+// three entries went one dependent gather after another before.
 template <int WARPS, int NVEC, class V, class T, class Epi>
 __global__ void __launch_bounds__(WARPS * 32)
     k_ell(EllView<V, T> A, VecSet<T, NVEC> xs, Epi epi) {
     const int64_t r = (int64_t)blockIdx.x * (WARPS * 32) + threadIdx.x;
     typename Epi::Acc acc;
     epi.init(acc);
-    if (r < A.rows) {
-        const int a = ld_keep(A.ptr + r);
-        const int len = ld_keep(A.ptr + r + 1) - a;
-        const typename Epi::Pre pre = epi.pre_global((int)r);
+    const bool in = r < A.rows;
+    const int len = in ? ld_keep(A.ptr + r + 1) - ld_keep(A.ptr + r) : 0;
+    const int w = __reduce_max_sync(FULL_MASK, len);
+    // (lanes without a row walk the last one's entries)
+    const int64_t k = in ? r : A.rows - 1;
+    typename Epi::Pre pre{};
+    if constexpr (epi_split<Epi>::value)
+        if (in) pre = epi.pre_static((int)r);
 #pragma unroll 1
-        for (int p = 0; p < NVEC; p++) epi.row(p, (int)r, ell_row(A, r, len, pick(xs.v, p)), pre, acc);
+    for (int p = 0; p < NVEC; p++) {
+        const V* vp = nullptr;
+        if constexpr (!is_pm1<V>::value) vp = A.val + k;
+        const T sum = row_sum<true>(A.idx + k, vp, A.rows, w, len, pick(xs.v, p), [&] {
+            if (p > 0) return;
+            grid_wait();
+            grid_release();
+            if constexpr (epi_split<Epi>::value) {
+                if (in) epi.pre_dynamic((int)r, pre);
+            } else if (in) pre = epi.pre_global((int)r);
+        });
+        if (in) epi.row(p, (int)r, sum, pre, acc);
     }
     epi.finish(acc);
 }
@@ -150,7 +140,11 @@ inline unsigned ell4_grid(int64_t rows, int warps, int64_t max_blocks) {
 template <int WARPS, int NVEC, class V, class T, class Epi>
 void launch_ell(const EllView<V, T>& A, const VecSet<T, NVEC>& xs, const Epi& epi, cudaStream_t s) {
     if (A.rows == 0 || tiles_dry_run()) return;
-    k_ell<WARPS, NVEC, V, T, Epi><<<ell_grid(A.rows, WARPS), WARPS * 32, 0, s>>>(A, xs, epi);
+    const unsigned grid = ell_grid(A.rows, WARPS);
+    if (chain_this((int64_t)grid * WARPS * 32, is_pm1<V>::value ? 0 : (int)sizeof(T)))
+        launch_chained(k_ell<WARPS, NVEC, V, T, Epi>, grid, WARPS * 32u, s, A, xs, epi);
+    else
+        k_ell<WARPS, NVEC, V, T, Epi><<<grid, WARPS * 32, 0, s>>>(A, xs, epi);
     CK_LAUNCH();
 }
 template <int WARPS, class V, class T, class Epi>

@@ -5,6 +5,8 @@
 // Epilogue interface (per row r, per input vector p):
 //   struct Pre;                      inputs of one row, loaded before the gathers
 //   Pre pre_global(int r) const;     loads them
+//   SPLIT (the step epilogues): pre_global in two parts, pre_static for what no
+//   kernel of a step chain writes and pre_dynamic for the rest
 //   void row(int p, int r, T s, const Pre&, Acc&)   rows of short tiles
 //   void row_long(int p, int r, T s, int lid, Acc&)  long rows (one lane)
 //   void init(Acc&); void finish(Acc&);             block reductions
@@ -86,10 +88,20 @@ struct PrimalEpi {
     int avg;
     const T* __restrict__ dsc;  // SCALED: d2
     using Acc = NoAcc;
+    static constexpr bool SPLIT = true;
     struct Pre { T x, c, lv, uv, xa, d; };
+    __device__ __forceinline__ Pre pre_static(int j) const {
+        return Pre{T(0), ld_stream(c + j), ld_stream(lv + j), ld_stream(uv + j), T(0),
+                   SCALED ? ld_stream(dsc + j) : T(0)};
+    }
+    __device__ __forceinline__ void pre_dynamic(int j, Pre& q) const {
+        q.x = ld_stream(x + j);
+        q.xa = avg ? ld_stream(xa_old + j) : T(0);
+    }
     __device__ __forceinline__ Pre pre_global(int j) const {
-        return Pre{ld_stream(x + j), ld_stream(c + j), ld_stream(lv + j), ld_stream(uv + j),
-                   avg ? ld_stream(xa_old + j) : T(0), SCALED ? ld_stream(dsc + j) : T(0)};
+        Pre q = pre_static(j);
+        pre_dynamic(j, q);
+        return q;
     }
     __device__ void init(Acc&) {}
     __device__ __forceinline__ void row(int, int j, T s, const Pre& q, Acc&) {
@@ -127,10 +139,19 @@ struct DualEpi {
     T* __restrict__ ysn;         // SCALED: d1 .* y+
     const double* __restrict__ yoff;  // SHIFT: scaled base multipliers
     using Acc = NoAcc;
+    static constexpr bool SPLIT = true;
     struct Pre { T y, lc, uc, ya, d; };
+    __device__ __forceinline__ Pre pre_static(int i) const {
+        return Pre{T(0), ld_stream(lc + i), ld_stream(uc + i), T(0), SCALED ? ld_stream(dsc + i) : T(0)};
+    }
+    __device__ __forceinline__ void pre_dynamic(int i, Pre& q) const {
+        q.y = ld_stream(y + i);
+        q.ya = avg ? ld_stream(ya_old + i) : T(0);
+    }
     __device__ __forceinline__ Pre pre_global(int i) const {
-        return Pre{ld_stream(y + i), ld_stream(lc + i), ld_stream(uc + i),
-                   avg ? ld_stream(ya_old + i) : T(0), SCALED ? ld_stream(dsc + i) : T(0)};
+        Pre q = pre_static(i);
+        pre_dynamic(i, q);
+        return q;
     }
     __device__ void init(Acc&) {}
     __device__ __forceinline__ void row(int, int i, T s, const Pre& q, Acc&) {

@@ -78,70 +78,99 @@ __device__ __forceinline__ int ld_cs(const int32_t* p) {
     asm volatile("ld.global.cs.s32 %0, [%1];" : "=r"(v) : "l"(p));
     return v;
 }
-// N entries of a row from place p (stride 32): all loads, then all gathers, are
-// in flight together; entries beyond the row's length add -0 (its padding has
-// value 0 and index 0)
-template <int N, class T>
-__device__ __forceinline__ T sell_chunk(const int32_t* ip, const T* vp, int len,
-                                        const T* __restrict__ x, T s) {
+// N entries of a row from place ip / vp (stride `step`): the loads of all
+// entries are in flight together, then, after mid(), all gathers; entries
+// beyond the row's length add -0 (its padding has value 0 and index 0).
+// COH: the gathered vector may have been written by the kernel before, which ran
+// at the same time (a chained launch).
+template <int N, bool COH, class V, class T, class Mid>
+__device__ __forceinline__ T row_chunk(const int32_t* ip, const V* vp, int64_t step, int len,
+                                       const T* x, T s, Mid&& mid) {
     int c[N];
     T v[N], g[N];
 #pragma unroll
-    for (int u = 0; u < N; u++) c[u] = ld_cs(ip + u * 32);
+    for (int u = 0; u < N; u++) c[u] = ld_cs(ip + u * step);
+    if constexpr (!is_pm1<V>::value) {
 #pragma unroll
-    for (int u = 0; u < N; u++) v[u] = ld_stream(vp + u * 32);
+        for (int u = 0; u < N; u++) v[u] = (T)ld_stream(vp + u * step);
+    }
+    mid();
 #pragma unroll
-    for (int u = 0; u < N; u++) g[u] = gather<false>(x + c[u]);
+    for (int u = 0; u < N; u++) g[u] = gather<COH>(x + (is_pm1<V>::value ? pm1_col(c[u]) : c[u]));
 #pragma unroll
     for (int u = 0; u < N; u++) {
-        if constexpr (sizeof(T) == 8) s = __fma_rn(v[u], u < len ? g[u] : T(-0.0), s);
-        else {
+        if constexpr (is_pm1<V>::value) {
+            s = add_rn(s, u < len ? pm1_apply(c[u], g[u]) : T(-0.0));
+        } else if constexpr (sizeof(T) == 8) {
+            s = __fma_rn(v[u], u < len ? g[u] : T(-0.0), s);
+        } else {
             const T p = mul_rn(v[u], g[u]);
             s = add_rn(s, u < len ? p : T(-0.0));
         }
     }
     return s;
 }
-template <class T>
-__device__ __forceinline__ T sell_row(const int32_t* ip, const T* vp, int w, int len,
-                                      const T* __restrict__ x) {
-    T s = T(0);
-#pragma unroll 1
-    for (; w > 8; w -= 8, len -= 8, ip += 256, vp += 256) s = sell_chunk<8>(ip, vp, len, x, s);
+template <bool COH, class V, class T, class Mid>
+__device__ __forceinline__ T row_rest(const int32_t* ip, const V* vp, int64_t step, int w, int len,
+                                      const T* x, T s, Mid&& mid) {
     switch (w) {
-        case 8: return sell_chunk<8>(ip, vp, len, x, s);
-        case 7: return sell_chunk<7>(ip, vp, len, x, s);
-        case 6: return sell_chunk<6>(ip, vp, len, x, s);
-        case 5: return sell_chunk<5>(ip, vp, len, x, s);
-        case 4: return sell_chunk<4>(ip, vp, len, x, s);
-        case 3: return sell_chunk<3>(ip, vp, len, x, s);
-        case 2: return sell_chunk<2>(ip, vp, len, x, s);
-        case 1: return sell_chunk<1>(ip, vp, len, x, s);
-        default: return s;
+        case 8: return row_chunk<8, COH>(ip, vp, step, len, x, s, mid);
+        case 7: return row_chunk<7, COH>(ip, vp, step, len, x, s, mid);
+        case 6: return row_chunk<6, COH>(ip, vp, step, len, x, s, mid);
+        case 5: return row_chunk<5, COH>(ip, vp, step, len, x, s, mid);
+        case 4: return row_chunk<4, COH>(ip, vp, step, len, x, s, mid);
+        case 3: return row_chunk<3, COH>(ip, vp, step, len, x, s, mid);
+        case 2: return row_chunk<2, COH>(ip, vp, step, len, x, s, mid);
+        case 1: return row_chunk<1, COH>(ip, vp, step, len, x, s, mid);
+        default: mid(); return s;
     }
+}
+// A whole row of w stored entries (uniform over the warp), len of them its own;
+// mid() runs once, between the first entries' loads and their gathers.
+template <bool COH, class V, class T, class Mid>
+__device__ __forceinline__ T row_sum(const int32_t* ip, const V* vp, int64_t step, int w, int len,
+                                     const T* x, Mid&& mid) {
+    auto none = [] {};
+    T s = T(0);
+    if (w <= 8) return row_rest<COH>(ip, vp, step, w, len, x, s, mid);
+    s = row_chunk<8, COH>(ip, vp, step, len, x, s, mid);
+#pragma unroll 1
+    for (;;) {
+        w -= 8;
+        len -= 8;
+        ip += 8 * step;
+        if constexpr (!is_pm1<V>::value) vp += 8 * step;
+        if (w <= 8) break;
+        s = row_chunk<8, COH>(ip, vp, step, len, x, s, none);
+    }
+    return row_rest<COH>(ip, vp, step, w, len, x, s, none);
 }
 
 // one piece of a row longer than LONG_ROW (long_piece in tiles.cuh, with the
-// piece size at run time and four entries' loads in flight)
-template <class T, class Epi>
-__device__ __forceinline__ void sell_piece(const SellView<T>& S, const T* __restrict__ x, Epi& epi,
+// piece size at run time and LU entries' loads in flight)
+template <bool COH, int LU = 4, class T, class Epi>
+__device__ __forceinline__ void sell_piece(const SellView<T>& S, const T* x, Epi& epi,
                                            typename Epi::Acc& acc, int4 t, int lane) {
     const int row = t.x, piece = -t.y - 1, lid = t.z, slot = t.w;
     const int rb = ld_keep(S.ptr + row), re = ld_keep(S.ptr + row + 1);
     const int npieces = (re - rb + S.tile - 1) / S.tile;
     const int a = rb + piece * S.tile, b = min(a + S.tile, re);
+    if (COH) {
+        grid_wait();
+        grid_release();
+    }
     T s = T(0);
-    for (int e = a + lane; e < b; e += 128) {
-        int c[4];
-        T v[4], g[4];
+    for (int e = a + lane; e < b; e += 32 * LU) {
+        int c[LU];
+        T v[LU], g[LU];
 #pragma unroll
-        for (int u = 0; u < 4; u++) c[u] = e + 32 * u < b ? ld_cs(S.cidx + e + 32 * u) : 0;
+        for (int u = 0; u < LU; u++) c[u] = e + 32 * u < b ? ld_cs(S.cidx + e + 32 * u) : 0;
 #pragma unroll
-        for (int u = 0; u < 4; u++) v[u] = e + 32 * u < b ? ld_stream(S.cval + e + 32 * u) : T(0);
+        for (int u = 0; u < LU; u++) v[u] = e + 32 * u < b ? ld_stream(S.cval + e + 32 * u) : T(0);
 #pragma unroll
-        for (int u = 0; u < 4; u++) g[u] = gather<false>(x + c[u]);
+        for (int u = 0; u < LU; u++) g[u] = gather<COH>(x + c[u]);
 #pragma unroll
-        for (int u = 0; u < 4; u++)
+        for (int u = 0; u < LU; u++)
             if (e + 32 * u < b) {
                 if constexpr (sizeof(T) == 8) s = __fma_rn(v[u], g[u], s);
                 else s = add_rn(s, mul_rn(v[u], g[u]));
@@ -168,16 +197,19 @@ __device__ __forceinline__ void sell_piece(const SellView<T>& S, const T* __rest
     }
 }
 
-// the long pieces first (they take longest), then a warp per slice
-template <int WARPS, class T, class Epi>
+// The long pieces first (they take longest), then a warp per slice.  CHAIN: a
+// chained launch (grid_wait), which loads the entries and the bounds before it
+// waits for the kernel before it.
+template <int WARPS, bool CHAIN, class T, class Epi>
 __global__ void __launch_bounds__(WARPS * 32)
-    k_sell(const SellView<T> S, const T* __restrict__ x, Epi epi) {
+    k_sell(SellView<T> S, const T* x, Epi epi) {
+    constexpr bool SPLIT = CHAIN && epi_split<Epi>::value;
     const int lane = threadIdx.x & 31;
     const int task = blockIdx.x * WARPS + (threadIdx.x >> 5);
     typename Epi::Acc acc;
     epi.init(acc);
     if (task < S.nltasks) {
-        sell_piece(S, x, epi, acc, S.ltasks[task], lane);
+        sell_piece<CHAIN>(S, x, epi, acc, S.ltasks[task], lane);
     } else if (task - S.nltasks < S.nslices) {
         const int s = task - S.nltasks, k = s * 32 + lane;
         const int o = ld_keep(S.off + s), w = ld_keep(S.off + s + 1) - o;
@@ -185,9 +217,20 @@ __global__ void __launch_bounds__(WARPS * 32)
         const int r = S.perm ? ld_keep(S.perm + k) : k;
         const bool in = len != SELL_SKIP;
         typename Epi::Pre pre{};
-        if (in) pre = epi.pre_global(r);
-        const T sum = sell_row(S.idx + (int64_t)o * 32 + lane, S.val + (int64_t)o * 32 + lane, w,
-                               in ? len : 0, x);
+        if (in) {
+            if constexpr (SPLIT) pre = epi.pre_static(r);
+            else if constexpr (!CHAIN) pre = epi.pre_global(r);
+        }
+        const T sum = row_sum<CHAIN>(S.idx + (int64_t)o * 32 + lane, S.val + (int64_t)o * 32 + lane,
+                                     (int64_t)32, w, in ? len : 0, x, [&] {
+                                         if constexpr (CHAIN) {
+                                             grid_wait();
+                                             grid_release();
+                                             if constexpr (SPLIT) {
+                                                 if (in) epi.pre_dynamic(r, pre);
+                                             } else if (in) pre = epi.pre_global(r);
+                                         }
+                                     });
         if (in) epi.row(0, r, sum, pre, acc);
     }
     epi.finish(acc);
@@ -200,10 +243,15 @@ template <class T, class Epi>
 void launch_sell(const SellView<T>& S, const T* x, const Epi& epi, cudaStream_t s) {
     const int64_t tasks = (int64_t)S.nslices + S.nltasks;
     if (tasks == 0 || tiles_dry_run()) return;
-    if (tasks < 152 * 16)
-        k_sell<2, T, Epi><<<(unsigned)((tasks + 1) / 2), 64, 0, s>>>(S, x, epi);
-    else
-        k_sell<8, T, Epi><<<(unsigned)((tasks + 7) / 8), 256, 0, s>>>(S, x, epi);
+    const int warps = tasks < 152 * 16 ? 2 : 8;
+    const unsigned grid = (unsigned)((tasks + warps - 1) / warps);
+    if (chain_this(tasks * 32, (int)sizeof(T))) {
+        if (warps == 2) launch_chained(k_sell<2, true, T, Epi>, grid, 64u, s, S, x, epi);
+        else launch_chained(k_sell<8, true, T, Epi>, grid, 256u, s, S, x, epi);
+    } else {
+        if (warps == 2) k_sell<2, false, T, Epi><<<grid, 64, 0, s>>>(S, x, epi);
+        else k_sell<8, false, T, Epi><<<grid, 256, 0, s>>>(S, x, epi);
+    }
     CK_LAUNCH();
 }
 

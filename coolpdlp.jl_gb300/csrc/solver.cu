@@ -1450,11 +1450,18 @@ struct StateT : StateBase {
         }
         tiles_dry_run() = false;
         CK(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
+        chain_launches() = true;
         int par = parity;
-        for (int k = 0; k < len; k++) {
-            enqueue_step(par, coef.p + k, s);
-            par ^= 1;
+        try {
+            for (int k = 0; k < len; k++) {
+                enqueue_step(par, coef.p + k, s);
+                par ^= 1;
+            }
+        } catch (...) {
+            chain_launches() = false;
+            throw;
         }
+        chain_launches() = false;
         CK(cudaStreamEndCapture(s, &g));
         if (graph[parity]) cudaGraphExecDestroy(graph[parity]);
         CK(cudaGraphInstantiate(&graph[parity], g, 0));

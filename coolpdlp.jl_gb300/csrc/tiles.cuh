@@ -145,8 +145,15 @@ __device__ __forceinline__ void load4v(const double* p, T (&o)[4]) {
     asm volatile("ld.global.cs.v2.f64 {%0, %1}, [%2];" : "=d"(c), "=d"(d) : "l"(p + 2));
     o[0] = (T)a; o[1] = (T)b; o[2] = (T)c; o[3] = (T)d;
 }
+// epilogues whose row inputs split into static and dynamic ones
+template <class E, class = void>
+struct epi_split : std::false_type {};
+template <class E>
+struct epi_split<E, std::enable_if_t<E::SPLIT>> : std::true_type {};
+
 // gathers of x[col]: through the read-only path (COH = false) or with a
-// coherent load (COH = true); same ordering property as the loads above
+// coherent load (COH = true: vectors that a kernel running at the same time
+// wrote); same ordering property as the loads above
 template <bool COH>
 __device__ __forceinline__ float gather(const float* p) {
     float v;
@@ -238,6 +245,7 @@ __device__ __forceinline__ void short_tile(const CsrView<V, T>& A, const VecSet<
                                            Epi& epi, typename Epi::Acc& acc, int r0, int r1,
                                            int nz0, int nz1, int lane, T* prod) {
     constexpr int NV4 = ITEMS / 4 + 1;  // 4-element chunks per lane (+1: alignment slack)
+    constexpr bool SPLIT = epi_split<Epi>::value && !COH;  // a step kernel (k_tiles)
     const int base = nz0 & ~3;
     int ra[RPL], rb[RPL];
     typename Epi::Pre pre[RPL];
@@ -278,7 +286,7 @@ __device__ __forceinline__ void short_tile(const CsrView<V, T>& A, const VecSet<
 #pragma unroll
             for (int q = 0; q < 4; q++)
                 xg[j][q] = (e + q >= nz0 && e + q < nz1)
-                               ? gather<COH>(xv + (is_pm1<V>::value ? pm1_col(cc[j][q]) : cc[j][q]))
+                               ? gather<COH || SPLIT>(xv + (is_pm1<V>::value ? pm1_col(cc[j][q]) : cc[j][q]))
                                : T(0);
         }
         // products to shared memory, indexed from the aligned window start.
@@ -356,6 +364,7 @@ __device__ __forceinline__ void long_piece(const CsrView<V, T>& A, const VecSet<
     const int npieces = (re - rb + TILE - 1) / TILE;
     const int a = rb + piece * TILE;
     const int b = min(a + TILE, re);
+    constexpr bool SPLIT = epi_split<Epi>::value && !COH;
     T s[NVEC];
 #pragma unroll
     for (int p = 0; p < NVEC; p++) s[p] = T(0);
@@ -364,11 +373,12 @@ __device__ __forceinline__ void long_piece(const CsrView<V, T>& A, const VecSet<
         if constexpr (is_pm1<V>::value) {
 #pragma unroll
             for (int p = 0; p < NVEC; p++)
-                s[p] = add_rn(s[p], pm1_apply(cc, gather<COH>(xs.v[p] + pm1_col(cc))));
+                s[p] = add_rn(s[p], pm1_apply(cc, gather<COH || SPLIT>(xs.v[p] + pm1_col(cc))));
         } else {
             const T vv = load1v<V, T>(A.val + e);
 #pragma unroll
-            for (int p = 0; p < NVEC; p++) s[p] = add_rn(s[p], mul_rn(vv, gather<COH>(xs.v[p] + cc)));
+            for (int p = 0; p < NVEC; p++)
+                s[p] = add_rn(s[p], mul_rn(vv, gather<COH || SPLIT>(xs.v[p] + cc)));
         }
     }
 #pragma unroll
@@ -418,6 +428,12 @@ __global__ void __launch_bounds__(WARPS * 32, sizeof(T) == 8 ? CPDLP_F64_MIN_BLO
     __shared__ __align__(16) T prod[WARPS][tile_buf<ITEMS>()];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int task = blockIdx.x * WARPS + w;
+    // a step of a chain waits here, before any load: holding a tile's entries
+    // over the wait took the FP32 kernels from 56-64 to 92-103 registers
+    if constexpr (epi_split<Epi>::value) {
+        grid_wait();
+        grid_release();
+    }
     typename Epi::Acc acc;
     epi.init(acc);
     if (task < A.nltasks) {
@@ -475,10 +491,15 @@ void launch_tiles_w(const TilePlan& plan, const CsrView<V, T>& view, const VecSe
     const int64_t tasks = (int64_t)plan.ntasks + plan.nltasks;
     if (tasks == 0) return;
     const unsigned grid = (unsigned)((tasks + WARPS - 1) / WARPS);
+    const bool chain = chain_this((int64_t)grid * WARPS * 32, is_pm1<V>::value ? 0 : (int)sizeof(T));
+    auto start = [&](auto kern) {
+        if (chain) launch_chained(kern, grid, WARPS * 32, s, view, xs, epi);
+        else kern<<<grid, WARPS * 32, 0, s>>>(view, xs, epi);
+    };
 #define CPDLP_TILES(IT, R, M)                                                 \
     prefer_l1<k_tiles<IT, WARPS, NVEC, V, T, Epi, R, M>>(WARPS * 32, s);      \
     if (!tiles_dry_run())                                                     \
-        k_tiles<IT, WARPS, NVEC, V, T, Epi, R, M><<<grid, WARPS * 32, 0, s>>>(view, xs, epi)
+        start(k_tiles<IT, WARPS, NVEC, V, T, Epi, R, M>)
     if (plan.medium) {
         if (plan.rpl != 2) fail(CPDLP_ERR_ARGUMENT, "tile plan with long rows needs 64-row tiles");
         switch (plan.items) {
