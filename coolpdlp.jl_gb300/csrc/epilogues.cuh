@@ -25,6 +25,7 @@ struct NoAcc {};
 template <class T>
 struct StoreEpi {  // out = s (mul! with alpha = true, beta = false)
     T* out;
+    static constexpr bool CHAIN = true;
     using Acc = NoAcc;
     struct Pre {};
     __device__ Pre pre_global(int) const { return Pre{}; }
@@ -40,6 +41,7 @@ template <class T>
 struct ScaledStoreEpi {
     T* out;
     const T* __restrict__ dsc;
+    static constexpr bool CHAIN = true;
     using Acc = NoAcc;
     struct Pre {};
     __device__ Pre pre_global(int) const { return Pre{}; }
@@ -88,7 +90,7 @@ struct PrimalEpi {
     int avg;
     const T* __restrict__ dsc;  // SCALED: d2
     using Acc = NoAcc;
-    static constexpr bool SPLIT = true;
+    static constexpr bool SPLIT = true, CHAIN = true;
     struct Pre { T x, c, lv, uv, xa, d; };
     __device__ __forceinline__ Pre pre_static(int j) const {
         return Pre{T(0), ld_stream(c + j), ld_stream(lv + j), ld_stream(uv + j), T(0),
@@ -139,7 +141,7 @@ struct DualEpi {
     T* __restrict__ ysn;         // SCALED: d1 .* y+
     const double* __restrict__ yoff;  // SHIFT: scaled base multipliers
     using Acc = NoAcc;
-    static constexpr bool SPLIT = true;
+    static constexpr bool SPLIT = true, CHAIN = true;
     struct Pre { T y, lc, uc, ya, d; };
     __device__ __forceinline__ Pre pre_static(int i) const {
         return Pre{T(0), ld_stream(lc + i), ld_stream(uc + i), T(0), SCALED ? ld_stream(dsc + i) : T(0)};
@@ -370,7 +372,9 @@ struct RayColEpi {
 };
 
 // power method, second product: Ax_j = (A' s)_j; accumulates x.Ax and Ax.Ax
-// (SCALED: the product gathered D1 s and Ax_j is the row sum times d2_j)
+// (SCALED: the product gathered D1 s and Ax_j is the row sum times d2_j).
+// With a ticket, the grid's last block sums the partials (block_out, `rows` of
+// them with the long rows') and leaves theta = x.Ax and 1 / ||Ax|| in scal.
 template <class T, bool SCALED = false>
 struct PowerEpi {
     const T* __restrict__ x;
@@ -378,6 +382,10 @@ struct PowerEpi {
     double* block_out;
     double* long_out;
     const T* __restrict__ dsc = nullptr;
+    unsigned* ticket = nullptr;
+    double* scal = nullptr;
+    int64_t rows = 0;
+    static constexpr bool CHAIN = true;
     struct Acc { double v[2]; };
     struct Pre { T x; };
     __device__ Pre pre_global(int j) const { return Pre{ld_stream(x + j)}; }
@@ -394,7 +402,14 @@ struct PowerEpi {
         long_out[(size_t)lid * 2] = (double)ld_stream(x + j) * (double)s;
         long_out[(size_t)lid * 2 + 1] = (double)s * (double)s;
     }
-    __device__ void finish(Acc& a) { block_reduce_store<2>(a.v, block_out); }
+    __device__ void finish(Acc& a) {
+        block_reduce_store<2>(a.v, block_out);
+        double q[2];
+        if (ticket && last_block_sum<2>(block_out, rows, ticket, q)) {
+            scal[0] = q[0];
+            scal[1] = 1.0 / sqrt(q[1]);
+        }
+    }
 };
 
 }  // namespace cpdlp

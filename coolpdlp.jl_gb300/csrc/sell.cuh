@@ -45,20 +45,22 @@ struct SellSide {
     void release() { *this = SellSide(); }
 };
 
-template <class T>
+// V: the stored values, T: the vectors and sums (FP64 over FP32 values in the
+// power method)
+template <class V, class T = V>
 struct SellView {
     const int32_t* __restrict__ off;
     const uint8_t* __restrict__ len;
     const int32_t* __restrict__ perm;
     const int32_t* __restrict__ idx;
-    const T* __restrict__ val;
+    const V* __restrict__ val;
     const int4* __restrict__ ltasks;
     int32_t* counters;
-    T* partials;
+    T* partials;                       // npieces
     int32_t nslices, nltasks, tile;
     const int32_t* __restrict__ ptr;   // the CSR, for the long rows
     const int32_t* __restrict__ cidx;
-    const T* __restrict__ cval;
+    const V* __restrict__ cval;
 };
 
 // The slices of a CSR (device; hp: its row pointer on the host); tile: the
@@ -67,10 +69,15 @@ template <class T>
 void build_sell(SellSide<T>& S, const std::vector<int32_t>& hp, const int32_t* ptr,
                 const int32_t* idx, const T* val, int64_t rows, int tile, cudaStream_t s);
 
-template <class T>
-SellView<T> sell_view(const SellSide<T>& S, const int32_t* ptr, const int32_t* idx, const T* val) {
-    return SellView<T>{S.off.p, S.len.p, S.perm.p, S.idx.p, S.val.p, S.ltasks.p, S.counters.p,
-                       S.partials.p, S.nslices, S.nltasks, S.tile, ptr, idx, val};
+template <class V, class T>
+SellView<V, T> sell_view(const SellSide<V>& S, const int32_t* ptr, const int32_t* idx, const V* val,
+                         T* partials) {
+    return SellView<V, T>{S.off.p, S.len.p, S.perm.p, S.idx.p, S.val.p, S.ltasks.p, S.counters.p,
+                          partials, S.nslices, S.nltasks, S.tile, ptr, idx, val};
+}
+template <class V>
+SellView<V> sell_view(const SellSide<V>& S, const int32_t* ptr, const int32_t* idx, const V* val) {
+    return sell_view<V, V>(S, ptr, idx, val, S.partials.p);
 }
 
 __device__ __forceinline__ int ld_cs(const int32_t* p) {
@@ -148,8 +155,8 @@ __device__ __forceinline__ T row_sum(const int32_t* ip, const V* vp, int64_t ste
 
 // one piece of a row longer than LONG_ROW (long_piece in tiles.cuh, with the
 // piece size at run time and LU entries' loads in flight)
-template <bool COH, int LU = 4, class T, class Epi>
-__device__ __forceinline__ void sell_piece(const SellView<T>& S, const T* x, Epi& epi,
+template <bool COH, int LU = 4, class V, class T, class Epi>
+__device__ __forceinline__ void sell_piece(const SellView<V, T>& S, const T* x, Epi& epi,
                                            typename Epi::Acc& acc, int4 t, int lane) {
     const int row = t.x, piece = -t.y - 1, lid = t.z, slot = t.w;
     const int rb = ld_keep(S.ptr + row), re = ld_keep(S.ptr + row + 1);
@@ -166,7 +173,7 @@ __device__ __forceinline__ void sell_piece(const SellView<T>& S, const T* x, Epi
 #pragma unroll
         for (int u = 0; u < LU; u++) c[u] = e + 32 * u < b ? ld_cs(S.cidx + e + 32 * u) : 0;
 #pragma unroll
-        for (int u = 0; u < LU; u++) v[u] = e + 32 * u < b ? ld_stream(S.cval + e + 32 * u) : T(0);
+        for (int u = 0; u < LU; u++) v[u] = e + 32 * u < b ? (T)ld_stream(S.cval + e + 32 * u) : T(0);
 #pragma unroll
         for (int u = 0; u < LU; u++) g[u] = gather<COH>(x + c[u]);
 #pragma unroll
@@ -200,9 +207,9 @@ __device__ __forceinline__ void sell_piece(const SellView<T>& S, const T* x, Epi
 // The long pieces first (they take longest), then a warp per slice.  CHAIN: a
 // chained launch (grid_wait), which loads the entries and the bounds before it
 // waits for the kernel before it.
-template <int WARPS, bool CHAIN, class T, class Epi>
+template <int WARPS, bool CHAIN, class V, class T, class Epi>
 __global__ void __launch_bounds__(WARPS * 32)
-    k_sell(SellView<T> S, const T* x, Epi epi) {
+    k_sell(SellView<V, T> S, const T* x, Epi epi) {
     constexpr bool SPLIT = CHAIN && epi_split<Epi>::value;
     const int lane = threadIdx.x & 31;
     const int task = blockIdx.x * WARPS + (threadIdx.x >> 5);
@@ -236,22 +243,34 @@ __global__ void __launch_bounds__(WARPS * 32)
     epi.finish(acc);
 }
 
-// Eight warps a block; two when the whole grid is small, so that it covers all
-// SMs (an FP64 block of eight warps keeps one SM's FP64 pipe busy while others
-// are idle).
-template <class T, class Epi>
-void launch_sell(const SellView<T>& S, const T* x, const Epi& epi, cudaStream_t s) {
+// blocks of a launch of eight warps each (the block-partial rows of a reducing
+// epilogue; its long-row outputs, one per counter, follow)
+template <class V>
+int64_t sell_blocks(const SellSide<V>& S) {
+    return ((int64_t)S.nslices + S.nltasks + TILE_WARPS - 1) / TILE_WARPS;
+}
+
+// Eight warps a block; two, without a reducing epilogue, when the whole grid is
+// small, so that it covers all SMs (an FP64 block of eight warps keeps one SM's
+// FP64 pipe busy while others are idle).
+template <class V, class T, class Epi>
+void launch_sell(const SellView<V, T>& S, const T* x, const Epi& epi, cudaStream_t s) {
     const int64_t tasks = (int64_t)S.nslices + S.nltasks;
     if (tasks == 0 || tiles_dry_run()) return;
-    const int warps = tasks < 152 * 16 ? 2 : 8;
-    const unsigned grid = (unsigned)((tasks + warps - 1) / warps);
-    if (chain_this(tasks * 32, (int)sizeof(T))) {
-        if (warps == 2) launch_chained(k_sell<2, true, T, Epi>, grid, 64u, s, S, x, epi);
-        else launch_chained(k_sell<8, true, T, Epi>, grid, 256u, s, S, x, epi);
-    } else {
-        if (warps == 2) k_sell<2, false, T, Epi><<<grid, 64, 0, s>>>(S, x, epi);
-        else k_sell<8, false, T, Epi><<<grid, 256, 0, s>>>(S, x, epi);
+    constexpr bool REDUCES = !std::is_empty<typename Epi::Acc>::value;
+    const bool chain = chain_this(tasks * 32, (int)sizeof(T));
+    if constexpr (!REDUCES) {
+        if (tasks < 152 * 16) {
+            const unsigned grid = (unsigned)((tasks + 1) / 2);
+            if (chain) launch_chained(k_sell<2, true, V, T, Epi>, grid, 64u, s, S, x, epi);
+            else k_sell<2, false, V, T, Epi><<<grid, 64, 0, s>>>(S, x, epi);
+            CK_LAUNCH();
+            return;
+        }
     }
+    const unsigned grid = (unsigned)((tasks + TILE_WARPS - 1) / TILE_WARPS);
+    if (chain) launch_chained(k_sell<TILE_WARPS, true, V, T, Epi>, grid, TILE_WARPS * 32u, s, S, x, epi);
+    else k_sell<TILE_WARPS, false, V, T, Epi><<<grid, TILE_WARPS * 32, 0, s>>>(S, x, epi);
     CK_LAUNCH();
 }
 

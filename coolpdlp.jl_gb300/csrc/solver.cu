@@ -258,47 +258,42 @@ __global__ void k_scales(const T* __restrict__ lc, const T* __restrict__ uc,
 // ---------------------------------------------------------------------------
 // epilogues of the tile engine
 // ---------------------------------------------------------------------------
-// One power-method iteration is captured as a graph and runs without the host:
-//   k_power_theta:    theta = x.Ax, inv = 1/||Ax|| from the reduced partials
-//   k_power_residual: r = Ax - theta*x, x = Ax * inv (block partials of ||r||^2)
-//   k_power_finish:   ||r||, then the iteration's (theta, ||r||) go to slot it % depth
-//                     of a mapped host ring and the device iteration counter advances
-// so the host can queue several iterations ahead and check each one's stopping
-// rule when its slot is written (powm!, linalg.jl:86-96, IterativeSolvers 0.9.4).
+// One power-method iteration is captured as a graph and runs without the host,
+// in three kernels, each started early (grid_wait): the product with A, the
+// product with A' whose last block leaves theta = x.Ax and 1/||Ax|| (PowerEpi),
+// and k_power_residual: r = Ax - theta*x, x = Ax/||Ax||, whose last block writes
+// (theta, ||r||) to slot it % depth of a mapped host ring and advances the
+// device iteration counter.  (With reductions and scalars in kernels of their
+// own, seven in all, an iteration of a 63,000-nonzero LP took 25 us.)  The host
+// queues several iterations ahead and checks each one's stopping rule when its
+// slot is written (powm!, linalg.jl:86-96, IterativeSolvers 0.9.4).
 struct PowerSlot {
     double theta, residual;
 };
-__global__ void k_power_theta(const double* __restrict__ q, double* __restrict__ scal,
-                              const int* __restrict__ it, PowerSlot* ring, int depth) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        const double theta = q[0];
-        const double nrm = sqrt(q[1]);
-        scal[0] = theta;
-        scal[1] = 1.0 / nrm;
-        ring[*it % depth].theta = theta;
-    }
-}
 // (d2, xs non-null: a narrow matrix, whose first product gathers xs = d2 .* x)
 __global__ void __launch_bounds__(RED_THREADS)
-    k_power_residual(double* __restrict__ x, const double* __restrict__ Ax,
-                     const double* __restrict__ scal, int64_t n, double* __restrict__ part,
-                     const double* __restrict__ d2, double* __restrict__ xs) {
-    const double theta = scal[0], inv = scal[1];
+    k_power_residual(double* __restrict__ x, const double* __restrict__ Ax, const double* scal,
+                     int64_t n, double* part, const double* __restrict__ d2,
+                     double* __restrict__ xs, unsigned* ticket, int* it, PowerSlot* ring, int depth) {
+    grid_wait();
+    grid_release();
+    const double theta = __ldcg(scal), inv = __ldcg(scal + 1);
     double acc[1] = {0.0};
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < n; j += stride) {
-        const double r = add_rn(mul_rn(-theta, x[j]), Ax[j]);
+        const double ax = __ldcg(Ax + j);
+        const double r = add_rn(mul_rn(-theta, x[j]), ax);
         acc[0] += r * r;
-        const double xn = mul_rn(Ax[j], inv);
+        const double xn = mul_rn(ax, inv);
         x[j] = xn;
         if (xs) xs[j] = mul_rn(d2[j], xn);
     }
     block_reduce_store<1>(acc, part);
-}
-__global__ void k_power_finish(const double* __restrict__ r2, int* it, PowerSlot* ring,
-                               int depth) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        ring[*it % depth].residual = sqrt(r2[0]);
+    double r2[1];
+    if (last_block_sum<1>(part, gridDim.x, ticket, r2)) {
+        PowerSlot* slot = ring + *it % depth;
+        slot->theta = theta;
+        slot->residual = sqrt(r2[0]);
         __threadfence_system();
         *it += 1;
     }
@@ -426,7 +421,7 @@ void launch_side(const ProblemT<T>& P, int side, const CsrView<V, VT>& view,
     if constexpr (std::is_same<typename Epi::Acc, NoAcc>::value && std::is_same<V, T>::value &&
                   std::is_same<VT, T>::value && NVEC == 1) {
         if (P.sell[side].on) {
-            launch_sell(sell_view<T>(P.sell[side], view.ptr, view.idx, view.val), xs.v[0], epi, s);
+            launch_sell(sell_view(P.sell[side], view.ptr, view.idx, view.val), xs.v[0], epi, s);
             return;
         }
     }
@@ -479,16 +474,27 @@ void build_ell(Handle& h, ProblemT<T>& P, int side, const std::vector<int32_t>& 
 }
 
 // Autotuner of one matrix's product (side 0: rows of A, side 1: rows of A'):
-// each candidate -- CSR tile shapes (nonzeros per lane) and, when allowed,
-// ELL -- runs the fused step kernel that uses the matrix (the primal step for
-// A', the dual step for A) on scratch vectors, timed with CUDA events on the
-// handle's stream.  The heuristic's tile shape is kept unless another
-// candidate is at least 3% faster.  Decisions are cached per matrix shape and
-// requested format for the process.  With ELL chosen the slabs stay in P.
+// the fused step kernel that uses the matrix (the primal step for A', the dual
+// step for A) runs on scratch vectors with CSR tiles and, where allowed, ELL,
+// timed with CUDA events on the handle's stream; ELL is kept when it is at
+// least 3% faster.  The engines sum a row of at most LONG_ROW entries in the
+// same order, so the choice does not change FP32 results; the tile size would
+// (it is also the piece size of long rows), so it follows from the size alone
+// (wave_items).  Decisions are cached per matrix shape and requested format for
+// the process.  With ELL chosen the slabs stay in P.
 constexpr int64_t AUTOTUNE_MIN_NNZ = 1 << 21;
 constexpr int FMT_SELL = -1;  // the tuner's name for the sliced engine (internal)
 // ELL is a candidate when its slabs hold at most this many times the nonzeros
 constexpr int64_t ELL_MAX_PADDING = 3;
+
+// Nonzeros per lane of a large matrix's tiles.  Four blocks of eight 512-nonzero
+// tiles are resident on an SM; between 0.95 and 1.39 such waves the last one is
+// nearly empty, and 256-nonzero tiles were 3% to 8% faster (5 of 6 timing runs
+// at 2.7M to 3.3M nonzeros, none at 2.1M or from 3.6M to 24M).
+int wave_items(int64_t nnz, int items, int num_sms) {
+    const double waves = (double)nnz / ((double)num_sms * 4 * TILE_WARPS * 512);
+    return items == 16 && waves > 0.95 && waves < 1.39 ? 8 : items;
+}
 
 struct SideChoice {
     int fmt;
@@ -498,6 +504,7 @@ struct SideChoice {
 template <class T, class Launch>
 SideChoice tune_side(Handle& h, ProblemT<T>& P, int side, const std::vector<int32_t>& hp,
                      int heuristic, bool try_csr, bool try_ell, int which, Launch&& launch) {
+    if (!try_ell) return SideChoice{CPDLP_FMT_CSR, heuristic};
     static std::mutex mu;
     static std::map<std::tuple<int64_t, int64_t, int64_t, int, int, int, int>, SideChoice> cache;
     const int64_t rows = side_rows(P, side), cols = side_rows(P, 1 - side);
@@ -532,17 +539,10 @@ SideChoice tune_side(Handle& h, ProblemT<T>& P, int side, const std::vector<int3
     };
     try {
         if (try_csr) {
-            const int cands[3] = {heuristic, heuristic == 4 ? 8 : 4, heuristic == 16 ? 8 : 16};
-            for (int items : cands) {
-                TilePlan plan;
-                build_tile_plan(hp, (int32_t)rows, items, plan, s);
-                DBuf<T> part((size_t)std::max(plan.npieces, 1));
-                const float ms = timed(CPDLP_FMT_CSR, plan, part.p);
-                if (items == heuristic ? ms < best_ms : ms < 0.97f * best_ms) {
-                    best_ms = ms;
-                    best = SideChoice{CPDLP_FMT_CSR, items};
-                }
-            }
+            TilePlan plan;
+            build_tile_plan(hp, (int32_t)rows, heuristic, plan, s);
+            DBuf<T> part((size_t)std::max(plan.npieces, 1));
+            best_ms = timed(CPDLP_FMT_CSR, plan, part.p);
         }
         if (try_ell) {
             build_ell(h, P, side, hp);
@@ -926,6 +926,10 @@ ProblemBase* make_problem(Handle& h, const cpdlp_lp* lp, const cpdlp_params* prm
     CK(cudaMemcpyAsync(hp1.data(), P->at_ptr.p, sizeof(int32_t) * (n + 1), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
     int items_A = choose_items(nnz, m, prm->tile_nnz), items_At = choose_items(nnz, n, prm->tile_nnz);
+    if (prm->tile_nnz == 0 && nnz >= AUTOTUNE_MIN_NNZ) {
+        items_A = wave_items(nnz, items_A, h.num_sms);
+        items_At = wave_items(nnz, items_At, h.num_sms);
+    }
     // the product format: matrix_type (COO solves on the CSR engine), or the
     // autotuner's choice for large matrices
     const int32_t mt = prm->matrix_type;
@@ -982,7 +986,7 @@ ProblemBase* make_problem(Handle& h, const cpdlp_lp* lp, const cpdlp_params* prm
                 const CsrView<T, T> V{Q->at_ptr.p, Q->at_idx.p, Q->at_val.p, pl.tasks.p, pl.ntasks,
                                       pl.ltasks.p, pl.nltasks, pl.counters.p, part};
                 PrimalEpi<T> pe{vx.p, Q->c.p, Q->lv.p, Q->uv.p, vxn.p, vxb.p, vxa.p, vxa2.p, {cf.p}, 1};
-                if (fmt == FMT_SELL) launch_sell(sell_view<T>(Q->sell[1], V.ptr, V.idx, V.val), vy.p, pe, s);
+                if (fmt == FMT_SELL) launch_sell(sell_view(Q->sell[1], V.ptr, V.idx, V.val), vy.p, pe, s);
                 else if (fmt == CPDLP_FMT_ELL) launch_ell<TILE_WARPS>(ell_view<T, T>(*Q, 1, Q->at_ptr.p), VecSet<T, 1>{{vy.p}}, pe, s);
                 else launch_tiles<1>(pl, V, VecSet<T, 1>{{vy.p}}, pe, s);
             }
@@ -999,7 +1003,7 @@ ProblemBase* make_problem(Handle& h, const cpdlp_lp* lp, const cpdlp_params* prm
                 const CsrView<T, T> V{Q->a_ptr.p, Q->a_idx.p, Q->a_val.p, pl.tasks.p, pl.ntasks,
                                       pl.ltasks.p, pl.nltasks, pl.counters.p, part};
                 DualEpi<T> de{vy.p, Q->lc.p, Q->uc.p, vyn.p, vya.p, vya2.p, {cf.p}, 1};
-                if (fmt == FMT_SELL) launch_sell(sell_view<T>(Q->sell[0], V.ptr, V.idx, V.val), vxb.p, de, s);
+                if (fmt == FMT_SELL) launch_sell(sell_view(Q->sell[0], V.ptr, V.idx, V.val), vxb.p, de, s);
                 else if (fmt == CPDLP_FMT_ELL) launch_ell<TILE_WARPS>(ell_view<T, T>(*Q, 0, Q->a_ptr.p), VecSet<T, 1>{{vxb.p}}, de, s);
                 else launch_tiles<1>(pl, V, VecSet<T, 1>{{vxb.p}}, de, s);
             }
@@ -1214,9 +1218,19 @@ double spectral_norm_T(Handle& h, ProblemT<V>& P, const cpdlp_params* prm, int64
     std::vector<double> x0;
     gaussian_vector(prm->power_seed, n, x0);
     DBuf<double> x((size_t)(n > 0 ? n : 1)), Ax((size_t)(n > 0 ? n : 1)), sv((size_t)(m > 0 ? m : 1));
-    DBuf<double> pA((size_t)std::max(P.planA.npieces, 1)), pAt((size_t)std::max(P.planAt.npieces, 1));
+    DBuf<double> pA((size_t)std::max(std::max(P.planA.npieces, P.sell[0].npieces), 1)),
+        pAt((size_t)std::max(std::max(P.planAt.npieces, P.sell[1].npieces), 1));
     DBuf<double> scal(4);
     DBuf<int> d_it(1);
+    // the second product's partials: its blocks', then its long rows'
+    const bool sell = !P.pm1 && P.sell[1].on;
+    const int64_t blocks = sell ? sell_blocks(P.sell[1]) : side_blocks(P, 1, TILE_WARPS),
+                  rows = sell ? blocks + (int64_t)P.sell[1].counters.n : side_partials(P, 1, TILE_WARPS);
+    DBuf<double> part((size_t)std::max<int64_t>(rows, 1) * 2);
+    DBuf<unsigned> tickets(2);
+    CK(cudaMemsetAsync(part.p, 0, part.bytes(), s));  // (a side without long rows has one unused counter)
+    CK(cudaMemsetAsync(tickets.p, 0, tickets.bytes(), s));
+    CK(cudaMemsetAsync(scal.p, 0, scal.bytes(), s));
     if (n > 0) CK(cudaMemcpyAsync(x.p, x0.data(), sizeof(double) * n, cudaMemcpyHostToDevice, s));
     order_to_internal(P, 1, x.p, s);  // the start vector of the caller's column order
     CK(cudaMemsetAsync(d_it.p, 0, sizeof(int), s));
@@ -1285,24 +1299,25 @@ double spectral_norm_T(Handle& h, ProblemT<V>& P, const cpdlp_params* prm, int64
     {
         cudaGraph_t g = nullptr;
         CK(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-        double* const blk = P.red_cols.p;
-        double* const lng = P.red_cols.p + (size_t)side_blocks(P, 1, TILE_WARPS) * 2;
+        chain_launches() = true;
+        struct Off { ~Off() { chain_launches() = false; } } off;
+        double* const blk = part.p;
+        double* const lng = part.p + (size_t)blocks * 2;
         if (P.pm1) {
             launch_side(P, 0, A1, VecSet<double, 1>{{xs.p}}, ScaledStoreEpi<double>{sv.p, P.D1.p}, s);
-            PowerEpi<double, true> pe{x.p, Ax.p, blk, lng, P.D2.p};
+            PowerEpi<double, true> pe{x.p, Ax.p, blk, lng, P.D2.p, tickets.p, scal.p, rows};
             launch_side(P, 1, At1, VecSet<double, 1>{{sv.p}}, pe, s);
         } else {
-            launch_side(P, 0, A, VecSet<double, 1>{{x.p}}, StoreEpi<double>{sv.p}, s);
-            PowerEpi<double> pe{x.p, Ax.p, blk, lng};
-            launch_side(P, 1, At, VecSet<double, 1>{{sv.p}}, pe, s);
+            const PowerEpi<double> pe{x.p, Ax.p, blk, lng, nullptr, tickets.p, scal.p, rows};
+            const StoreEpi<double> se{sv.p};
+            if (P.sell[0].on) launch_sell(sell_view(P.sell[0], P.a_ptr.p, P.a_idx.p, P.a_val.p, pA.p), (const double*)x.p, se, s);
+            else launch_side(P, 0, A, VecSet<double, 1>{{x.p}}, se, s);
+            if (sell) launch_sell(sell_view(P.sell[1], P.at_ptr.p, P.at_idx.p, P.at_val.p, pAt.p), (const double*)sv.p, pe, s);
+            else launch_side(P, 1, At, VecSet<double, 1>{{sv.p}}, pe, s);
         }
-        reduce_partials(P.red_cols.p, P.rows_At_partials, 2, P.red_out.p, s);
-        k_power_theta<<<1, 32, 0, s>>>(P.red_out.p, scal.p, d_it.p, dring, DEPTH);
-        k_power_residual<<<gr, RED_THREADS, 0, s>>>(x.p, Ax.p, scal.p, n, P.red_rows.p,
-                                                    P.pm1 ? P.D2.p : nullptr,
-                                                    P.pm1 ? xs.p : nullptr);
-        reduce_partials(P.red_rows.p, gr, 1, P.red_out.p + 2, s);
-        k_power_finish<<<1, 32, 0, s>>>(P.red_out.p + 2, d_it.p, dring, DEPTH);
+        launch_chained(k_power_residual, gr, (unsigned)RED_THREADS, s, x.p, (const double*)Ax.p,
+                       (const double*)scal.p, n, P.red_rows.p, (const double*)(P.pm1 ? P.D2.p : nullptr),
+                       P.pm1 ? xs.p : nullptr, tickets.p + 1, d_it.p, dring, DEPTH);
         const cudaError_t launch_err = cudaGetLastError();
         const cudaError_t end_err = cudaStreamEndCapture(s, &g);
         CK(launch_err);

@@ -151,6 +151,12 @@ struct epi_split : std::false_type {};
 template <class E>
 struct epi_split<E, std::enable_if_t<E::SPLIT>> : std::true_type {};
 
+// epilogues that run in chains of kernels (grid_wait)
+template <class E, class = void>
+struct epi_chain : std::false_type {};
+template <class E>
+struct epi_chain<E, std::enable_if_t<E::CHAIN>> : std::true_type {};
+
 // gathers of x[col]: through the read-only path (COH = false) or with a
 // coherent load (COH = true: vectors that a kernel running at the same time
 // wrote); same ordering property as the loads above
@@ -245,7 +251,7 @@ __device__ __forceinline__ void short_tile(const CsrView<V, T>& A, const VecSet<
                                            Epi& epi, typename Epi::Acc& acc, int r0, int r1,
                                            int nz0, int nz1, int lane, T* prod) {
     constexpr int NV4 = ITEMS / 4 + 1;  // 4-element chunks per lane (+1: alignment slack)
-    constexpr bool SPLIT = epi_split<Epi>::value && !COH;  // a step kernel (k_tiles)
+    constexpr bool IN_CHAIN = epi_chain<Epi>::value;
     const int base = nz0 & ~3;
     int ra[RPL], rb[RPL];
     typename Epi::Pre pre[RPL];
@@ -286,7 +292,7 @@ __device__ __forceinline__ void short_tile(const CsrView<V, T>& A, const VecSet<
 #pragma unroll
             for (int q = 0; q < 4; q++)
                 xg[j][q] = (e + q >= nz0 && e + q < nz1)
-                               ? gather<COH || SPLIT>(xv + (is_pm1<V>::value ? pm1_col(cc[j][q]) : cc[j][q]))
+                               ? gather<COH || IN_CHAIN>(xv + (is_pm1<V>::value ? pm1_col(cc[j][q]) : cc[j][q]))
                                : T(0);
         }
         // products to shared memory, indexed from the aligned window start.
@@ -364,7 +370,7 @@ __device__ __forceinline__ void long_piece(const CsrView<V, T>& A, const VecSet<
     const int npieces = (re - rb + TILE - 1) / TILE;
     const int a = rb + piece * TILE;
     const int b = min(a + TILE, re);
-    constexpr bool SPLIT = epi_split<Epi>::value && !COH;
+    constexpr bool IN_CHAIN = epi_chain<Epi>::value;
     T s[NVEC];
 #pragma unroll
     for (int p = 0; p < NVEC; p++) s[p] = T(0);
@@ -373,12 +379,12 @@ __device__ __forceinline__ void long_piece(const CsrView<V, T>& A, const VecSet<
         if constexpr (is_pm1<V>::value) {
 #pragma unroll
             for (int p = 0; p < NVEC; p++)
-                s[p] = add_rn(s[p], pm1_apply(cc, gather<COH || SPLIT>(xs.v[p] + pm1_col(cc))));
+                s[p] = add_rn(s[p], pm1_apply(cc, gather<COH || IN_CHAIN>(xs.v[p] + pm1_col(cc))));
         } else {
             const T vv = load1v<V, T>(A.val + e);
 #pragma unroll
             for (int p = 0; p < NVEC; p++)
-                s[p] = add_rn(s[p], mul_rn(vv, gather<COH || SPLIT>(xs.v[p] + cc)));
+                s[p] = add_rn(s[p], mul_rn(vv, gather<COH || IN_CHAIN>(xs.v[p] + cc)));
         }
     }
 #pragma unroll
@@ -430,7 +436,7 @@ __global__ void __launch_bounds__(WARPS * 32, sizeof(T) == 8 ? CPDLP_F64_MIN_BLO
     const int task = blockIdx.x * WARPS + w;
     // a step of a chain waits here, before any load: holding a tile's entries
     // over the wait took the FP32 kernels from 56-64 to 92-103 registers
-    if constexpr (epi_split<Epi>::value) {
+    if constexpr (epi_chain<Epi>::value) {
         grid_wait();
         grid_release();
     }
@@ -491,7 +497,8 @@ void launch_tiles_w(const TilePlan& plan, const CsrView<V, T>& view, const VecSe
     const int64_t tasks = (int64_t)plan.ntasks + plan.nltasks;
     if (tasks == 0) return;
     const unsigned grid = (unsigned)((tasks + WARPS - 1) / WARPS);
-    const bool chain = chain_this((int64_t)grid * WARPS * 32, is_pm1<V>::value ? 0 : (int)sizeof(T));
+    const bool chain = epi_chain<Epi>::value &&
+                       chain_this((int64_t)grid * WARPS * 32, is_pm1<V>::value ? 0 : (int)sizeof(T));
     auto start = [&](auto kern) {
         if (chain) launch_chained(kern, grid, WARPS * 32, s, view, xs, epi);
         else kern<<<grid, WARPS * 32, 0, s>>>(view, xs, epi);
@@ -829,6 +836,48 @@ __device__ __forceinline__ void block_reduce_store(const double (&v)[Q], double*
         for (int ww = 0; ww < W; ww++) s += red[ww][threadIdx.x];
         out[(size_t)blockIdx.x * Q + threadIdx.x] = s;
     }
+}
+
+// The last block of a grid to get here (a ticket in global memory, no waiting)
+// sums `rows` rows of Q partials that the grid's blocks wrote, in a fixed order;
+// true, and the sums in out, in its thread 0 only.  W warps per block; the
+// ticket is zero between launches.
+template <int Q, int W = TILE_WARPS>
+__device__ __forceinline__ bool last_block_sum(const double* part, int64_t rows, unsigned* ticket,
+                                               double (&out)[Q]) {
+    __shared__ double red[W][Q];
+    __shared__ bool last;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!last) return false;
+    __threadfence();
+    double v[Q];
+#pragma unroll
+    for (int q = 0; q < Q; q++) v[q] = 0.0;
+#pragma unroll 4
+    for (int64_t r = threadIdx.x; r < rows; r += W * 32)
+#pragma unroll
+        for (int q = 0; q < Q; q++) v[q] += __ldcg(part + r * Q + q);
+#pragma unroll
+    for (int q = 0; q < Q; q++) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v[q] += __shfl_xor_sync(FULL_MASK, v[q], o);
+        if (lane == 0) red[w][q] = v[q];
+    }
+    __syncthreads();
+    if (threadIdx.x != 0) return false;
+    *ticket = 0;
+#pragma unroll
+    for (int q = 0; q < Q; q++) {
+        out[q] = red[0][q];
+        for (int ww = 1; ww < W; ww++) out[q] += red[ww][q];
+    }
+    return true;
 }
 
 // Sums `nrows` rows of q partials into out[q] in a fixed order (one block);
