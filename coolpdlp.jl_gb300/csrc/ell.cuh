@@ -47,7 +47,7 @@ __global__ void __launch_bounds__(WARPS * 32)
     for (int p = 0; p < NVEC; p++) {
         const V* vp = nullptr;
         if constexpr (!is_pm1<V>::value) vp = A.val + k;
-        const T sum = row_sum<true>(A.idx + k, vp, A.rows, w, len, pick(xs.v, p), [&] {
+        const T sum = row_sum<true, sizeof(T) == 8 && !is_pm1<V>::value>(A.idx + k, vp, A.rows, w, len, pick(xs.v, p), [&] {
             if (p > 0) return;
             grid_wait();
             grid_release();

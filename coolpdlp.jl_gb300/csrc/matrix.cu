@@ -16,6 +16,7 @@ struct MulEpi {  // c[i] = alpha*s + beta*c[i]; beta == 0 does not read c (mat_c
     T* out;
     T alpha, beta;
     int use_beta;
+    static constexpr bool EXACT = true;
     struct Acc {};
     struct Pre { T c; };
     __device__ Pre pre_global(int r) const { return Pre{use_beta ? out[r] : T(0)}; }
@@ -29,36 +30,64 @@ struct MulEpi {  // c[i] = alpha*s + beta*c[i]; beta == 0 does not read c (mat_c
     __device__ void finish(Acc&) {}
 };
 
-// spmv_ell! (mat_ell.jl:72-89): one thread per row, column-major slabs,
-// 1-based column indices with 0 as padding.
+// N slabs of one row from slab k: all column indices and values, then all
+// gathers, are in flight together; padding (index 0) adds -0 or is skipped
+template <int N, class T>
+__device__ __forceinline__ T ell_chunk(const int32_t* __restrict__ col1, const T* __restrict__ val,
+                                       int64_t m, const T* __restrict__ b, T s, bool& more) {
+    int j[N];
+    T v[N], g[N];
+#pragma unroll
+    for (int u = 0; u < N; u++) j[u] = ld_cs(col1 + u * m);
+    more = j[N - 1] != 0;
+    if (!__any_sync(FULL_MASK, j[0] != 0)) return s;
+#pragma unroll
+    for (int u = 0; u < N; u++) v[u] = ld_stream(val + u * m);
+#pragma unroll
+    for (int u = 0; u < N; u++) g[u] = gather<false>(b + (j[u] != 0 ? j[u] - 1 : 0));
+#pragma unroll
+    for (int u = 0; u < N; u++) {
+        if constexpr (sizeof(T) == 8) {  // (a whole warp's padding costs the FP64 pipe nothing)
+            if (j[u] != 0) s = add_rn(s, mul_rn(v[u], g[u]));
+        } else {
+            s = add_rn(s, j[u] != 0 ? mul_rn(v[u], g[u]) : T(-0.0));
+        }
+    }
+    return s;
+}
+// spmv_ell! (mat_ell.jl:72-89): one thread per row, column-major slabs, 1-based
+// column indices with 0 as padding, each row summed in column order.  Up to
+// eight slabs at a time (one after another the chain of index, gather and sum
+// cost 8 us for the 128 x 128 flow LP's rows of 8), and a warp stops at the end
+// of its longest row.
 template <class T>
 __global__ void k_spmv_ell(const int32_t* __restrict__ col1, const T* __restrict__ val, int64_t m,
                            int64_t d, const T* __restrict__ b, T* __restrict__ c, T alpha, T beta,
                            int use_beta) {
-    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= m) return;
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int64_t r = i < m ? i : m - 1;  // (idle lanes walk the last row)
+    const T c0 = use_beta ? c[r] : T(0);
     T s = T(0);
-    for (int64_t k = 0; k < d; k++) {
-        const int32_t j = col1[i + k * m];
-        if (j != 0) s = add_rn(s, mul_rn(val[i + k * m], b[j - 1]));
+    col1 += r;
+    val += r;
+    bool more = true;
+    for (; d > 8 && __any_sync(FULL_MASK, more); d -= 8, col1 += 8 * m, val += 8 * m)
+        s = ell_chunk<8>(col1, val, m, b, s, more);
+    if (__any_sync(FULL_MASK, more)) switch ((int)d) {
+        case 8: s = ell_chunk<8>(col1, val, m, b, s, more); break;
+        case 7: s = ell_chunk<7>(col1, val, m, b, s, more); break;
+        case 6: s = ell_chunk<6>(col1, val, m, b, s, more); break;
+        case 5: s = ell_chunk<5>(col1, val, m, b, s, more); break;
+        case 4: s = ell_chunk<4>(col1, val, m, b, s, more); break;
+        case 3: s = ell_chunk<3>(col1, val, m, b, s, more); break;
+        case 2: s = ell_chunk<2>(col1, val, m, b, s, more); break;
+        case 1: s = ell_chunk<1>(col1, val, m, b, s, more); break;
+        default: break;
     }
+    if (i >= m) return;
     T v = mul_rn(alpha, s);
-    if (use_beta) v = add_rn(v, mul_rn(beta, c[i]));
+    if (use_beta) v = add_rn(v, mul_rn(beta, c0));
     c[i] = v;
-}
-
-// mul! for COO (mat_coo.jl:68-80): c .*= beta, then atomic c[i] += alpha*v*b[j]
-template <class T>
-__global__ void k_scale_or_zero(T* __restrict__ c, int64_t m, T beta, int use_beta) {
-    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < m) c[i] = use_beta ? mul_rn(c[i], beta) : T(0);
-}
-template <class T>
-__global__ void k_spmv_coo(const int32_t* __restrict__ row, const int32_t* __restrict__ col,
-                           const T* __restrict__ val, int64_t nnz, const T* __restrict__ b,
-                           T* __restrict__ c, T alpha) {
-    int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (k < nnz) atomicAdd(c + row[k], mul_rn(mul_rn(alpha, val[k]), b[col[k]]));
 }
 
 // GPUSparseMatrixELL(A) (mat_ell.jl:54-70) from the device CSR
@@ -77,6 +106,11 @@ __global__ void k_build_ell(const int32_t* __restrict__ ptr, const int32_t* __re
     }
 }
 
+template <class T>
+__global__ void k_convert(const double* __restrict__ in, T* __restrict__ out, int64_t len) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < len) out[i] = (T)in[i];
+}
 __global__ void k_to_i64_plus(const int32_t* __restrict__ in, int64_t* __restrict__ out, int64_t len,
                               int64_t add) {
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -109,30 +143,41 @@ template <>
 DBuf<float>& vals_of<float>(Matrix& M) { return M.vf; }
 
 template <class T>
+SellSide<T>& sell_of(Matrix& M);
+template <>
+SellSide<double>& sell_of<double>(Matrix& M) { return M.selld; }
+template <>
+SellSide<float>& sell_of<float>(Matrix& M) { return M.sellf; }
+template <class T>
+DBuf<T>& csr_vals(Matrix& M);
+template <>
+DBuf<double>& csr_vals<double>(Matrix& M) { return M.format == CPDLP_FMT_COO ? M.cd : M.vd; }
+template <>
+DBuf<float>& csr_vals<float>(Matrix& M) { return M.format == CPDLP_FMT_COO ? M.cf : M.vf; }
+
+// the product's engines over a CSR on the device (hp: its row pointer)
+template <class T>
+void build_engines(Matrix& M, const std::vector<int32_t>& hp, const DBuf<int32_t>& ptr,
+                   const DBuf<int32_t>& idx, const DBuf<T>& val, cudaStream_t s) {
+    const int items = choose_items(M.nnz, M.m, 0);
+    build_tile_plan(hp, (int32_t)M.m, items, M.plan, s);
+    M.part.alloc((size_t)(M.plan.npieces > 0 ? M.plan.npieces : 1) * sizeof(double));
+    // the sliced engine by the rule of the solver's steps: little padding and, in
+    // FP32, few entries in long rows
+    SellSide<T>& L = sell_of<T>(M);
+    if (M.nnz > 0) {
+        build_sell<T>(L, hp, ptr.p, idx.p, val.p, M.m, 32 * items, s);
+        L.on = (double)L.entries <= SELL_MAX_PADDING * (double)M.nnz &&
+               (sizeof(T) == 8 || (double)L.long_nnz <= SELL_MAX_LONG_F32 * (double)M.nnz);
+        if (!L.on) L.release();
+    }
+}
+
+template <class T>
 void build_T(Handle& h, Matrix& M, CscPair& S) {
     cudaStream_t s = h.stream;
     const int64_t m = M.m, nnz = M.nnz;
     const size_t zn = (size_t)(nnz > 0 ? nnz : 1);
-    if (M.format == CPDLP_FMT_COO) {
-        M.ptr = std::move(S.idx1);   // rowval (0-based), findnz order
-        M.idx = std::move(S.col1);   // colval (0-based)
-        vals_of<T>(M).alloc(zn);
-        if (nnz > 0) {
-            if (std::is_same<T, double>::value)
-                CK(cudaMemcpyAsync(vals_of<T>(M).p, S.val1.p, sizeof(double) * nnz,
-                                   cudaMemcpyDeviceToDevice, s));
-            else {
-                DBuf<int32_t> iota(zn);
-                std::vector<int32_t> hi((size_t)nnz);
-                for (int64_t k = 0; k < nnz; k++) hi[(size_t)k] = (int32_t)k;
-                CK(cudaMemcpyAsync(iota.p, hi.data(), sizeof(int32_t) * nnz, cudaMemcpyHostToDevice, s));
-                gather_values<T, double>(S.val1.p, iota.p, vals_of<T>(M).p, nnz, s);
-                CK(cudaStreamSynchronize(s));
-            }
-        }
-        CK(cudaStreamSynchronize(s));
-        return;
-    }
     // CSR of A: S2 structure with A's values permuted into it (padded for the
     // aligned 128-bit tile loads)
     DBuf<T> v2(zn + PAD_ELEMS);
@@ -145,8 +190,23 @@ void build_T(Handle& h, Matrix& M, CscPair& S) {
         M.ptr = std::move(S.ptr2);
         M.idx = std::move(S.idx2);
         vals_of<T>(M) = std::move(v2);
-        build_tile_plan(hp, (int32_t)m, choose_items(nnz, m, 0), M.plan, s);
-        M.part.alloc((size_t)(M.plan.npieces > 0 ? M.plan.npieces : 1) * sizeof(double));
+        build_engines<T>(M, hp, M.ptr, M.idx, vals_of<T>(M), s);
+        return;
+    }
+    if (M.format == CPDLP_FMT_COO) {
+        // the triplets in findnz order, and the CSR copy that mul! runs over
+        vals_of<T>(M).alloc(zn);
+        if (nnz > 0) {
+            k_convert<T><<<grid_for(nnz, 256), 256, 0, s>>>(S.val1.p, vals_of<T>(M).p, nnz);
+            CK_LAUNCH();
+        }
+        M.ptr = std::move(S.idx1);   // rowval (0-based)
+        M.idx = std::move(S.col1);   // colval (0-based)
+        M.cptr = std::move(S.ptr2);
+        M.cidx = std::move(S.idx2);
+        csr_vals<T>(M) = std::move(v2);
+        build_engines<T>(M, hp, M.cptr, M.cidx, csr_vals<T>(M), s);
+        CK(cudaStreamSynchronize(s));
         return;
     }
     // ELL: width d = maximum(diff(rowptr)) (mat_ell.jl:57)
@@ -179,24 +239,28 @@ void spmv_T(Handle& h, const Matrix& M, const T* b, T* c, double alpha, double b
     cudaStream_t s = h.stream;
     const T a = (T)alpha, bb = (T)beta;
     const int ub = beta != 0.0;
-    const DBuf<T>& vals = vals_of<T>(const_cast<Matrix&>(M));
-    if (M.format == CPDLP_FMT_CSR) {
-        CsrView<T, T> v{M.ptr.p, M.idx.p, vals.p, M.plan.tasks.p, M.plan.ntasks,
-                        M.plan.ltasks.p, M.plan.nltasks, M.plan.counters.p,
-                        reinterpret_cast<T*>(M.part.p)};
-        MulEpi<T> e{c, a, bb, ub};
-        launch_tiles<1>(M.plan, v, VecSet<T, 1>{{b}}, e, s);
-    } else if (M.format == CPDLP_FMT_ELL) {
+    if (M.format == CPDLP_FMT_ELL) {
+        const DBuf<T>& vals = vals_of<T>(const_cast<Matrix&>(M));
         if (M.m > 0)
             k_spmv_ell<T><<<grid_for(M.m, 256), 256, 0, s>>>(M.idx.p, vals.p, M.m, M.width, b, c, a,
                                                              bb, ub);
         CK_LAUNCH();
-    } else {
-        if (M.m > 0) k_scale_or_zero<T><<<grid_for(M.m, 256), 256, 0, s>>>(c, M.m, bb, ub);
-        if (M.nnz > 0)
-            k_spmv_coo<T><<<grid_for(M.nnz, 256), 256, 0, s>>>(M.ptr.p, M.idx.p, vals.p, M.nnz, b, c, a);
-        CK_LAUNCH();
+        return;
     }
+    // CSR, or COO over its CSR copy: the reference's COO product (mat_coo.jl:68-80)
+    // adds in no fixed order; in column order it needs no atomics and one kernel
+    const bool coo = M.format == CPDLP_FMT_COO;
+    const int32_t *ptr = coo ? M.cptr.p : M.ptr.p, *idx = coo ? M.cidx.p : M.idx.p;
+    const T* val = csr_vals<T>(const_cast<Matrix&>(M)).p;
+    const MulEpi<T> e{c, a, bb, ub};
+    const SellSide<T>& L = sell_of<T>(const_cast<Matrix&>(M));
+    if (L.on) {
+        launch_sell(sell_view(L, ptr, idx, val), b, e, s);
+        return;
+    }
+    CsrView<T, T> v{ptr, idx, val, M.plan.tasks.p, M.plan.ntasks, M.plan.ltasks.p, M.plan.nltasks,
+                    M.plan.counters.p, reinterpret_cast<T*>(M.part.p)};
+    launch_tiles<1>(M.plan, v, VecSet<T, 1>{{b}}, e, s);
 }
 
 template <class T>

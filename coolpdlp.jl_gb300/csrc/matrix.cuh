@@ -2,6 +2,7 @@
 #pragma once
 
 #include "cpdlp_common.cuh"
+#include "sell.cuh"
 #include "sparse_build.cuh"
 #include "tiles.cuh"
 
@@ -10,7 +11,10 @@ namespace cpdlp {
 // Storage per format (device, int32 indices):
 //  CSR: ptr = rowptr (m+1, 0-based), idx = colval (0-based), values; tile plan
 //  ELL: idx = colval (m*width, column-major, 1-based, 0 = padding), values
-//  COO: ptr = rowval (0-based), idx = colval (0-based), values, findnz order
+//  COO: ptr = rowval (0-based), idx = colval (0-based), values, findnz order;
+//       mul! runs over a CSR copy (cptr, cidx, cd / cf)
+// CSR and COO products run on the sliced engine where it holds the matrix well
+// (sell), else on the tile plan.
 struct Matrix {
     Handle* h = nullptr;
     int32_t format = CPDLP_FMT_CSR;
@@ -19,6 +23,11 @@ struct Matrix {
     DBuf<int32_t> ptr, idx;
     DBuf<double> vd;
     DBuf<float> vf;
+    DBuf<int32_t> cptr, cidx;  // COO: the CSR copy
+    DBuf<double> cd;
+    DBuf<float> cf;
+    SellSide<double> selld;
+    SellSide<float> sellf;
     TilePlan plan;
     DBuf<unsigned char> part;  // long-row partials (bytes)
 };

@@ -26,6 +26,10 @@
 namespace cpdlp {
 
 constexpr int SELL_WINDOW = 256;
+// the slices may hold this many times the nonzeros; FP32 without the
+// autotuner: the share of the nonzeros in rows longer than LONG_ROW
+constexpr double SELL_MAX_PADDING = 1.5;
+constexpr double SELL_MAX_LONG_F32 = 0.05;
 constexpr uint8_t SELL_SKIP = 255;  // no row, or a row that the long pieces take
 
 template <class T>
@@ -90,7 +94,8 @@ __device__ __forceinline__ int ld_cs(const int32_t* p) {
 // beyond the row's length add -0 (its padding has value 0 and index 0).
 // COH: the gathered vector may have been written by the kernel before, which ran
 // at the same time (a chained launch).
-template <int N, bool COH, class V, class T, class Mid>
+// FUSED: one rounding an entry (FP64 steps), else the product and the sum round.
+template <int N, bool COH, bool FUSED, class V, class T, class Mid>
 __device__ __forceinline__ T row_chunk(const int32_t* ip, const V* vp, int64_t step, int len,
                                        const T* x, T s, Mid&& mid) {
     int c[N];
@@ -108,7 +113,7 @@ __device__ __forceinline__ T row_chunk(const int32_t* ip, const V* vp, int64_t s
     for (int u = 0; u < N; u++) {
         if constexpr (is_pm1<V>::value) {
             s = add_rn(s, u < len ? pm1_apply(c[u], g[u]) : T(-0.0));
-        } else if constexpr (sizeof(T) == 8) {
+        } else if constexpr (FUSED) {
             s = __fma_rn(v[u], u < len ? g[u] : T(-0.0), s);
         } else {
             const T p = mul_rn(v[u], g[u]);
@@ -117,30 +122,30 @@ __device__ __forceinline__ T row_chunk(const int32_t* ip, const V* vp, int64_t s
     }
     return s;
 }
-template <bool COH, class V, class T, class Mid>
+template <bool COH, bool FUSED, class V, class T, class Mid>
 __device__ __forceinline__ T row_rest(const int32_t* ip, const V* vp, int64_t step, int w, int len,
                                       const T* x, T s, Mid&& mid) {
     switch (w) {
-        case 8: return row_chunk<8, COH>(ip, vp, step, len, x, s, mid);
-        case 7: return row_chunk<7, COH>(ip, vp, step, len, x, s, mid);
-        case 6: return row_chunk<6, COH>(ip, vp, step, len, x, s, mid);
-        case 5: return row_chunk<5, COH>(ip, vp, step, len, x, s, mid);
-        case 4: return row_chunk<4, COH>(ip, vp, step, len, x, s, mid);
-        case 3: return row_chunk<3, COH>(ip, vp, step, len, x, s, mid);
-        case 2: return row_chunk<2, COH>(ip, vp, step, len, x, s, mid);
-        case 1: return row_chunk<1, COH>(ip, vp, step, len, x, s, mid);
+        case 8: return row_chunk<8, COH, FUSED>(ip, vp, step, len, x, s, mid);
+        case 7: return row_chunk<7, COH, FUSED>(ip, vp, step, len, x, s, mid);
+        case 6: return row_chunk<6, COH, FUSED>(ip, vp, step, len, x, s, mid);
+        case 5: return row_chunk<5, COH, FUSED>(ip, vp, step, len, x, s, mid);
+        case 4: return row_chunk<4, COH, FUSED>(ip, vp, step, len, x, s, mid);
+        case 3: return row_chunk<3, COH, FUSED>(ip, vp, step, len, x, s, mid);
+        case 2: return row_chunk<2, COH, FUSED>(ip, vp, step, len, x, s, mid);
+        case 1: return row_chunk<1, COH, FUSED>(ip, vp, step, len, x, s, mid);
         default: mid(); return s;
     }
 }
 // A whole row of w stored entries (uniform over the warp), len of them its own;
 // mid() runs once, between the first entries' loads and their gathers.
-template <bool COH, class V, class T, class Mid>
+template <bool COH, bool FUSED, class V, class T, class Mid>
 __device__ __forceinline__ T row_sum(const int32_t* ip, const V* vp, int64_t step, int w, int len,
                                      const T* x, Mid&& mid) {
     auto none = [] {};
     T s = T(0);
-    if (w <= 8) return row_rest<COH>(ip, vp, step, w, len, x, s, mid);
-    s = row_chunk<8, COH>(ip, vp, step, len, x, s, mid);
+    if (w <= 8) return row_rest<COH, FUSED>(ip, vp, step, w, len, x, s, mid);
+    s = row_chunk<8, COH, FUSED>(ip, vp, step, len, x, s, mid);
 #pragma unroll 1
     for (;;) {
         w -= 8;
@@ -148,14 +153,67 @@ __device__ __forceinline__ T row_sum(const int32_t* ip, const V* vp, int64_t ste
         ip += 8 * step;
         if constexpr (!is_pm1<V>::value) vp += 8 * step;
         if (w <= 8) break;
-        s = row_chunk<8, COH>(ip, vp, step, len, x, s, none);
+        s = row_chunk<8, COH, FUSED>(ip, vp, step, len, x, s, none);
     }
-    return row_rest<COH>(ip, vp, step, w, len, x, s, none);
+    return row_rest<COH, FUSED>(ip, vp, step, w, len, x, s, none);
 }
+// The same with the loads of the next eight entries over the gathers and the sum
+// of the ones before: for a product by itself, whose kernel has registers left
+// (FP64 power-law 240,000 nonzeros 33 -> 28 us a call).  The step kernels need
+// theirs for occupancy: 64-76 registers instead of 40-48 took the FP64 6M-nonzero
+// steps from 0.089 to 0.107 ms.
+template <bool COH, bool FUSED, class V, class T>
+__device__ __forceinline__ T row_sum_ahead(const int32_t* ip, const V* vp, int64_t step, int w,
+                                           int len, const T* x) {
+    auto none = [] {};
+    T s = T(0);
+    if (w <= 8) return row_rest<COH, FUSED>(ip, vp, step, w, len, x, s, none);
+    int c[8];
+    V v[8];
+    auto load = [&] {
+#pragma unroll
+        for (int u = 0; u < 8; u++) c[u] = ld_cs(ip + u * step);
+#pragma unroll
+        for (int u = 0; u < 8; u++) v[u] = ld_stream(vp + u * step);
+    };
+    load();
+#pragma unroll 1
+    for (;;) {
+        T g[8], a[8];
+#pragma unroll
+        for (int u = 0; u < 8; u++) g[u] = gather<COH>(x + c[u]);
+#pragma unroll
+        for (int u = 0; u < 8; u++) a[u] = (T)v[u];
+        const int n = len;
+        w -= 8;
+        len -= 8;
+        ip += 8 * step;
+        vp += 8 * step;
+        const bool full = w >= 8;
+        if (full) load();
+#pragma unroll
+        for (int u = 0; u < 8; u++) {
+            if constexpr (FUSED) s = __fma_rn(a[u], u < n ? g[u] : T(-0.0), s);
+            else {
+                const T p = mul_rn(a[u], g[u]);
+                s = add_rn(s, u < n ? p : T(-0.0));
+            }
+        }
+        if (!full) break;
+    }
+    return row_rest<COH, FUSED>(ip, vp, step, w, len, x, s, none);
+}
+
+// epilogues whose FP64 sums round every product and every addition (mul!, whose
+// sums of up to LONG_ROW entries are the reference's)
+template <class E, class = void>
+struct epi_exact : std::false_type {};
+template <class E>
+struct epi_exact<E, std::enable_if_t<E::EXACT>> : std::true_type {};
 
 // one piece of a row longer than LONG_ROW (long_piece in tiles.cuh, with the
 // piece size at run time and LU entries' loads in flight)
-template <bool COH, int LU = 4, class V, class T, class Epi>
+template <bool COH, bool FUSED, int LU = 4, class V, class T, class Epi>
 __device__ __forceinline__ void sell_piece(const SellView<V, T>& S, const T* x, Epi& epi,
                                            typename Epi::Acc& acc, int4 t, int lane) {
     const int row = t.x, piece = -t.y - 1, lid = t.z, slot = t.w;
@@ -179,7 +237,7 @@ __device__ __forceinline__ void sell_piece(const SellView<V, T>& S, const T* x, 
 #pragma unroll
         for (int u = 0; u < LU; u++)
             if (e + 32 * u < b) {
-                if constexpr (sizeof(T) == 8) s = __fma_rn(v[u], g[u], s);
+                if constexpr (FUSED) s = __fma_rn(v[u], g[u], s);
                 else s = add_rn(s, mul_rn(v[u], g[u]));
             }
     }
@@ -195,10 +253,20 @@ __device__ __forceinline__ void sell_piece(const SellView<V, T>& S, const T* x, 
         done = atomicAdd(&S.counters[lid], 1);
     }
     done = __shfl_sync(FULL_MASK, done, 0);
-    if (done == npieces - 1 && lane == 0) {
-        __threadfence();
-        T tot = T(0);
-        for (int q = 0; q < npieces; q++) tot = add_rn(tot, __ldcg(S.partials + slot + q));
+    if (done != npieces - 1) return;
+    __threadfence();
+    // the partials, 32 at a time: in FP32 added in piece order, like the tile
+    // engine, in FP64 by a tree (156 dependent FP64 additions took 5 us)
+    T tot = T(0);
+    for (int q0 = 0; q0 < npieces; q0 += 32) {
+        const T v = q0 + lane < npieces ? __ldcg(S.partials + slot + q0 + lane) : T(0);
+        if constexpr (sizeof(T) == 8) tot = add_rn(tot, v);
+        else
+            for (int q = 0; q < min(32, npieces - q0); q++)
+                tot = add_rn(tot, __shfl_sync(FULL_MASK, v, q));
+    }
+    if constexpr (sizeof(T) == 8) tot = warp_sum_tree(tot);
+    if (lane == 0) {
         epi.row_long(0, row, tot, lid, acc);
         S.counters[lid] = 0;
     }
@@ -211,12 +279,13 @@ template <int WARPS, bool CHAIN, class V, class T, class Epi>
 __global__ void __launch_bounds__(WARPS * 32)
     k_sell(SellView<V, T> S, const T* x, Epi epi) {
     constexpr bool SPLIT = CHAIN && epi_split<Epi>::value;
+    constexpr bool FUSED = sizeof(T) == 8 && !epi_exact<Epi>::value;
     const int lane = threadIdx.x & 31;
     const int task = blockIdx.x * WARPS + (threadIdx.x >> 5);
     typename Epi::Acc acc;
     epi.init(acc);
     if (task < S.nltasks) {
-        sell_piece<CHAIN>(S, x, epi, acc, S.ltasks[task], lane);
+        sell_piece<CHAIN, FUSED>(S, x, epi, acc, S.ltasks[task], lane);
     } else if (task - S.nltasks < S.nslices) {
         const int s = task - S.nltasks, k = s * 32 + lane;
         const int o = ld_keep(S.off + s), w = ld_keep(S.off + s + 1) - o;
@@ -228,16 +297,23 @@ __global__ void __launch_bounds__(WARPS * 32)
             if constexpr (SPLIT) pre = epi.pre_static(r);
             else if constexpr (!CHAIN) pre = epi.pre_global(r);
         }
-        const T sum = row_sum<CHAIN>(S.idx + (int64_t)o * 32 + lane, S.val + (int64_t)o * 32 + lane,
-                                     (int64_t)32, w, in ? len : 0, x, [&] {
-                                         if constexpr (CHAIN) {
-                                             grid_wait();
-                                             grid_release();
-                                             if constexpr (SPLIT) {
-                                                 if (in) epi.pre_dynamic(r, pre);
-                                             } else if (in) pre = epi.pre_global(r);
-                                         }
-                                     });
+        const int32_t* ip = S.idx + (int64_t)o * 32 + lane;
+        const V* vp = S.val + (int64_t)o * 32 + lane;
+        T sum;
+        if constexpr (epi_exact<Epi>::value) {  // mul!
+            static_assert(!CHAIN, "a product by itself is not chained");
+            sum = row_sum_ahead<CHAIN, FUSED>(ip, vp, (int64_t)32, w, in ? len : 0, x);
+        } else {
+            sum = row_sum<CHAIN, FUSED>(ip, vp, (int64_t)32, w, in ? len : 0, x, [&] {
+                if constexpr (CHAIN) {
+                    grid_wait();
+                    grid_release();
+                    if constexpr (SPLIT) {
+                        if (in) epi.pre_dynamic(r, pre);
+                    } else if (in) pre = epi.pre_global(r);
+                }
+            });
+        }
         if (in) epi.row(0, r, sum, pre, acc);
     }
     epi.finish(acc);
@@ -258,19 +334,23 @@ void launch_sell(const SellView<V, T>& S, const T* x, const Epi& epi, cudaStream
     const int64_t tasks = (int64_t)S.nslices + S.nltasks;
     if (tasks == 0 || tiles_dry_run()) return;
     constexpr bool REDUCES = !std::is_empty<typename Epi::Acc>::value;
-    const bool chain = chain_this(tasks * 32, (int)sizeof(T));
-    if constexpr (!REDUCES) {
-        if (tasks < 152 * 16) {
-            const unsigned grid = (unsigned)((tasks + 1) / 2);
-            if (chain) launch_chained(k_sell<2, true, V, T, Epi>, grid, 64u, s, S, x, epi);
-            else k_sell<2, false, V, T, Epi><<<grid, 64, 0, s>>>(S, x, epi);
-            CK_LAUNCH();
-            return;
+    auto start = [&](auto warps) {
+        constexpr int W = decltype(warps)::value;
+        const unsigned grid = (unsigned)((tasks + W - 1) / W);
+        if constexpr (!epi_exact<Epi>::value) {
+            if (chain_this(tasks * 32, (int)sizeof(T))) {
+                launch_chained(k_sell<W, true, V, T, Epi>, grid, W * 32u, s, S, x, epi);
+                return;
+            }
         }
+        k_sell<W, false, V, T, Epi><<<grid, W * 32, 0, s>>>(S, x, epi);
+    };
+    if constexpr (!REDUCES) {
+        if (tasks < 152 * 16) start(std::integral_constant<int, 2>{});
+        else start(std::integral_constant<int, TILE_WARPS>{});
+    } else {
+        start(std::integral_constant<int, TILE_WARPS>{});
     }
-    const unsigned grid = (unsigned)((tasks + TILE_WARPS - 1) / TILE_WARPS);
-    if (chain) launch_chained(k_sell<TILE_WARPS, true, V, T, Epi>, grid, TILE_WARPS * 32u, s, S, x, epi);
-    else k_sell<TILE_WARPS, false, V, T, Epi><<<grid, TILE_WARPS * 32, 0, s>>>(S, x, epi);
     CK_LAUNCH();
 }
 

@@ -571,11 +571,6 @@ SideChoice tune_side(Handle& h, ProblemT<T>& P, int side, const std::vector<int3
     return best;
 }
 
-// the slices may hold this many times the nonzeros; FP32 without the
-// autotuner: the share of the nonzeros in rows longer than LONG_ROW
-constexpr double SELL_MAX_PADDING = 1.5;
-constexpr double SELL_MAX_LONG_F32 = 0.05;
-
 // The sliced engine against the tile plan the autotuner chose for this side:
 // kept when its step kernel is 3% faster; decided once per matrix shape.
 template <class T, class Launch>
