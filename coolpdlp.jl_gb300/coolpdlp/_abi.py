@@ -165,7 +165,7 @@ EXPORTED_SYMBOLS = (
     "cpdlp_abi_version", "cpdlp_params_default", "cpdlp_create", "cpdlp_destroy",
     "cpdlp_last_error", "cpdlp_synchronize", "cpdlp_stream",
     "cpdlp_matrix_from_csc", "cpdlp_matrix_destroy", "cpdlp_matrix_shape",
-    "cpdlp_matrix_export", "cpdlp_spmv",
+    "cpdlp_matrix_export", "cpdlp_spmv", "cpdlp_spmv_after",
     "cpdlp_problem_create", "cpdlp_problem_destroy", "cpdlp_problem_scaling",
     "cpdlp_state_create", "cpdlp_state_destroy", "cpdlp_state_solve", "cpdlp_state_step",
     "cpdlp_state_kkt", "cpdlp_state_vectors", "cpdlp_state_solution", "cpdlp_state_stats",
@@ -199,6 +199,7 @@ def _declare(lib):
         "cpdlp_matrix_shape": (c_int32, [H, P64, P64, P64, P64]),
         "cpdlp_matrix_export": (c_int32, [H, H, P64, P64, PD]),
         "cpdlp_spmv": (c_int32, [H, H, c_void_p, c_void_p, c_double, c_double]),
+        "cpdlp_spmv_after": (c_int32, [H, H, c_void_p, c_void_p, c_double, c_double, c_void_p]),
         "cpdlp_problem_create": (c_int32, [H, POINTER(LPC), POINTER(ParamsC), POINTER(H)]),
         "cpdlp_problem_destroy": (c_int32, [H]),
         "cpdlp_problem_scaling": (c_int32, [H, H, PD, PD]),

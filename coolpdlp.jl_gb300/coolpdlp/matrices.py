@@ -57,20 +57,34 @@ class _GPUSparseMatrix:
 
     def mul(self, c, b, alpha: float = 1.0, beta: float = 0.0):
         """mul!(c, A, b, alpha, beta) with torch CUDA tensors; beta == 0 does not read c."""
-        import torch
-        tdt = torch.float64 if self.dtype == np.float64 else torch.float32
+        tdt, current_stream = self._torch or self._load_torch()
         if not (b.is_cuda and c.is_cuda) or b.dtype != tdt or c.dtype != tdt:
             raise A.ArgumentError(A.ERR_ARGUMENT, "b and c must be CUDA tensors of the matrix eltype")
         if b.numel() != self.n or c.numel() != self.m:
             raise A.DimensionMismatch(A.ERR_DIMENSION, "mul!: vector sizes do not match the matrix")
         if not (b.is_contiguous() and c.is_contiguous()):
             raise A.ArgumentError(A.ERR_ARGUMENT, "vectors must be contiguous")
-        # order the library's stream after torch's current stream
-        torch.cuda.current_stream(b.device).synchronize()
-        self.handle.check(self.handle.lib.cpdlp_spmv(self.handle.h, self.ptr, c_void_p(b.data_ptr()),
-                                                     c_void_p(c.data_ptr()), float(alpha),
-                                                     float(beta)), "mul!")
+        # the library's stream runs it after torch's current stream (a call costs
+        # 10 us of Python with the eltype looked up and the stream waited for here)
+        rc = self._spmv(self.handle.h, self.ptr, b.data_ptr(), c.data_ptr(), float(alpha),
+                        float(beta), current_stream(b.device.index))
+        if rc != A.OK:
+            self.handle.check(rc, "mul!")
         return c
+
+    _torch = None
+
+    def _load_torch(self):
+        """The torch eltype, and the raw current stream of a device."""
+        import torch
+        tdt = torch.float64 if self.dtype == np.float64 else torch.float32
+        raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+        if raw is None:
+            def raw(device):
+                return torch.cuda.current_stream(device).cuda_stream
+        self._spmv = self.handle.lib.cpdlp_spmv_after
+        self._torch = (tdt, raw)
+        return self._torch
 
     def close(self):
         if getattr(self, "ptr", None):

@@ -182,6 +182,22 @@ int cpdlp_spmv(cpdlp_handle* h, const cpdlp_matrix* A, const void* b, void* c, d
     });
 }
 
+int cpdlp_spmv_after(cpdlp_handle* h, const cpdlp_matrix* A, const void* b, void* c, double alpha,
+                     double beta, void* stream) {
+    NEED(h);
+    if (!A) return CPDLP_ERR_ARGUMENT;
+    return guarded(h, [&] {
+        // an idle stream costs a query; waiting for it unasked cost 3 us
+        const cudaError_t e = cudaStreamQuery(static_cast<cudaStream_t>(stream));
+        if (e == cudaErrorNotReady) {
+            cudaGetLastError();  // (not an error: nothing may find it later)
+            CK(cudaStreamSynchronize(static_cast<cudaStream_t>(stream)));
+        } else CK(e);
+        matrix_spmv(*H(h), *reinterpret_cast<const Matrix*>(A), b, c, alpha, beta);
+        CK(cudaStreamSynchronize(h->stream));
+    });
+}
+
 int cpdlp_spmv_csr_noalloc(cpdlp_handle* h, int64_t m, int64_t n, int64_t nnz,
                            const int32_t* rowptr, const int32_t* colval, const void* nzval,
                            int32_t value_type, const void* b, void* c, double alpha,

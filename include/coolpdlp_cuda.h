@@ -281,6 +281,11 @@ int cpdlp_matrix_export(cpdlp_handle* h, const cpdlp_matrix* A, int64_t* ptr,
 int cpdlp_spmv(cpdlp_handle* h, const cpdlp_matrix* A, const void* b, void* c,
                double alpha, double beta);
 
+/* The same after everything queued on `stream` (a cudaStream_t; null: the legacy
+ * default stream), the stream that wrote b and c. */
+int cpdlp_spmv_after(cpdlp_handle* h, const cpdlp_matrix* A, const void* b, void* c,
+                     double alpha, double beta, void* stream);
+
 /* sort_rows_columns(milp) (src/components/permutation.jl:1-46): the LP with
  * its variables ordered by increasing column length and its constraints by
  * increasing row length (stable: ties keep their index order, as Julia's
