@@ -67,7 +67,7 @@ __global__ void k_sell_fill(const int32_t* __restrict__ ptr, const int32_t* __re
     for (int q = 0; q < w; q++) {
         const int64_t e = ((int64_t)o + q) * 32 + k % 32;
         oidx[e] = q < n ? idx[a + q] : 0;
-        oval[e] = q < n ? val[a + q] : T(0);
+        if (oval) oval[e] = q < n ? val[a + q] : T(0);
     }
 }
 
@@ -139,7 +139,7 @@ void build_sell(SellSide<T>& S, const std::vector<int32_t>& hp, const int32_t* p
     }
     S.entries = 32 * (int64_t)sorted_units;
     S.idx.alloc((size_t)std::max<int64_t>(S.entries, 1));
-    S.val.alloc((size_t)std::max<int64_t>(S.entries, 1));
+    if (val) S.val.alloc((size_t)std::max<int64_t>(S.entries, 1));
     k_sell_fill<T><<<grid_for(padded, 256), 256, 0, s>>>(ptr, idx, val, S.off.p, S.len.p, S.perm.p, padded,
                                                          S.idx.p, S.val.p);
     CK_LAUNCH();

@@ -68,7 +68,8 @@ struct SellView {
 };
 
 // The slices of a CSR (device; hp: its row pointer on the host); tile: the
-// piece size of long rows.  Leaves S.on false; S.entries tells the padding.
+// piece size of long rows; val null: narrow storage.  Leaves S.on false; S.entries
+// tells the padding.
 template <class T>
 void build_sell(SellSide<T>& S, const std::vector<int32_t>& hp, const int32_t* ptr,
                 const int32_t* idx, const T* val, int64_t rows, int tile, cudaStream_t s);
@@ -211,6 +212,13 @@ struct epi_exact : std::false_type {};
 template <class E>
 struct epi_exact<E, std::enable_if_t<E::EXACT>> : std::true_type {};
 
+// narrow +-1 storage: the signs in the indices, no values
+template <class T>
+SellView<Pm1, T> sell_view_pm1(const SellSide<T>& S, const int32_t* ptr, const int32_t* idx) {
+    return SellView<Pm1, T>{S.off.p, S.len.p, S.perm.p, S.idx.p, nullptr, S.ltasks.p, S.counters.p,
+                            S.partials.p, S.nslices, S.nltasks, S.tile, ptr, idx, nullptr};
+}
+
 // one piece of a row longer than LONG_ROW (long_piece in tiles.cuh, with the
 // piece size at run time and LU entries' loads in flight)
 template <bool COH, bool FUSED, int LU = 4, class V, class T, class Epi>
@@ -230,14 +238,17 @@ __device__ __forceinline__ void sell_piece(const SellView<V, T>& S, const T* x, 
         T v[LU], g[LU];
 #pragma unroll
         for (int u = 0; u < LU; u++) c[u] = e + 32 * u < b ? ld_cs(S.cidx + e + 32 * u) : 0;
+        if constexpr (!is_pm1<V>::value) {
 #pragma unroll
-        for (int u = 0; u < LU; u++) v[u] = e + 32 * u < b ? (T)ld_stream(S.cval + e + 32 * u) : T(0);
+            for (int u = 0; u < LU; u++) v[u] = e + 32 * u < b ? (T)ld_stream(S.cval + e + 32 * u) : T(0);
+        }
 #pragma unroll
-        for (int u = 0; u < LU; u++) g[u] = gather<COH>(x + c[u]);
+        for (int u = 0; u < LU; u++) g[u] = gather<COH>(x + (is_pm1<V>::value ? pm1_col(c[u]) : c[u]));
 #pragma unroll
         for (int u = 0; u < LU; u++)
             if (e + 32 * u < b) {
-                if constexpr (FUSED) s = __fma_rn(v[u], g[u], s);
+                if constexpr (is_pm1<V>::value) s = add_rn(s, pm1_apply(c[u], g[u]));
+                else if constexpr (FUSED) s = __fma_rn(v[u], g[u], s);
                 else s = add_rn(s, mul_rn(v[u], g[u]));
             }
     }
@@ -298,7 +309,8 @@ __global__ void __launch_bounds__(WARPS * 32)
             else if constexpr (!CHAIN) pre = epi.pre_global(r);
         }
         const int32_t* ip = S.idx + (int64_t)o * 32 + lane;
-        const V* vp = S.val + (int64_t)o * 32 + lane;
+        const V* vp = nullptr;
+        if constexpr (!is_pm1<V>::value) vp = S.val + (int64_t)o * 32 + lane;
         T sum;
         if constexpr (epi_exact<Epi>::value) {  // mul!
             static_assert(!CHAIN, "a product by itself is not chained");
@@ -338,7 +350,7 @@ void launch_sell(const SellView<V, T>& S, const T* x, const Epi& epi, cudaStream
         constexpr int W = decltype(warps)::value;
         const unsigned grid = (unsigned)((tasks + W - 1) / W);
         if constexpr (!epi_exact<Epi>::value) {
-            if (chain_this(tasks * 32, (int)sizeof(T))) {
+            if (chain_this(tasks * 32, is_pm1<V>::value ? 0 : (int)sizeof(T))) {
                 launch_chained(k_sell<W, true, V, T, Epi>, grid, W * 32u, s, S, x, epi);
                 return;
             }

@@ -418,6 +418,13 @@ void launch_side(const ProblemT<T>& P, int side, const CsrView<V, VT>& view,
                  const VecSet<VT, NVEC>& xs, const Epi& epi, cudaStream_t s) {
     // epilogues without block reductions over the problem's own values: the
     // sliced engine, where the problem has it
+    if constexpr (std::is_same<typename Epi::Acc, NoAcc>::value && is_pm1<V>::value &&
+                  std::is_same<VT, T>::value && NVEC == 1) {
+        if (P.sell[side].on) {
+            launch_sell(sell_view_pm1(P.sell[side], view.ptr, view.idx), xs.v[0], epi, s);
+            return;
+        }
+    }
     if constexpr (std::is_same<typename Epi::Acc, NoAcc>::value && std::is_same<V, T>::value &&
                   std::is_same<VT, T>::value && NVEC == 1) {
         if (P.sell[side].on) {
@@ -1081,18 +1088,19 @@ ProblemBase* make_problem(Handle& h, const cpdlp_lp* lp, const cpdlp_params* prm
     }
     mark("formats, autotuner, density order");
     // below the autotuner's sizes, with the library's own choice of engine (no
-    // ELL, no pinned tile size) and valued storage: a small LP runs its blocks on
+    // ELL, no pinned tile size): a small LP with valued storage runs its blocks on
     // the resident kernels, others step on the sliced engine, where its padding
     // is small and, in FP32, few entries are in long rows (us a step, tiles and
     // slices: FP64 flow 63,000 nonzeros 8.9, 5.5, random 1,000,000 42.7, 20.2,
     // power-law 240,000 with a quarter in long rows 17.1, 14.7; FP32 random
     // 1,000,000 15.7, 14.2, 200,000 9.3, 7.8, power-law 240,000 10.1, 10.9)
-    if (!tune && !pm1 && mt != CPDLP_FMT_ELL && prm->tile_nnz == 0) {
-        res_single_build<T>(*P, hp2, hp1, s);
+    if (!tune && mt != CPDLP_FMT_ELL && prm->tile_nnz == 0) {
+        if (!pm1) res_single_build<T>(*P, hp2, hp1, s);
         for (int side = 0; side < 2 && P->rlp.cs == 0 && nnz > 0; side++) {
             SellSide<T>& S = P->sell[side];
             build_sell<T>(S, side == 0 ? hp2 : hp1, side == 0 ? P->a_ptr.p : P->at_ptr.p,
-                          side == 0 ? P->a_idx.p : P->at_idx.p, side == 0 ? P->a_val.p : P->at_val.p,
+                          side == 0 ? P->a_idx.p : P->at_idx.p,
+                          pm1 ? nullptr : side == 0 ? P->a_val.p : P->at_val.p,
                           side_rows(*P, side), 32 * (side == 0 ? items_A : items_At), s);
             S.on = (double)S.entries <= SELL_MAX_PADDING * (double)nnz &&
                    (sizeof(T) == 8 || (double)S.long_nnz <= SELL_MAX_LONG_F32 * (double)nnz);
@@ -1162,27 +1170,25 @@ ProblemBase* make_problem(Handle& h, const cpdlp_lp* lp, const cpdlp_params* prm
 // ---------------------------------------------------------------------------
 // spectral norm: IterativeSolvers.powm! on Symmetrized(A, A') (linalg.jl:60-96)
 // ---------------------------------------------------------------------------
-uint64_t splitmix64_at(uint64_t seed, uint64_t counter) {
+__device__ __forceinline__ double uniform_at(uint64_t seed, uint64_t counter) {  // U(0, 1]
     uint64_t z = seed + (counter + 1) * 0x9E3779B97F4A7C15ULL;
     z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ULL;
     z = (z ^ (z >> 27)) * 0x94D049BB133111EBULL;
-    return z ^ (z >> 31);
+    z ^= z >> 31;
+    return (double)((z >> 11) + 1) * (1.0 / 9007199254740992.0);
 }
-
-// Gaussian start vector: SplitMix64 + Box-Muller, element i from counters 2i, 2i+1
-void gaussian_vector(uint64_t seed, int64_t len, std::vector<double>& out) {
-    out.resize((size_t)len);
-    // entry i depends only on (seed, i): blocks of 4,096 entries on host threads
-    // (one thread took 80-130 ms for 4M columns, most of a large LP's state setup)
-    const int64_t block = 4096;
-    parallel_for((len + block - 1) / block, [&](int64_t b) {
-        const int64_t end = std::min(len, (b + 1) * block);
-        for (int64_t i = b * block; i < end; i++) {
-            double u1 = (double)((splitmix64_at(seed, 2 * (uint64_t)i) >> 11) + 1) * (1.0 / 9007199254740992.0);
-            double u2 = (double)((splitmix64_at(seed, 2 * (uint64_t)i + 1) >> 11) + 1) * (1.0 / 9007199254740992.0);
-            out[(size_t)i] = std::sqrt(-2.0 * std::log(u1)) * std::cos(6.283185307179586 * u2);
-        }
-    });
+// Gaussian start vector: SplitMix64 + Box-Muller, element i of the caller's order
+// from counters 2i, 2i+1 (order: internal place -> the caller's, or null).  On
+// the host, 16 threads and the upload took 4 ms for 800,000 columns and 8 ms for
+// 4M, most of a large LP's state setup; here 4M elements take 1 ms (FP64 log,
+// sqrt and cos).
+__global__ void k_gaussian(uint64_t seed, const int32_t* __restrict__ order, int64_t n,
+                           double* __restrict__ x) {
+    const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= n) return;
+    const uint64_t i = order ? (uint64_t)order[k] : (uint64_t)k;
+    const double u1 = uniform_at(seed, 2 * i), u2 = uniform_at(seed, 2 * i + 1);
+    x[k] = sqrt(-2.0 * log(u1)) * cos(6.283185307179586 * u2);
 }
 
 double powm_default_tol(int64_t n, bool f32) {
@@ -1210,8 +1216,6 @@ double spectral_norm_T(Handle& h, ProblemT<V>& P, const cpdlp_params* prm, int64
     // FP32 iterates need theta to about 1%, not to eps(Float64) n^3 (which
     // can ask for n iterations on small or, through the Int64 wrap, huge LPs)
     const double rtol = std::is_same<V, float>::value ? POWER_RTOL_F32 : -1.0;
-    std::vector<double> x0;
-    gaussian_vector(prm->power_seed, n, x0);
     DBuf<double> x((size_t)(n > 0 ? n : 1)), Ax((size_t)(n > 0 ? n : 1)), sv((size_t)(m > 0 ? m : 1));
     DBuf<double> pA((size_t)std::max(std::max(P.planA.npieces, P.sell[0].npieces), 1)),
         pAt((size_t)std::max(std::max(P.planAt.npieces, P.sell[1].npieces), 1));
@@ -1226,8 +1230,11 @@ double spectral_norm_T(Handle& h, ProblemT<V>& P, const cpdlp_params* prm, int64
     CK(cudaMemsetAsync(part.p, 0, part.bytes(), s));  // (a side without long rows has one unused counter)
     CK(cudaMemsetAsync(tickets.p, 0, tickets.bytes(), s));
     CK(cudaMemsetAsync(scal.p, 0, scal.bytes(), s));
-    if (n > 0) CK(cudaMemcpyAsync(x.p, x0.data(), sizeof(double) * n, cudaMemcpyHostToDevice, s));
-    order_to_internal(P, 1, x.p, s);  // the start vector of the caller's column order
+    if (n > 0) {
+        k_gaussian<<<grid_for(n, 256), 256, 0, s>>>(prm->power_seed, P.ordered ? P.order_col.p : nullptr,
+                                                    n, x.p);
+        CK_LAUNCH();
+    }
     CK(cudaMemsetAsync(d_it.p, 0, sizeof(int), s));
     const CsrView<V, double> A{P.a_ptr.p, P.a_idx.p, P.a_val.p, P.planA.tasks.p, P.planA.ntasks,
                                P.planA.ltasks.p, P.planA.nltasks, P.planA.counters.p, pA.p};

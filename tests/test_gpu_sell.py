@@ -73,3 +73,17 @@ def test_sliced_fp64_against_oracle(handle, oracle, m, n, long_rows):
     for a, b in zip(_steps(handle, lp, prm, 50), want):
         assert np.max(np.abs(a - b)) <= 1e-9 * max(1.0, np.max(np.abs(b)))
     S.close()
+
+
+@pytest.mark.parametrize("side,K", [(3, 2), (9, 3), (12, 70)])
+def test_sliced_narrow_is_the_tile_engines_bits(handle, side, K):
+    """+-1 storage (signs in the indices): flow LPs, capacity rows of K entries
+    (70: long pieces)."""
+    from coolpdlp import generators as G, native, _abi as A
+    lp = G.multicommodity_flow_lp(side=side, K=K, seed=side)
+    prm = A.default_params_py(A.ALGO_PDLP)
+    prm.float_type = A.VAL_F32
+    pinned = native.copy_params(prm)
+    pinned.tile_nnz = 128
+    for a, b in zip(_steps(handle, lp, prm, 50), _steps(handle, lp, pinned, 50)):
+        assert np.array_equal(a, b)
