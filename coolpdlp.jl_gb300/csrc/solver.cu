@@ -1279,30 +1279,30 @@ double spectral_norm_T(Handle& h, ProblemT<V>& P, const cpdlp_params* prm, int64
         k_mul_vec<double><<<grid_for(n, 256), 256, 0, s>>>(x.p, P.D2.p, xs.p, n);
         CK_LAUNCH();
     }
-    constexpr int DEPTH = 8;  // iterations queued ahead of the host's stopping check
-    void* block = h.host_get(sizeof(PowerSlot) * DEPTH);
+    // Slots and launches in flight; after SINGLES iterations of one launch each,
+    // launches of GROUP: a launch, an event and its wait cost the host more (20
+    // us) than the three kernels of a medium LP's iteration take (9 us).
+    constexpr int RING = 64, LAUNCHES = 16, SINGLES = 8, GROUP = 8;
+    void* block = h.host_get(sizeof(PowerSlot) * RING);
     PowerSlot* ring = static_cast<PowerSlot*>(block);
     PowerSlot* dring = nullptr;
     CK(cudaHostGetDevicePointer((void**)&dring, ring, 0));
     struct Cleanup {
-        Handle& h; void* block; cudaStream_t s; cudaGraphExec_t exec = nullptr;
-        cudaEvent_t ev[DEPTH] = {};
+        Handle& h; void* block; cudaStream_t s;
+        cudaGraphExec_t exec[2] = {nullptr, nullptr};  // one iteration, GROUP of them
+        cudaEvent_t ev[LAUNCHES] = {};
         ~Cleanup() {
             cudaStreamSynchronize(s);  // speculative iterations finish before buffers go
-            if (exec) cudaGraphExecDestroy(exec);
+            for (cudaGraphExec_t e : exec)
+                if (e) cudaGraphExecDestroy(e);
             for (cudaEvent_t e : ev)
                 if (e) cudaEventDestroy(e);
             h.host_put(block);
         }
     } cleanup{h, block, s};
-    for (int k = 0; k < DEPTH; k++)
-        CK(cudaEventCreateWithFlags(&cleanup.ev[k], cudaEventDisableTiming));
+    for (cudaEvent_t& e : cleanup.ev) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     const unsigned gr = red_grid(h, n);
-    {
-        cudaGraph_t g = nullptr;
-        CK(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-        chain_launches() = true;
-        struct Off { ~Off() { chain_launches() = false; } } off;
+    auto iteration = [&] {
         double* const blk = part.p;
         double* const lng = part.p + (size_t)blocks * 2;
         if (P.pm1) {
@@ -1319,33 +1319,48 @@ double spectral_norm_T(Handle& h, ProblemT<V>& P, const cpdlp_params* prm, int64
         }
         launch_chained(k_power_residual, gr, (unsigned)RED_THREADS, s, x.p, (const double*)Ax.p,
                        (const double*)scal.p, n, P.red_rows.p, (const double*)(P.pm1 ? P.D2.p : nullptr),
-                       P.pm1 ? xs.p : nullptr, tickets.p + 1, d_it.p, dring, DEPTH);
+                       P.pm1 ? xs.p : nullptr, tickets.p + 1, d_it.p, dring, RING);
+    };
+    auto capture = [&](int count, cudaGraphExec_t& exec) {
+        cudaGraph_t g = nullptr;
+        CK(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
+        chain_launches() = true;
+        struct Off { ~Off() { chain_launches() = false; } } off;
+        for (int k = 0; k < count; k++) iteration();
         const cudaError_t launch_err = cudaGetLastError();
         const cudaError_t end_err = cudaStreamEndCapture(s, &g);
         CK(launch_err);
         CK(end_err);
-        const cudaError_t inst = cudaGraphInstantiate(&cleanup.exec, g, 0);
+        const cudaError_t inst = cudaGraphInstantiate(&exec, g, 0);
         cudaGraphDestroy(g);
         CK(inst);
-    }
+    };
     // powm!: iterate while !(it > maxiter || residual <= tol); it counts iterations run.
     // Iterations are queued ahead of the host's check, 2 at first and twice as
-    // many each time a result is read, up to DEPTH: an LP that stops after 2
-    // iterations (C1 with FP32 iterates) runs no 6 extra ones.
+    // many each time a result is read: an LP that stops after 2 iterations (C1
+    // with FP32 iterates) runs no 6 extra ones.
     double theta_d = 0.0;
-    int64_t launched = 0, it = 0, ahead = 2;
-    for (;;) {
+    int64_t launched = 0, it = 0, ahead = 2, queued = 0, read = 0;
+    int64_t ends[LAUNCHES];
+    for (bool stop = false; !stop;) {
         while (launched - it < ahead && launched <= maxiter) {
-            CK(cudaGraphLaunch(cleanup.exec, s));
-            CK(cudaEventRecord(cleanup.ev[launched % DEPTH], s));
-            launched++;
+            const bool many = launched >= SINGLES;
+            cudaGraphExec_t& exec = cleanup.exec[many];
+            if (!exec) capture(many ? GROUP : 1, exec);
+            CK(cudaGraphLaunch(exec, s));
+            CK(cudaEventRecord(cleanup.ev[queued % LAUNCHES], s));
+            launched += many ? GROUP : 1;
+            ends[queued++ % LAUNCHES] = launched;
         }
-        CK(cudaEventSynchronize(cleanup.ev[it % DEPTH]));
-        const PowerSlot slot = ring[it % DEPTH];
-        it++;
-        ahead = std::min<int64_t>(2 * ahead, DEPTH);
-        theta_d = slot.theta;
-        if (it > maxiter || slot.residual <= tol || slot.residual <= rtol * slot.theta) break;
+        CK(cudaEventSynchronize(cleanup.ev[read % LAUNCHES]));
+        const int64_t end = ends[read++ % LAUNCHES];
+        while (it < end && !stop) {
+            const PowerSlot slot = ring[it % RING];
+            it++;
+            theta_d = slot.theta;
+            stop = it > maxiter || slot.residual <= tol || slot.residual <= rtol * slot.theta;
+        }
+        ahead = std::min<int64_t>(2 * ahead, launched < SINGLES ? SINGLES : 3 * GROUP);
         if (now_seconds() >= deadline) break;
     }
     if (iters_out) *iters_out = it;
