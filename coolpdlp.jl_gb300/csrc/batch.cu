@@ -3,20 +3,21 @@
 // The LPs of a job are concatenated block-diagonally on the host and
 // preprocessed once by the single-LP device pipeline: Ruiz and Pock-Chambolle
 // scaling work on rows and columns, so the scaling of the concatenation equals
-// the scaling of each LP.  The tile partitions are rebuilt so that no tile
-// crosses an LP boundary.  One CTA solves one LP at a time and takes the next
-// LP from an atomic counter over a largest-first order when it finishes: power
-// method (linalg.jl:86-96), primal weight (step_size.jl:29-40), then blocks of
+// the scaling of each LP.  An LP that fits the shared memory of a CTA or of a
+// cluster (res_plan) is solved there by k_res_pdlp; the others by tile kernels
+// over global memory, with tile partitions that never cross an LP boundary.
+// One CTA or cluster solves one LP at a time and takes the next LP from an
+// atomic counter over a largest-first order when it finishes: power method (linalg.jl:86-96), primal weight (step_size.jl:29-40), then blocks of
 // check_every fused PDHG steps (pdlp.jl:96-136) with the four-iterate KKT
 // check, restart and termination logic (pdlp.jl:138-196, restart.jl:40-57,
 // termination.jl:89-101) run by the CTA itself, thread 0 taking the FP64
-// decisions.  Every loop is bounded by the LP's pass limit and time limit; no
-// CTA waits on another.
+// decisions.  Every loop is bounded by the LP's pass limit and time limit; CTAs
+// wait only on CTAs of their own cluster.
 //
-// An LP's arithmetic depends only on the LP and the tile size (its tiles, the
-// thread that owns each row, the order of every sum), never on the other LPs
-// of the job or on which CTA runs it, so an LP gives the same result alone and
-// in any mix.
+// An LP's route and arithmetic depend only on the LP, the value type and the
+// tile size (its slices or tiles, the thread that owns each row, the order of
+// every sum), never on the other LPs of the job or on which CTA runs it, so an
+// LP gives the same result alone and in any mix.
 //
 // The per-LP semantics are those of solve(milp, algo) (common.jl:186-209)
 // except that no error history is recorded.  With FP32 iterates, LPs whose
@@ -1783,7 +1784,17 @@ int64_t batch_footprint(int64_t count, const cpdlp_lp* lps, const cpdlp_params* 
     // bounds and costs, FP64 scalings, power-method vectors
     const int64_t mat = nnz * (2 * (4 + sv) + 40) + (m + n) * 16 + (1 << 16);
     const int64_t vec = n * (10 * sv + 6 * 8) + m * (8 * sv + 5 * 8);
-    return mat + vec + count * 256 + (4 << 20);
+    // LPs that may stay in shared memory: the slices of A and A' they are loaded
+    // from.  A slice of 32 rows is as wide as its longest row and the rows are in
+    // order of length, so the padding is at most the first slice's entries.
+    int64_t res = 0;
+    for (int64_t k = 0; k < count; k++) {
+        const int64_t lm = lps[k].m, ln = lps[k].n, lz = lps[k].nnz;
+        if (lm < 1 || ln < 1 || lz < 1 || lm > RES_MAX_DIM || ln > RES_MAX_DIM) continue;
+        const int64_t wide = 32 * (std::min<int64_t>(ln, LONG_ROW) + std::min<int64_t>(lm, LONG_ROW));
+        res += (2 * lz + wide) * (2 + sv) + (lm + ln + 64) * 8 + 256;
+    }
+    return mat + vec + res + count * 256 + (4 << 20);
 }
 
 void batch_solve(Handle& h, int64_t count, const cpdlp_lp* lps, const cpdlp_params* params,

@@ -7,9 +7,10 @@
 // row's length, so the padding is never read.  Consecutive threads read
 // consecutive addresses of a slab (coalesced).  A row's sum runs in its
 // column order, sequentially, like the reference's spmv_ell! loop, so every
-// row reproduces a sequential CPU sum exactly (in the CSR tile engine only
-// rows of at most LONG_ROW nonzeros do).  Narrow +-1 storage carries the sign
-// in the index (~col for -1) and has no value slab.
+// FP32 row reproduces a sequential CPU sum exactly (in the CSR tile engine only
+// rows of at most LONG_ROW nonzeros do); FP64 sums are fused multiply-adds.
+// Narrow +-1 storage carries the sign in the index (~col for -1) and has no
+// value slab.
 #pragma once
 
 #include "sell.cuh"

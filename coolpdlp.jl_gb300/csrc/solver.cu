@@ -1,15 +1,19 @@
 // solver.cu -- single-LP PDLP / PDHG on one GB300.
 //
 // Per PDHG step two fused kernels run (pdlp.jl:96-124):
-//   primal: s = (A' y)_j (warp tiles over the rows of A')  ->
+//   primal: s = (A' y)_j (over the rows of A')  ->
 //           x+ = proj_box(x - tau*(c - s), lv, uv), xbar = 2x+ - x,
 //           avg_x = a*x+ + b*avg_x_last                      (pdlp.jl:110-113, :126-136)
-//   dual:   s = (A xbar)_i (warp tiles over the rows of A)  ->
+//   dual:   s = (A xbar)_i (over the rows of A)  ->
 //           y+ = y - sigma*s - sigma*proj_box(y/sigma - s, -uc, -lc),
 //           avg_y = a*y+ + b*avg_y_last                      (pdlp.jl:115-117)
 // Iterates ping-pong between two buffers (the reference swaps sol/sol_last,
 // pdlp.jl:101, and copies avg into avg_last, :129; here the average ping-pongs
-// too).  check_every steps are captured once as a CUDA graph per buffer parity.
+// too).  The row sums come from warp tiles (tiles.cuh), slices (sell.cuh) or ELL
+// slabs (ell.cuh), chosen per matrix.  check_every steps are captured once as a
+// CUDA graph per buffer parity.  An LP small enough for the shared memory of one
+// CTA or cluster runs the check_every steps and the check's sums in one launch
+// instead (resident_single.cu).
 // Every check evaluates the KKT errors of sol, avg, sol_last and avg_last in
 // ONE pass over both matrices (four gathered vectors per nonzero), with FP64
 // accumulation, a deterministic block-then-tree reduction and one small
@@ -496,8 +500,8 @@ constexpr int64_t ELL_MAX_PADDING = 3;
 
 // Nonzeros per lane of a large matrix's tiles.  Four blocks of eight 512-nonzero
 // tiles are resident on an SM; between 0.95 and 1.39 such waves the last one is
-// nearly empty, and 256-nonzero tiles were 3% to 8% faster (5 of 6 timing runs
-// at 2.7M to 3.3M nonzeros, none at 2.1M or from 3.6M to 24M).
+// nearly empty, and 256-nonzero tiles were at least 3% faster (5 of 6 timing runs
+// at 2.7M to 3.3M nonzeros, 1 of 6 at 2.1M, none from 3.6M to 24M).
 int wave_items(int64_t nnz, int items, int num_sms) {
     const double waves = (double)nnz / ((double)num_sms * 4 * TILE_WARPS * 512);
     return items == 16 && waves > 0.95 && waves < 1.39 ? 8 : items;
@@ -1178,10 +1182,9 @@ __device__ __forceinline__ double uniform_at(uint64_t seed, uint64_t counter) { 
     return (double)((z >> 11) + 1) * (1.0 / 9007199254740992.0);
 }
 // Gaussian start vector: SplitMix64 + Box-Muller, element i of the caller's order
-// from counters 2i, 2i+1 (order: internal place -> the caller's, or null).  On
-// the host, 16 threads and the upload took 4 ms for 800,000 columns and 8 ms for
-// 4M, most of a large LP's state setup; here 4M elements take 1 ms (FP64 log,
-// sqrt and cos).
+// from counters 2i, 2i+1 (order: internal place -> the caller's, or null).  Bound
+// by the FP64 log, sqrt and cos; 16 host threads and the upload instead made the
+// solve of an LP of 800,000 columns 5 ms longer.
 __global__ void k_gaussian(uint64_t seed, const int32_t* __restrict__ order, int64_t n,
                            double* __restrict__ x) {
     const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1280,8 +1283,9 @@ double spectral_norm_T(Handle& h, ProblemT<V>& P, const cpdlp_params* prm, int64
         CK_LAUNCH();
     }
     // Slots and launches in flight; after SINGLES iterations of one launch each,
-    // launches of GROUP: a launch, an event and its wait cost the host more (20
-    // us) than the three kernels of a medium LP's iteration take (9 us).
+    // launches of GROUP: a launch, an event and its wait cost the host more than
+    // the three kernels of a medium LP's iteration take (256 x 256 flow LP: 25 us
+    // an iteration one by one, 17 us in groups; its solve 15.5 -> 14.4 ms).
     constexpr int RING = 64, LAUNCHES = 16, SINGLES = 8, GROUP = 8;
     void* block = h.host_get(sizeof(PowerSlot) * RING);
     PowerSlot* ring = static_cast<PowerSlot*>(block);

@@ -133,7 +133,7 @@ typedef struct cpdlp_params {
      * errors), and PDLP continues in FP64 if a round makes no progress.
      * Batched solves and jobs continue in FP64 instead (cpdlp_batch_solve). */
     double refine_reltol;
-    /* EXT: CSR tile size in nonzeros for the SpMV work partition (0 = autotune). */
+    /* EXT: CSR tile size in nonzeros for the SpMV work partition (0 = by problem size). */
     int32_t tile_nnz;
     /* EXT: storage flags (CPDLP_TILE_*); 0 = defaults. */
     int32_t tile_flags;
@@ -150,14 +150,15 @@ typedef struct cpdlp_params {
     double infeasibility_tol;
     /* matrix_type M of Algorithm{A}(T, Ti, M) (src/components/conversion.jl:
      * 37-55, src/problems/modify.jl:80-105): the product format of the
-     * single-LP solve's matrices A and A'.  CPDLP_FMT_CSR: the CSR tile
-     * engine (tile shape autotuned for large matrices); CPDLP_FMT_ELL: the
+     * single-LP solve's matrices A and A'.  CPDLP_FMT_CSR: the CSR
+     * engines (tiles, or slices of 32 rows; large matrices: the faster by
+     * timing); CPDLP_FMT_ELL: the
      * reference's ELL layout (column-major, width = the longest row), one
      * thread per row, each row summed in column order; CPDLP_FMT_COO: solved
      * on the CSR engine (the reference's COO product accumulates with atomics
      * in a run-dependent order; CSR sums each row in COO's column order);
      * CPDLP_FMT_AUTO (default, EXT): for matrices of at least 2^21 nonzeros
-     * the autotuner times CSR tile shapes and ELL (when its padding is at
+     * the autotuner times CSR tiles, CSR slices and ELL (when its padding is at
      * most 3x the nonzeros) and keeps the fastest per matrix, otherwise CSR.
      * Batched solves and jobs use the CSR engine. */
     int32_t matrix_type;
