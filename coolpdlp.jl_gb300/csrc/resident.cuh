@@ -251,14 +251,12 @@ constexpr int RES_SUMS = 5;  // most values of one sum
 // CTA's next sums do not meet a slow one's reads.
 template <int CS, int NW>
 constexpr int res_sh() { return 2 * RES_SUMS * CS * NW + 8; }
-template <int Q, int CS, int NW, class F>
-__device__ __forceinline__ void res_sum(double (&v)[Q], double* sh, int& phase, bool busy,
-                                        F&& finish) {
+// a warp's part of the sums, stored into every CTA's slots
+template <int Q, int CS, int NW>
+__device__ __forceinline__ void res_partial(const double (&v)[Q], double* slot, bool busy) {
     static_assert(Q <= RES_SUMS && Q <= NW, "a warp per value");
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     constexpr int P = CS * NW;  // warps of the group
-    double* slot = sh + 8 + phase * (RES_SUMS * P);
-    phase ^= 1;
     double d = 0.0;
     int which = lane / (Q <= 4 ? 8 : 4);
     if (!busy) {
@@ -301,14 +299,35 @@ __device__ __forceinline__ void res_sum(double (&v)[Q], double* sh, int& phase, 
     if ((lane & (Q <= 4 ? 7 : 3)) == 0 && which < Q)
         res_put<CS>(slot + which * P + rank * NW + w, d, rank);
     __syncwarp();
+}
+// value q of all warps of the group, by one warp (whole in every lane)
+template <int CS, int NW>
+__device__ __forceinline__ double res_total(const double* slot, int q) {
+    constexpr int P = CS * NW;
+    const int lane = threadIdx.x & 31;
+    double s = 0.0;
+#pragma unroll
+    for (int k = 0; k < (P + 31) / 32; k++)
+        if (k * 32 + lane < P) s = k ? s + slot[q * P + k * 32 + lane] : slot[q * P + lane];
+#pragma unroll
+    for (int o = (P < 32 ? P : 32) / 2; o > 0; o >>= 1) s += __shfl_xor_sync(FULL_MASK, s, o);
+    return s;
+}
+template <int CS, int NW>
+__device__ __forceinline__ double* res_slot(double* sh, int& phase) {
+    double* slot = sh + 8 + phase * (RES_SUMS * CS * NW);
+    phase ^= 1;
+    return slot;
+}
+template <int Q, int CS, int NW, class F>
+__device__ __forceinline__ void res_sum(double (&v)[Q], double* sh, int& phase, bool busy,
+                                        F&& finish) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    double* slot = res_slot<CS, NW>(sh, phase);
+    res_partial<Q, CS, NW>(v, slot, busy);
     res_sync<CS>();
     if (w < Q) {
-        double s = 0.0;
-#pragma unroll
-        for (int k = 0; k < (P + 31) / 32; k++)
-            if (k * 32 + lane < P) s = k ? s + slot[w * P + k * 32 + lane] : slot[w * P + lane];
-#pragma unroll
-        for (int o = (P < 32 ? P : 32) / 2; o > 0; o >>= 1) s += __shfl_xor_sync(FULL_MASK, s, o);
+        const double s = res_total<CS, NW>(slot, w);
         if (lane == 0) sh[w] = finish(w, s);
     }
     __syncthreads();
@@ -648,16 +667,24 @@ __device__ __noinline__ void res_kkt_sums(const ResGeo& G, const T* gx, const T*
 // powm! iterations (linalg.jl:86-96) in FP64 over the stored values, from the
 // vector px (loaded whole into every CTA): stops after an iteration whose
 // residual is at most tol or rtol * theta, after iteration maxiter + 1 or after
-// max_here iterations of this call.  The residual of an iteration needs its
-// theta, so its norm is summed with the next iteration's theta (one exchange
-// an iteration); the extra iteration's own theta is dropped.  it0 iterations
-// ran before, the last with theta_prev.
+// max_here iterations of this call.  it0 iterations ran before, the last with
+// theta_prev.
+// A chain of two products, two exchanges and the sums for theta and the scale
+// bounds it.  So A'Ax is sent unscaled and the sums overlap its exchange and the
+// next product with A, whose result takes the scale instead (a single CTA
+// exchanges nothing and scales x first); three warps that
+// (mostly) have no slices of A finish the sums.  The residual of an iteration
+// needs its theta, so its norm is summed with the next iteration's theta: two
+// products beyond the last iteration are dropped.  FP64 1,000 x 2,000 on 8 CTAs:
+// a solve with 1,725 iterations 14.0 -> 12.8 ms; 128 LPs of up to 600 rows
+// 38-42 -> 32-37 ms.
 template <class T, int CS, int NT>
 __device__ __noinline__ void res_power(const ResGeo& G, int64_t it0, int64_t max_here,
                                        int64_t maxiter, double tol, double rtol, double theta_prev,
                                        ResPower& P, double* sh, int& phase, ResWait& W,
                                        unsigned& parity_io) {
     constexpr int NW = NT / 32;
+    static_assert(NW >= 3, "three warps finish the sums");
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, rank = G.rank;
     const int LA = G.LA, LAt = G.LAt, n = G.R.n;
     const T *valA = &sm_at<T>(G.o.valA) + lane, *valAt = &sm_at<T>(G.o.valAt) + lane;
@@ -665,69 +692,113 @@ __device__ __noinline__ void res_power(const ResGeo& G, int64_t it0, int64_t max
     const uint32_t *offA = &sm_at<uint32_t>(G.o.offA), *offAt = &sm_at<uint32_t>(G.o.offAt);
     const uint8_t *lenA = &sm_at<uint8_t>(G.o.lenA) + lane, *lenAt = &sm_at<uint8_t>(G.o.lenAt) + lane;
     const double *px = &sm_at<double>(G.px), *ps = &sm_at<double>(G.ps);
-    double *pxown = &sm_at<double>(G.px) + G.baseAt, *psown = &sm_at<double>(G.ps) + G.baseA;
-    double* pax = &sm_at<double>(G.pax) + lane;
+    double *pxown = &sm_at<double>(G.px) + G.baseAt + lane, *psown = &sm_at<double>(G.ps) + G.baseA + lane;
+    double* pax = &sm_at<double>(G.pax) + lane;  // own x, scaled
     unsigned parity = parity_io;
-    double theta = theta_prev, residual = INFINITY;
+    double theta = theta_prev, residual = INFINITY, inv = 1.0;
     int64_t it = it0;
     bool stop = false;
-    double r2 = 0.0;       // own part of the last iteration's residual^2
-    bool pending = false;  // an iteration's residual is not summed yet
-    for (;;) {
+    double r2 = 0.0;               // own part of the last iteration's residual^2
+    const double* slot = nullptr;  // sums on their way
+    bool pending = false;          // they hold an iteration's residual
+    const int wa = (w + NW - LAt % NW) % NW;  // slices of A start after those of A'
+    const int wq = NW - 1 - w;                // the last three warps finish the sums
+    auto product = [&] {
 #pragma unroll 1
-        for (int l = w; l < LA; l += NW) {
+        for (int l = wa; l < LA; l += NW) {
             const uint32_t o = offA[l];
-            psown[l * 32 + lane] = slice_sum(idxA + (o >> 8) * 32, valA + (o >> 8) * 32,
-                                             (int)(o & 255u), lenA[l * 32], px);
-            res_send<CS>(psown + l * 32, &W.bar[0], rank);
+            psown[l * 32] = slice_sum(idxA + (o >> 8) * 32, valA + (o >> 8) * 32, (int)(o & 255u),
+                                      lenA[l * 32], px);
         }
+    };
+    auto rescale = [&] {
+        r2 = 0.0;
+#pragma unroll 1
+        for (int l = w; l < LAt; l += NW) {
+            const double ax = pxown[l * 32];
+            if ((l * CS + rank) * 32 + lane < n) {
+                const double rr = __fma_rn(-theta, pax[l * 32], ax);
+                r2 = __fma_rn(rr, rr, r2);
+            }
+            pax[l * 32] = mul_rn(ax, inv);
+        }
+    };
+    auto keep = [&] {
+#pragma unroll 1
+        for (int l = w; l < LAt; l += NW) pxown[l * 32] = pax[l * 32];
+    };
+#pragma unroll 1
+    for (int l = w; l < LAt; l += NW) pax[l * 32] = pxown[l * 32];
+    for (;;) {
+        // theta, 1 / |A'Ax| and the residual of the iteration before (negative
+        // when it ends the iteration)
+        if (slot && wq < 3) {
+            __syncwarp();
+            if constexpr (CS > 1) res_wait<CS>();
+            const double s = res_total<CS, NW>(slot, wq);
+            double f = s;
+            if (wq == 1) f = rsqrt(s);
+            if (wq == 2) {
+                const double res = sqrt(s);
+                f = res <= tol || (rtol > 0 && res <= rtol * theta) ? -1.0 - res : res;
+            }
+            if (lane == 0) sh[wq] = f;
+            __syncwarp();
+        }
+        if constexpr (CS > 1) {
+            product();
+            __syncwarp();
+            if (slot && wq >= 3) res_wait<CS>();
+        }
+        __syncthreads();
+        if (pending) {
+            residual = sh[2];
+            it++;
+            stop = it > maxiter || __double_as_longlong(residual) < 0;
+            if (stop || it - it0 >= max_here || (CS > 1 && W.failed)) break;
+        }
+        if (slot) {
+            theta = sh[0];
+            inv = sh[1];
+        }
+        if constexpr (CS > 1) {
+#pragma unroll 1
+            for (int l = wa; l < LA; l += NW) {
+                psown[l * 32] = mul_rn(psown[l * 32], inv);
+                res_send<CS>(psown + l * 32 - lane, &W.bar[0], rank);
+            }
+            if (slot) rescale();
+        } else {
+            if (slot) {
+                rescale();
+                keep();
+                __syncthreads();
+            }
+            product();
+        }
+        pending = slot != nullptr;
         res_receive<CS>(W, 0, G.remA * 8u, parity);
         double v[3] = {0.0, 0.0, r2};
 #pragma unroll 1
         for (int l = w; l < LAt; l += NW) {
-            const int r = (l * CS + rank) * 32 + lane;
             const uint32_t o = offAt[l];
             const double s = slice_sum(idxAt + (o >> 8) * 32, valAt + (o >> 8) * 32,
                                        (int)(o & 255u), lenAt[l * 32], ps);
-            pax[l * 32] = s;
-            if (r < n) {
-                v[0] = __fma_rn(pxown[l * 32 + lane], s, v[0]);
+            pxown[l * 32] = s;
+            res_send<CS>(pxown + l * 32 - lane, &W.bar[1], rank);
+            if ((l * CS + rank) * 32 + lane < n) {
+                v[0] = __fma_rn(pax[l * 32], s, v[0]);
                 v[1] = __fma_rn(s, s, v[1]);
             }
         }
         __syncwarp();
-        // theta, 1 / |A'Ax| and the previous iteration's residual (negative when
-        // it ends the iteration)
-        res_sum<3, CS, NW>(v, sh, phase, w < LAt, [&](int q, double s) {
-            if (q == 0) return s;
-            if (q == 1) return rsqrt(s);
-            const double res = sqrt(s);
-            return res <= tol || (rtol > 0 && res <= rtol * theta) ? -1.0 - res : res;
-        });
-        if (pending) {
-            const bool small = __double_as_longlong(v[2]) < 0;
-            residual = v[2];
-            it++;
-            stop = it > maxiter || small;
-            if (stop || it - it0 >= max_here || (CS > 1 && W.failed)) break;
-        }
-        theta = v[0];
-        const double inv = v[1];
-        r2 = 0.0;
-#pragma unroll 1
-        for (int l = w; l < LAt; l += NW) {
-            const int r = (l * CS + rank) * 32 + lane;
-            const double ax = pax[l * 32];
-            if (r < n) {
-                const double rr = __fma_rn(-theta, pxown[l * 32 + lane], ax);
-                r2 = __fma_rn(rr, rr, r2);
-            }
-            pxown[l * 32 + lane] = mul_rn(ax, inv);
-            res_send<CS>(pxown + l * 32, &W.bar[1], rank);
-        }
-        pending = true;
+        double* put = res_slot<CS, NW>(sh, phase);
+        res_partial<3, CS, NW>(v, put, w < LAt);
+        slot = put;
+        if constexpr (CS > 1) res_arrive<CS>();
         res_receive<CS>(W, 1, G.remAt * 8u, parity);
     }
+    keep();
     if (__double_as_longlong(residual) < 0) residual = -1.0 - residual;
     P.theta = theta;
     P.residual = residual;

@@ -1284,8 +1284,9 @@ double spectral_norm_T(Handle& h, ProblemT<V>& P, const cpdlp_params* prm, int64
     }
     // Slots and launches in flight; after SINGLES iterations of one launch each,
     // launches of GROUP: a launch, an event and its wait cost the host more than
-    // the three kernels of a medium LP's iteration take (256 x 256 flow LP: 25 us
-    // an iteration one by one, 17 us in groups; its solve 15.5 -> 14.4 ms).
+    // the three kernels of a medium LP's iteration take (FP64: solve of a flow LP of
+    // 63,000 nonzeros 15.5 -> 14.4 ms; power method and setup of a random LP of
+    // 1M nonzeros 7.9 -> 3.1 ms).
     constexpr int RING = 64, LAUNCHES = 16, SINGLES = 8, GROUP = 8;
     void* block = h.host_get(sizeof(PowerSlot) * RING);
     PowerSlot* ring = static_cast<PowerSlot*>(block);
