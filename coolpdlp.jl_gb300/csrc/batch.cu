@@ -33,6 +33,7 @@
 #include <cooperative_groups.h>
 
 #include "batch.cuh"
+#include "cta_budget.h"
 #include "epilogues.cuh"
 #include "resident.cuh"
 #include "solver.cuh"
@@ -1255,6 +1256,21 @@ struct Run : RunBase {
         int64_t nbig = 0;
         if (nclusters > 0 && nclusters_p > 0)
             while (nbig < ntile && nz_off[order[nbig] + 1] - nz_off[order[nbig]] >= cmin) nbig++;
+        // the CTAs of each launch that runs beside the others: the tile kernel, its
+        // cluster form, the resident classes.  Work in us of a CTA per step: 24 for
+        // 5,500 nonzeros over global memory; resident a CTA takes about 1 and 0.5 per
+        // 1,000 nonzeros of its own.
+        auto nnz_of = [&](int32_t k) { return (double)(nz_off[k + 1] - nz_off[k]); };
+        std::vector<CtaShare> shares{
+            {1, std::min<int64_t>(ntile - nbig, (int64_t)std::max(per_sm, 1) * rh.num_sms), 0.0},
+            {CLUSTER_CTAS, std::min<int64_t>(nbig, nclusters), 0.0}};
+        for (int64_t k = 0; k < ntile; k++) shares[k < nbig ? 1 : 0].work += nnz_of(order[k]) / 230.0;
+        for (const LaunchClass& cl : classes) {
+            CtaShare sh{cl.cs, (int64_t)cl.lps.size(), 0.0};
+            for (int32_t k : cl.lps) sh.work += cl.cs + nnz_of(k) / 2000.0;
+            shares.push_back(sh);
+        }
+        const bool serial = share_ctas(shares, max_ctas);
         // power-method start vectors: the single-LP generator, per LP from counter
         // 0, so every LP's vector is a prefix of one vector (computed once)
         int64_t nmax = 0;
@@ -1320,9 +1336,13 @@ struct Run : RunBase {
             pb.count = (int32_t)nbig;
             pb.next = d_next.p + 3;
             int64_t nc = std::min<int64_t>(nbig, nclusters_p);
-            if (max_ctas > 0) nc = std::min<int64_t>(nc, std::max<int64_t>(max_ctas / CLUSTER_CTAS, 1));
+            if (max_ctas > 0) nc = std::min(nc, shares[1].groups);
             ccfg.gridDim = dim3((unsigned)(nc * CLUSTER_CTAS));
             CK(cudaLaunchKernelEx(&ccfg, pkc, pb));
+            if (serial) {
+                CK(cudaEventRecord(ev2, s2));
+                CK(cudaStreamWaitEvent(s, ev2, 0));
+            }
         }
         if (ntile > nbig) {
             PowerArgs<T> ps1 = pg;
@@ -1330,14 +1350,10 @@ struct Run : RunBase {
             ps1.count = (int32_t)(ntile - nbig);
             ps1.next = d_next.p + 1;
             int64_t pgrid = std::min<int64_t>(ntile - nbig, (int64_t)std::max(per_sm_p, 1) * rh.num_sms);
-            if (max_ctas > 0) pgrid = std::min(pgrid, max_ctas);
-            pgrid = std::max<int64_t>(pgrid, 1);
+            if (max_ctas > 0) pgrid = std::min(pgrid, shares[0].groups);
             pk<<<(unsigned)pgrid, BT, 0, s>>>(ps1);
             CK_LAUNCH();
         }
-        int64_t grid = std::min<int64_t>(count, (int64_t)std::max(per_sm, 1) * rh.num_sms);
-        if (max_ctas > 0) grid = std::min(grid, max_ctas);
-        grid = std::max<int64_t>(grid, 1);
         BatchArgs<T> g;
         g.A = CsrView<T, T>{P.a_ptr.p, P.a_idx.p, P.a_val.p, planA.tasks.p, planA.ntasks,
                             planA.ltasks.p, planA.nltasks, planA.counters.p, partA.p};
@@ -1366,18 +1382,22 @@ struct Run : RunBase {
             gb.order = d_order.p;
             gb.count = (int32_t)nbig;
             gb.next = d_next.p + 2;
-            int64_t nc = std::min<int64_t>(nbig, nclusters);
-            if (max_ctas > 0) nc = std::min<int64_t>(nc, std::max<int64_t>(max_ctas / CLUSTER_CTAS, 1));
-            ccfg.gridDim = dim3((unsigned)(nc * CLUSTER_CTAS));
+            if (serial) {
+                CK(cudaEventRecord(ev2, s));
+                CK(cudaStreamWaitEvent(s2, ev2, 0));
+            }
+            ccfg.gridDim = dim3((unsigned)(shares[1].groups * CLUSTER_CTAS));
             CK(cudaLaunchKernelEx(&ccfg, kclu, gb));  // after s2's power method
             CK(cudaEventRecord(ev2, s2));
+            if (serial) CK(cudaStreamWaitEvent(s, ev2, 0));
         }
-        launch_resident(g, classes, ntile, max_ctas);
+        launch_resident(g, classes, ntile, shares, serial);
         if (ntile > nbig) {
+            if (serial)
+                for (cudaEvent_t e : class_ev) CK(cudaStreamWaitEvent(s, e, 0));
             g.order = d_order.p + nbig;
             g.count = (int32_t)(ntile - nbig);
-            grid = std::max<int64_t>(std::min<int64_t>(grid, ntile - nbig), 1);
-            kern<<<(unsigned)grid, BT, 0, s>>>(g);
+            kern<<<(unsigned)shares[0].groups, BT, 0, s>>>(g);
             CK_LAUNCH();
         }
         if (nbig > 0) CK(cudaStreamWaitEvent(s, ev2, 0));
@@ -1463,11 +1483,9 @@ struct Run : RunBase {
     }
 
     template <int CS, int NT>
-    void launch_class(const ResArgs<T>& a, const LaunchClass& c, int64_t max_ctas, cudaStream_t s) {
+    void launch_class(const ResArgs<T>& a, const LaunchClass& c, int64_t groups, cudaStream_t s) {
         auto kern = k_res_pdlp<T, CS, NT>;
         CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RES_MAX_SMEM));
-        int64_t groups = (int64_t)c.lps.size();
-        if (max_ctas > 0) groups = std::min<int64_t>(groups, std::max<int64_t>(max_ctas / CS, 1));
         cudaLaunchAttribute attr[1];
         attr[0].id = cudaLaunchAttributeClusterDimension;
         attr[0].val.clusterDim.x = CS;
@@ -1486,8 +1504,9 @@ struct Run : RunBase {
     std::vector<cudaStream_t> class_s;
     std::vector<cudaEvent_t> class_ev;
     // the classes' kernels, each on its own stream after everything queued on s
+    // (serial: and after the class before it), with the groups of shares[2 + class]
     void launch_resident(const BatchArgs<T>& g, const std::vector<LaunchClass>& classes, int64_t first,
-                         int64_t max_ctas) {
+                         const std::vector<CtaShare>& shares, bool serial) {
         if (classes.empty()) return;
         cudaStream_t s = rh.stream;
         class_ev.resize(classes.size(), nullptr);
@@ -1500,7 +1519,7 @@ struct Run : RunBase {
             const LaunchClass& c = classes[k];
             CK(cudaStreamCreateWithFlags(&class_s[k], cudaStreamNonBlocking));
             CK(cudaEventCreateWithFlags(&class_ev[k], cudaEventDisableTiming));
-            CK(cudaStreamWaitEvent(class_s[k], ready, 0));
+            CK(cudaStreamWaitEvent(class_s[k], serial && k > 0 ? class_ev[k - 1] : ready, 0));
             ResArgs<T> a;
             a.b = g;
             a.b.order = d_order.p + first;
@@ -1511,10 +1530,11 @@ struct Run : RunBase {
             a.x_start = pw_start.p;
             first += (int64_t)c.lps.size();
             const bool wide = c.threads == 512;
-            if (c.cs == 1) wide ? launch_class<1, 512>(a, c, max_ctas, class_s[k]) : launch_class<1, 256>(a, c, max_ctas, class_s[k]);
-            else if (c.cs == 2) wide ? launch_class<2, 512>(a, c, max_ctas, class_s[k]) : launch_class<2, 256>(a, c, max_ctas, class_s[k]);
-            else if (c.cs == 4) wide ? launch_class<4, 512>(a, c, max_ctas, class_s[k]) : launch_class<4, 256>(a, c, max_ctas, class_s[k]);
-            else wide ? launch_class<8, 512>(a, c, max_ctas, class_s[k]) : launch_class<8, 256>(a, c, max_ctas, class_s[k]);
+            const int64_t groups = shares[2 + k].groups;
+            if (c.cs == 1) wide ? launch_class<1, 512>(a, c, groups, class_s[k]) : launch_class<1, 256>(a, c, groups, class_s[k]);
+            else if (c.cs == 2) wide ? launch_class<2, 512>(a, c, groups, class_s[k]) : launch_class<2, 256>(a, c, groups, class_s[k]);
+            else if (c.cs == 4) wide ? launch_class<4, 512>(a, c, groups, class_s[k]) : launch_class<4, 256>(a, c, groups, class_s[k]);
+            else wide ? launch_class<8, 512>(a, c, groups, class_s[k]) : launch_class<8, 256>(a, c, groups, class_s[k]);
             CK(cudaEventRecord(class_ev[k], class_s[k]));
         }
     }
@@ -1556,7 +1576,7 @@ struct Job {
     Handle jh;                 // device and a stream for the cancel flag
     cpdlp_params prm{};
     int items = BATCH_ITEMS;
-    int64_t max_ctas = 0;      // > 0: at most this many CTAs per launch
+    int64_t max_ctas = 0;      // > 0: at most this many CTAs of a phase run at a time
     std::vector<LPData> lps;
     std::vector<double> target;  // final relative KKT tolerance per LP
     std::vector<std::vector<double>> x, y;

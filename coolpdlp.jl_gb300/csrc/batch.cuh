@@ -16,8 +16,9 @@ struct Job;
 // the job's own stream and launches the solve; returns without waiting for
 // it.  reltol (count entries or NULL) gives each LP's target relative KKT
 // error; x0 / y0 (count pointers or NULL; NULL entries = cold start) give
-// warm starts in original units.  max_ctas > 0 caps the CTAs of each launch
-// (leaving SMs to jobs submitted later).
+// warm starts in original units.  max_ctas > 0 caps the CTAs that each
+// phase of the job runs at a time, over all its launches (cta_budget.h), which
+// leaves SMs to jobs submitted later; an LP on a cluster takes the cluster's.
 Job* job_submit(Handle& h, int64_t count, const cpdlp_lp* lps, const cpdlp_params* params,
                 const double* reltol, const double* const* x0, const double* const* y0,
                 int64_t max_ctas);

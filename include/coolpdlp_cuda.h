@@ -464,8 +464,9 @@ int cpdlp_batch_solve(cpdlp_handle* h, int64_t count, const cpdlp_lp* lps,
  * termination_reltol stop there in FP32 and finish in an FP64 phase
  * warm-started from the FP32 solution.  x0 / y0: `count` warm starts in
  * original units (NULL, or NULL entries, for a cold start).  max_ctas > 0
- * caps the CTAs (concurrent LPs) of the job's launches, leaving SMs to jobs
- * submitted later; 0 fills the GPU.
+ * caps the CTAs that a phase of the job runs at a time, over all its launches,
+ * leaving SMs to jobs submitted later (an LP on a thread-block cluster takes the
+ * CTAs of the cluster, of which one may be more than the cap); 0 fills the GPU.
  * Each LP is available as soon as its CTA finishes it: the kernel writes the
  * LP's result into mapped host memory and sets its done flag.
  * cpdlp_poll never blocks: it takes every LP finished so far, launches the
