@@ -744,9 +744,9 @@ struct ResArgs {
 template <class T, int CS, int NT>
 __device__ __forceinline__ void res_kkt(ResGeo& G, const BatchArgs<T>& b, const BatchCtl& C,
                                         const T* gx, const T* gy, cpdlp_kkt_errors* out, double* sh,
-                                        int& phase) {
+                                        int& phase, ResWait& W) {
     double v[5];
-    res_kkt_sums<T, CS, NT>(G, gx, gy, b.invD1t + C.L.row_off, b.invD2t + C.L.col_off, v, sh, phase);
+    res_kkt_sums<T, CS, NT>(G, gx, gy, b.invD1t + C.L.row_off, b.invD2t + C.L.col_off, v, sh, phase, W);
     if (threadIdx.x == 0) {
         out->primal = sqrt(v[0]);
         out->primal_scale = C.pscale;
@@ -802,7 +802,7 @@ __device__ __forceinline__ void solve_resident(const ResArgs<T>& g, BatchCtl& C,
             q[2] += sv * sv;
             q[3] += cj * cj;
         }
-        res_sum<4, CS, NT / 32>(q, sh, phase);
+        res_sum<4, CS, NT / 32>(q, sh, phase, W);
         const double cn = sqrt(q[3]), bn = sqrt(q[1]);
         omega = !pdlp ? 1.0 : (cn > b.prm.zero_tol && bn > b.prm.zero_tol) ? cn / bn : 1.0;
         if (pdlp && C.L.omega0 > 0) omega = C.L.omega0;
@@ -844,7 +844,7 @@ __device__ __forceinline__ void solve_resident(const ResArgs<T>& g, BatchCtl& C,
         for (int p = 0; p < nv; p++)
             res_kkt<T, CS, NT>(G, b, C, p == 0 ? d.x : p == 1 ? d.xa : p == 2 ? d.xl : d.xal,
                                p == 0 ? d.y : p == 1 ? d.ya : p == 2 ? d.yl : d.yal, &C.e[p], sh,
-                               phase);
+                               phase, W);
         // ---- the clock and the cancel flag, read once for the group by rank 0
         if (rank == 0 && tid == 0) {
             C.tl_hit = (double)(global_ns() - C.t_start) >= tlim_ns ? 1 : 0;
@@ -863,7 +863,7 @@ __device__ __forceinline__ void solve_resident(const ResArgs<T>& g, BatchCtl& C,
         int flag = C.flag;
         __syncthreads();
         if (flag == 2) {
-            res_kkt<T, CS, NT>(G, b, C, gxr, gyr, &C.e_restart, sh, phase);
+            res_kkt<T, CS, NT>(G, b, C, gxr, gyr, &C.e_restart, sh, phase, W);
             if (tid == 0) {
                 C.restart_valid = 1;
                 const double w = C.omega;
@@ -891,7 +891,7 @@ __device__ __forceinline__ void solve_resident(const ResArgs<T>& g, BatchCtl& C,
                 q[1] += dd * dd;
                 gyr[i] = v;
             }
-            res_sum<2, CS, NT / 32>(q, sh, phase);
+            res_sum<2, CS, NT / 32>(q, sh, phase, W);
             const double dx = sqrt(q[0]), dy = sqrt(q[1]), th = b.prm.primal_weight_damping;
             if (dx > b.prm.zero_tol && dy > b.prm.zero_tol)
                 omega = exp(th * log(dy / dx) + (1.0 - th) * log(omega));
@@ -915,7 +915,8 @@ __device__ __forceinline__ void solve_resident(const ResArgs<T>& g, BatchCtl& C,
     for (int i = gt; i < m; i += GT) b.out_y[r0 + i] = b.D1[r0 + i] * (double)__ldcg(d.y + i);
     __threadfence_system();
     Grp<CS>::sync();
-    // (a wait that ran out leaves the done flag unset: the host reports an error)
+    // (a wait that ran out in any CTA of the group, which the last check's sums
+    // told all of them, leaves the done flag unset: the host reports an error)
     if (rank == 0 && tid == 0 && !W.failed) publish(b, C, eta, theta, omega, tab.es);
 }
 

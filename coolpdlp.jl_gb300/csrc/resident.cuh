@@ -105,8 +105,11 @@ __device__ __forceinline__ void res_put(double* p, double v, int rank) {
 // some of both vectors: res_plan gives each at least one slice of A and of A'.
 struct ResWait {
     uint64_t bar[2];   // mbarriers: 0 for y (and Ax), 1 for xbar (and x)
-    int failed;        // a wait ran out (never, unless the kernel is wrong)
+    // a wait ran out (never, unless the kernel is wrong): here, or in any CTA of
+    // the group before the last sum over the group (res_flag)
+    int failed;
 };
+constexpr int RES_TRIES = 1 << 20;  // of a wait
 // one warp sends slice block p[0..32) (whole in local shared memory)
 template <int CS, class V>
 __device__ __forceinline__ void res_send(const V* p, uint64_t* bar, int rank) {
@@ -130,18 +133,21 @@ __device__ __forceinline__ void res_send(const V* p, uint64_t* bar, int rank) {
     }
 }
 // waits for `bytes` of the other ranks; parity: the barrier's phases so far,
-// modulo 2 (advanced).  Also a CTA barrier.
+// modulo 2 (advanced), and RES_GAVE_UP once a wait ran out: a phase that did not
+// complete takes no second arrival.  Also a CTA barrier.
+constexpr unsigned RES_GAVE_UP = 1u << 31;
 template <int CS>
-__device__ __forceinline__ void res_receive(ResWait& W, int which, uint32_t bytes, unsigned& parity) {
+__device__ __forceinline__ void res_receive(ResWait& W, int which, uint32_t bytes, unsigned& parity,
+                                            int most_tries = RES_TRIES) {
     __syncthreads();
     if constexpr (CS > 1) {
         const uint32_t mb = smem_addr(&W.bar[which]);
-        if (threadIdx.x == 0)
+        if (threadIdx.x == 0 && !(parity & RES_GAVE_UP))
             asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(mb), "r"(bytes)
                          : "memory");
         const unsigned par = (parity >> which) & 1u;
         uint32_t ok = 0;
-        for (int tries = 0; tries < (1 << 20); tries++) {
+        for (int tries = 0; tries < most_tries; tries++) {
             asm volatile(
                 "{\n\t.reg .pred p;\n\t"
                 "mbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
@@ -151,8 +157,11 @@ __device__ __forceinline__ void res_receive(ResWait& W, int which, uint32_t byte
                 : "memory");
             if (ok || *(volatile int*)&W.failed) break;
         }
-        if (!ok) W.failed = 1;
         parity ^= 1u << which;
+        if (!ok) {
+            W.failed = 1;
+            parity |= RES_GAVE_UP;
+        }
     }
 }
 // before the first exchange (thread 0 of every CTA, then a group barrier)
@@ -249,8 +258,13 @@ constexpr int RES_SUMS = 5;  // most values of one sum
 // of the power method from 7.5 to 4.5 us (1,000 x 2,000, 16 warps a CTA).
 // sh: res_sh<CS, NW>() doubles; `phase` alternates the halves, so that a fast
 // CTA's next sums do not meet a slow one's reads.
+// With the sums every CTA learns whether a wait ran out in any of them: a CTA
+// that acted on its own wait alone would leave its loops, and the group's
+// barriers, at another point than the others.
 template <int CS, int NW>
-constexpr int res_sh() { return 2 * RES_SUMS * CS * NW + 8; }
+constexpr int res_slot_size() { return RES_SUMS * CS * NW + CS; }
+template <int CS, int NW>
+constexpr int res_sh() { return 2 * res_slot_size<CS, NW>() + 8; }
 // a warp's part of the sums, stored into every CTA's slots
 template <int Q, int CS, int NW>
 __device__ __forceinline__ void res_partial(const double (&v)[Q], double* slot, bool busy) {
@@ -300,6 +314,23 @@ __device__ __forceinline__ void res_partial(const double (&v)[Q], double* slot, 
         res_put<CS>(slot + which * P + rank * NW + w, d, rank);
     __syncwarp();
 }
+// whether a wait ran out in any CTA of the group before its res_put_flag (one
+// warp each, the group barrier between them); the same answer in every CTA
+template <int CS, int NW>
+__device__ __forceinline__ void res_put_flag(double* slot, const ResWait& W) {
+    const int lane = threadIdx.x & 31;
+    if (lane < CS) {
+        const double f = *(const volatile int*)&W.failed ? 1.0 : 0.0;
+        const uint32_t a = smem_addr(slot + RES_SUMS * CS * NW + res_rank<CS>());
+        asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(map_rank(a, lane)), "d"(f) : "memory");
+    }
+    __syncwarp();
+}
+template <int CS, int NW>
+__device__ __forceinline__ bool res_flag(const double* slot) {
+    const int lane = threadIdx.x & 31;
+    return __any_sync(FULL_MASK, lane < CS && slot[RES_SUMS * CS * NW + lane] != 0.0);
+}
 // value q of all warps of the group, by one warp (whole in every lane)
 template <int CS, int NW>
 __device__ __forceinline__ double res_total(const double* slot, int q) {
@@ -315,17 +346,21 @@ __device__ __forceinline__ double res_total(const double* slot, int q) {
 }
 template <int CS, int NW>
 __device__ __forceinline__ double* res_slot(double* sh, int& phase) {
-    double* slot = sh + 8 + phase * (RES_SUMS * CS * NW);
+    double* slot = sh + 8 + phase * res_slot_size<CS, NW>();
     phase ^= 1;
     return slot;
 }
 template <int Q, int CS, int NW, class F>
-__device__ __forceinline__ void res_sum(double (&v)[Q], double* sh, int& phase, bool busy,
+__device__ __forceinline__ void res_sum(double (&v)[Q], double* sh, int& phase, ResWait& W, bool busy,
                                         F&& finish) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     double* slot = res_slot<CS, NW>(sh, phase);
     res_partial<Q, CS, NW>(v, slot, busy);
+    if constexpr (CS > 1)
+        if (w == NW - 1) res_put_flag<CS, NW>(slot, W);
     res_sync<CS>();
+    if constexpr (CS > 1)
+        if (w == NW - 1 && res_flag<CS, NW>(slot) && lane == 0) W.failed = 1;
     if (w < Q) {
         const double s = res_total<CS, NW>(slot, w);
         if (lane == 0) sh[w] = finish(w, s);
@@ -337,8 +372,9 @@ __device__ __forceinline__ void res_sum(double (&v)[Q], double* sh, int& phase, 
 }
 
 template <int Q, int CS, int NW>
-__device__ __forceinline__ void res_sum(double (&v)[Q], double* sh, int& phase, bool busy = true) {
-    res_sum<Q, CS, NW>(v, sh, phase, busy, [](int, double s) { return s; });
+__device__ __forceinline__ void res_sum(double (&v)[Q], double* sh, int& phase, ResWait& W,
+                                        bool busy = true) {
+    res_sum<Q, CS, NW>(v, sh, phase, W, busy, [](int, double s) { return s; });
 }
 
 // the resident LP as one CTA of its group sees it (in shared memory)
@@ -613,7 +649,8 @@ __device__ __noinline__ void res_steps(const ResGeo& G, double eta, double omega
 // y and xb
 template <class T, int CS, int NT>
 __device__ __noinline__ void res_kkt_sums(const ResGeo& G, const T* gx, const T* gy, const T* invD1,
-                                          const T* invD2, double (&out)[5], double* sh, int& phase) {
+                                          const T* invD2, double (&out)[5], double* sh, int& phase,
+                                          ResWait& W) {
     const int lane = threadIdx.x & 31;
     res_load_xb<T, NT>(G, gx);
     res_load_y<T, NT>(G, gy);
@@ -659,7 +696,7 @@ __device__ __noinline__ void res_kkt_sums(const ResGeo& G, const T* gx, const T*
         }
     }
     __syncwarp();
-    res_sum<5, CS, NT / 32>(v, sh, phase, (int)(threadIdx.x >> 5) < max(G.LA, G.LAt));
+    res_sum<5, CS, NT / 32>(v, sh, phase, W, (int)(threadIdx.x >> 5) < max(G.LA, G.LAt));
 #pragma unroll
     for (int q = 0; q < 5; q++) out[q] = v[q];
 }
@@ -741,6 +778,7 @@ __device__ __noinline__ void res_power(const ResGeo& G, int64_t it0, int64_t max
             if (wq == 2) {
                 const double res = sqrt(s);
                 f = res <= tol || (rtol > 0 && res <= rtol * theta) ? -1.0 - res : res;
+                if (s == -INFINITY) f = s;  // a wait ran out: all CTAs leave here
             }
             if (lane == 0) sh[wq] = f;
             __syncwarp();
@@ -755,7 +793,7 @@ __device__ __noinline__ void res_power(const ResGeo& G, int64_t it0, int64_t max
             residual = sh[2];
             it++;
             stop = it > maxiter || __double_as_longlong(residual) < 0;
-            if (stop || it - it0 >= max_here || (CS > 1 && W.failed)) break;
+            if (stop || it - it0 >= max_here) break;
         }
         if (slot) {
             theta = sh[0];
@@ -778,7 +816,9 @@ __device__ __noinline__ void res_power(const ResGeo& G, int64_t it0, int64_t max
         }
         pending = slot != nullptr;
         res_receive<CS>(W, 0, G.remA * 8u, parity);
-        double v[3] = {0.0, 0.0, r2};
+        // (a sum of squares is never -inf; where it is no number already, the next
+        // sums tell the group)
+        double v[3] = {0.0, 0.0, CS > 1 && (parity & RES_GAVE_UP) ? -INFINITY : r2};
 #pragma unroll 1
         for (int l = w; l < LAt; l += NW) {
             const uint32_t o = offAt[l];
@@ -799,6 +839,7 @@ __device__ __noinline__ void res_power(const ResGeo& G, int64_t it0, int64_t max
         res_receive<CS>(W, 1, G.remAt * 8u, parity);
     }
     keep();
+    if (CS > 1 && threadIdx.x == 0 && residual == -INFINITY) W.failed = 1;
     if (__double_as_longlong(residual) < 0) residual = -1.0 - residual;
     P.theta = theta;
     P.residual = residual;

@@ -42,7 +42,7 @@ __global__ void __launch_bounds__(RS_NT) k_res_block(const __grid_constant__ Blo
         double v[5];
         res_kkt_sums<T, CS, RS_NT>(G, p == 0 ? d.x : p == 1 ? d.xa : p == 2 ? d.xl : d.xal,
                                    p == 0 ? d.y : p == 1 ? d.ya : p == 2 ? d.yl : d.yal, g.invD1,
-                                   g.invD2, v, sh, phase);
+                                   g.invD2, v, sh, phase, W);
         if (G.rank == 0 && threadIdx.x == 0)
             for (int q = 0; q < 5; q++) g.b.out[5 * p + q] = v[q];
     }
