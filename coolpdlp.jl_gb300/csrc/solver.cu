@@ -35,6 +35,7 @@
 #include "ell.cuh"
 #include "epilogues.cuh"
 #include "solver.cuh"
+#include "wait_flag.h"
 
 namespace cpdlp {
 
@@ -1509,6 +1510,11 @@ struct StateT : StateBase {
     // instead of evaluating): how many, 0 when none are ready
     int res_nv = 0;
     double* res_out() { return h->pinned_area(sizeof(double) * 64) + 32; }
+    WaitFlag gave_up;
+    // after a wait for the stream
+    void check_waits() {
+        if (gave_up.take()) fail(CPDLP_ERR_CUDA, "resident block: a wait ran out");
+    }
 
     // `len` steps in one resident launch, with the KKT sums of nv iterates
     void run_resident(int len, int nv) {
@@ -1522,7 +1528,7 @@ struct StateT : StateBase {
         b.avg = pdlp() ? 1 : 0;
         b.nv = nv;
         b.out = res_out();
-        res_out()[20] = 0.0;
+        gave_up.arm(b.out + 20);
         res_single_block<T>(*PT, b, h->stream);
         launches += 1;
         res_nv = nv;
@@ -1578,7 +1584,6 @@ struct StateT : StateBase {
     }
 
     void step(int64_t count) override {
-        res_out()[20] = 0.0;
         const int ce = prm.check_every > 0 ? prm.check_every : 100;
         while (count >= ce) {
             run_block(ce);
@@ -1586,7 +1591,7 @@ struct StateT : StateBase {
         }
         while (count-- > 0) run_single();
         CK(cudaStreamSynchronize(h->stream));
-        if (PT->rlp.cs > 0 && res_out()[20] != 0.0) fail(CPDLP_ERR_CUDA, "resident block: a wait ran out");
+        check_waits();
     }
 
     // KKT errors (errors.jl:65-109) of NV (1 or 4) (x, y) pairs in ONE
@@ -1658,6 +1663,7 @@ struct StateT : StateBase {
     void kkt_multi(const T* const (&xs)[NV], const T* const (&ys)[NV], cpdlp_kkt_errors* out) {
         if (kkt_hook) {
             kkt_hook(NV, xs, ys, out);
+            check_waits();
             return;
         }
         ProblemT<T>& P = *PT;
@@ -1666,8 +1672,8 @@ struct StateT : StateBase {
             // evaluated by the block that produced the iterates
             res_nv = 0;
             CK(cudaStreamSynchronize(s));
+            check_waits();
             const double* v = res_out();
-            if (v[20] != 0.0) fail(CPDLP_ERR_CUDA, "resident block: a wait ran out");
             for (int p = 0; p < NV; p++, v += 5) errors_from(v[0], v[1], v[2], v[3], v[4], out[p]);
             return;
         }
@@ -1680,6 +1686,7 @@ struct StateT : StateBase {
         double* pin = h->pinned_area(sizeof(double) * 64);
         CK(cudaMemcpyAsync(pin, P.red_out.p, sizeof(double) * 5 * NV, cudaMemcpyDeviceToHost, s));
         CK(cudaStreamSynchronize(s));
+        check_waits();
         for (int p = 0; p < NV; p++) {
             const double* col = pin + 2 * NV + 3 * p;
             errors_from(pin[2 * p], pin[2 * p + 1], col[0], col[1], col[2], out[p]);
