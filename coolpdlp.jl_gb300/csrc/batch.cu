@@ -11,8 +11,9 @@
 // check_every fused PDHG steps (pdlp.jl:96-136) with the four-iterate KKT
 // check, restart and termination logic (pdlp.jl:138-196, restart.jl:40-57,
 // termination.jl:89-101) run by the CTA itself, thread 0 taking the FP64
-// decisions.  Every loop is bounded by the LP's pass limit and time limit; CTAs
-// wait only on CTAs of their own cluster.
+// decisions.  Every loop is bounded: the power method by its iteration limit, the
+// blocks by the LP's pass limit and by its time limit, which counts from the
+// first block.  CTAs wait only on CTAs of their own cluster.
 //
 // An LP's route and arithmetic depend only on the LP, the value type and the
 // tile size (its slices or tiles, the thread that owns each row, the order of
@@ -784,6 +785,9 @@ __device__ __forceinline__ void solve_resident(const ResArgs<T>& g, BatchCtl& C,
         theta = P.theta;
         power_it = P.it;
     }
+    // an LP's clock starts with its steps on both routes (the tile kernels' power
+    // method is a kernel before theirs)
+    if (tid == 0) C.t_start = global_ns();
     const double eta = b.prm.invnorm_scaling * (1.0 / sqrt(theta));
     const T *c = b.c + c0, *lv = b.lv + c0, *uv = b.uv + c0, *lc = b.lc + r0, *uc = b.uc + r0;
     res_bounds<T, CS, NT>(G, c, lv, uv, lc, uc);
@@ -948,10 +952,7 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 4 : 2) k_res_pdlp(ResArgs<T> g
             }
             Grp<CS>::sync();  // rank 0's copy is read before it changes or exits
         }
-        if (threadIdx.x == 0 && C.lp >= 0) {
-            C.L = g.b.lps[C.lp];
-            C.t_start = global_ns();
-        }
+        if (threadIdx.x == 0 && C.lp >= 0) C.L = g.b.lps[C.lp];
         __syncthreads();
         if (C.lp < 0) break;
         if (C.cancelled) skip_one<T, CS, NT>(g.b, C);
