@@ -234,6 +234,24 @@ void build_T(Handle& h, Matrix& M, CscPair& S) {
     CK(cudaStreamSynchronize(s));
 }
 
+// The scratch of rows in several pieces (a counter a row, a partial sum a piece)
+// serves one product at a time: the matrix's own on the stream of its handle, a
+// product's own (in stream order) on another handle's.
+template <class T>
+struct PieceScratch {
+    DBuf<int32_t> counters;
+    DBuf<T> partials;
+    template <class View>
+    void give(Handle& h, const Matrix& M, int32_t npieces, size_t ncounters, View& v) {
+        if (&h == M.h || npieces == 0) return;
+        counters.alloc(ncounters);
+        partials.alloc((size_t)npieces);
+        CK(cudaMemsetAsync(counters.p, 0, counters.bytes(), h.stream));
+        v.counters = counters.p;
+        v.partials = partials.p;
+    }
+};
+
 template <class T>
 void spmv_T(Handle& h, const Matrix& M, const T* b, T* c, double alpha, double beta) {
     cudaStream_t s = h.stream;
@@ -254,12 +272,16 @@ void spmv_T(Handle& h, const Matrix& M, const T* b, T* c, double alpha, double b
     const T* val = csr_vals<T>(const_cast<Matrix&>(M)).p;
     const MulEpi<T> e{c, a, bb, ub};
     const SellSide<T>& L = sell_of<T>(const_cast<Matrix&>(M));
+    PieceScratch<T> scratch;
     if (L.on) {
-        launch_sell(sell_view(L, ptr, idx, val), b, e, s);
+        SellView<T> v = sell_view(L, ptr, idx, val);
+        scratch.give(h, M, L.npieces, L.counters.n, v);
+        launch_sell(v, b, e, s);
         return;
     }
     CsrView<T, T> v{ptr, idx, val, M.plan.tasks.p, M.plan.ntasks, M.plan.ltasks.p, M.plan.nltasks,
                     M.plan.counters.p, reinterpret_cast<T*>(M.part.p)};
+    scratch.give(h, M, M.plan.npieces, M.plan.counters.n, v);
     launch_tiles<1>(M.plan, v, VecSet<T, 1>{{b}}, e, s);
 }
 
@@ -320,6 +342,8 @@ void spmv_pm1(Handle& h, const Matrix& M, const float* b, float* c, double alpha
     CsrView<Pm1, float> v{M.ptr.p, M.idx.p, nullptr, M.plan.tasks.p, M.plan.ntasks,
                           M.plan.ltasks.p, M.plan.nltasks, M.plan.counters.p,
                           reinterpret_cast<float*>(M.part.p)};
+    PieceScratch<float> scratch;
+    scratch.give(h, M, M.plan.npieces, M.plan.counters.n, v);
     MulEpi<float> e{c, (float)alpha, (float)beta, beta != 0.0};
     launch_tiles<1>(M.plan, v, VecSet<float, 1>{{b}}, e, h.stream);
 }

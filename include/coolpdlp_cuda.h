@@ -278,7 +278,9 @@ int cpdlp_matrix_export(cpdlp_handle* h, const cpdlp_matrix* A, int64_t* ptr,
 
 /* LinearAlgebra.mul!(c, A, b, alpha, beta) (mat_csr.jl:81-92, mat_ell.jl:91-102,
  * mat_coo.jl:68-80): c = alpha*A*b + beta*c with b, c DEVICE vectors of the
- * matrix eltype.  beta == 0 is a strong zero: c is not read. */
+ * matrix eltype.  beta == 0 is a strong zero: c is not read.  h may be another
+ * handle than the one that built A (once that call has returned), and several
+ * handles may multiply by one matrix at the same time. */
 int cpdlp_spmv(cpdlp_handle* h, const cpdlp_matrix* A, const void* b, void* c,
                double alpha, double beta);
 
