@@ -166,8 +166,7 @@ void build_engines(Matrix& M, const std::vector<int32_t>& hp, const DBuf<int32_t
     // FP32, few entries in long rows
     SellSide<T>& L = sell_of<T>(M);
     if (M.nnz > 0) {
-        build_sell<T>(L, hp, ptr.p, idx.p, val.p, M.m, 32 * items, s);
-        L.on = (double)L.entries <= SELL_MAX_PADDING * (double)M.nnz &&
+        L.on = build_sell<T>(L, hp, ptr.p, idx.p, val.p, M.m, 32 * items, s) &&
                (sizeof(T) == 8 || (double)L.long_nnz <= SELL_MAX_LONG_F32 * (double)M.nnz);
         if (!L.on) L.release();
     }

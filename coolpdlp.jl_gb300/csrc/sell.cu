@@ -74,11 +74,11 @@ __global__ void k_sell_fill(const int32_t* __restrict__ ptr, const int32_t* __re
 }  // namespace
 
 template <class T>
-void build_sell(SellSide<T>& S, const std::vector<int32_t>& hp, const int32_t* ptr,
+bool build_sell(SellSide<T>& S, const std::vector<int32_t>& hp, const int32_t* ptr,
                 const int32_t* idx, const T* val, int64_t rows, int tile, cudaStream_t s) {
     S.release();
     S.tile = tile;
-    if (rows <= 0) return;
+    if (rows <= 0) return true;
     // rows longer than LONG_ROW
     std::vector<int4> longs;
     int32_t slot = 0, id = 0;
@@ -138,16 +138,22 @@ void build_sell(SellSide<T>& S, const std::vector<int32_t>& hp, const int32_t* p
         S.perm.release();
     }
     S.entries = 32 * (int64_t)sorted_units;
+    if ((double)S.entries > SELL_MAX_PADDING * (double)hp[(size_t)rows]) {
+        CK(cudaStreamSynchronize(s));
+        S.release();
+        return false;
+    }
     S.idx.alloc((size_t)std::max<int64_t>(S.entries, 1));
     if (val) S.val.alloc((size_t)std::max<int64_t>(S.entries, 1));
     k_sell_fill<T><<<grid_for(padded, 256), 256, 0, s>>>(ptr, idx, val, S.off.p, S.len.p, S.perm.p, padded,
                                                          S.idx.p, S.val.p);
     CK_LAUNCH();
     CK(cudaStreamSynchronize(s));  // (the host task list and the temporaries go out of scope)
+    return true;
 }
-template void build_sell<float>(SellSide<float>&, const std::vector<int32_t>&, const int32_t*,
+template bool build_sell<float>(SellSide<float>&, const std::vector<int32_t>&, const int32_t*,
                                 const int32_t*, const float*, int64_t, int, cudaStream_t);
-template void build_sell<double>(SellSide<double>&, const std::vector<int32_t>&, const int32_t*,
+template bool build_sell<double>(SellSide<double>&, const std::vector<int32_t>&, const int32_t*,
                                  const int32_t*, const double*, int64_t, int, cudaStream_t);
 
 }  // namespace cpdlp

@@ -68,10 +68,12 @@ struct SellView {
 };
 
 // The slices of a CSR (device; hp: its row pointer on the host); tile: the
-// piece size of long rows; val null: narrow storage.  Leaves S.on false; S.entries
-// tells the padding.
+// piece size of long rows; val null: narrow storage.  False, and nothing kept, when
+// they would hold more than SELL_MAX_PADDING times the nonzeros: that is seen
+// before they are allocated (a window with one row of 64 entries and 255 empty ones
+// pads 32 times).  Leaves S.on false.
 template <class T>
-void build_sell(SellSide<T>& S, const std::vector<int32_t>& hp, const int32_t* ptr,
+bool build_sell(SellSide<T>& S, const std::vector<int32_t>& hp, const int32_t* ptr,
                 const int32_t* idx, const T* val, int64_t rows, int tile, cudaStream_t s);
 
 template <class V, class T>

@@ -602,9 +602,9 @@ void tune_sell(Handle& h, ProblemT<T>& P, int side, const std::vector<int32_t>& 
     if (decided == 0) return;
     cudaStream_t s = h.stream;
     SellSide<T>& S = P.sell[side];
-    build_sell<T>(S, hp, side == 0 ? P.a_ptr.p : P.at_ptr.p, side == 0 ? P.a_idx.p : P.at_idx.p,
-                  side == 0 ? P.a_val.p : P.at_val.p, rows, 32 * items, s);
-    bool keep = (double)S.entries <= SELL_MAX_PADDING * (double)P.nnz;
+    bool keep = build_sell<T>(S, hp, side == 0 ? P.a_ptr.p : P.at_ptr.p,
+                              side == 0 ? P.a_idx.p : P.at_idx.p,
+                              side == 0 ? P.a_val.p : P.at_val.p, rows, 32 * items, s);
     if (decided < 0 && keep) {
         struct Events {
             cudaEvent_t e[2] = {};
@@ -1103,11 +1103,10 @@ ProblemBase* make_problem(Handle& h, const cpdlp_lp* lp, const cpdlp_params* prm
         if (!pm1) res_single_build<T>(*P, hp2, hp1, s);
         for (int side = 0; side < 2 && P->rlp.cs == 0 && nnz > 0; side++) {
             SellSide<T>& S = P->sell[side];
-            build_sell<T>(S, side == 0 ? hp2 : hp1, side == 0 ? P->a_ptr.p : P->at_ptr.p,
-                          side == 0 ? P->a_idx.p : P->at_idx.p,
-                          pm1 ? nullptr : side == 0 ? P->a_val.p : P->at_val.p,
-                          side_rows(*P, side), 32 * (side == 0 ? items_A : items_At), s);
-            S.on = (double)S.entries <= SELL_MAX_PADDING * (double)nnz &&
+            S.on = build_sell<T>(S, side == 0 ? hp2 : hp1, side == 0 ? P->a_ptr.p : P->at_ptr.p,
+                                 side == 0 ? P->a_idx.p : P->at_idx.p,
+                                 pm1 ? nullptr : side == 0 ? P->a_val.p : P->at_val.p,
+                                 side_rows(*P, side), 32 * (side == 0 ? items_A : items_At), s) &&
                    (sizeof(T) == 8 || (double)S.long_nnz <= SELL_MAX_LONG_F32 * (double)nnz);
             if (!S.on) S.release();
         }
