@@ -120,15 +120,20 @@ class Problem:
         self.p = p
 
     def layout(self) -> dict:
-        """cpdlp_problem_layout: format, CSR tile size and ELL width of the
-        products over the rows of A ("A") and of A' ("At")."""
+        """cpdlp_problem_layout and cpdlp_problem_engine: format, CSR tile size
+        and ELL width of the rows of A ("A") and of A' ("At"), and the engine that
+        the steps run on ("tiles", "slices", "ell", or "resident" on so many CTAs)."""
         fmt = (c_int32 * 2)()
         tile = (c_int32 * 2)()
         width = (c_int64 * 2)()
         self.handle.check(self.handle.lib.cpdlp_problem_layout(self.p, fmt, tile, width))
+        engine = (c_int32 * 2)()
+        ctas = c_int32()
+        self.handle.check(self.handle.lib.cpdlp_problem_engine(self.p, engine, byref(ctas)))
         names = {A.FMT_CSR: "CSR", A.FMT_ELL: "ELL"}
         return {side: {"format": names.get(fmt[k], str(fmt[k])), "tile_nnz": int(tile[k]),
-                       "ell_width": int(width[k])} for k, side in enumerate(("A", "At"))}
+                       "ell_width": int(width[k]), "engine": A.ENGINES[engine[k]],
+                       "resident_ctas": int(ctas.value)} for k, side in enumerate(("A", "At"))}
 
     def order(self):
         """cpdlp_problem_order: None when the solve runs in the caller's order,

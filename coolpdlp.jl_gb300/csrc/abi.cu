@@ -380,6 +380,14 @@ int cpdlp_problem_layout(const cpdlp_problem* p, int32_t* format, int32_t* tile_
     return CPDLP_OK;
 }
 
+int cpdlp_problem_engine(const cpdlp_problem* p, int32_t* engine, int32_t* resident_ctas) {
+    if (!p) return CPDLP_ERR_ARGUMENT;
+    const ProblemBase* P = reinterpret_cast<const ProblemBase*>(p);
+    for (int sd = 0; engine && sd < 2; sd++) engine[sd] = P->engine(sd);
+    if (resident_ctas) *resident_ctas = P->resident_ctas();
+    return CPDLP_OK;
+}
+
 int cpdlp_problem_order(cpdlp_handle* h, const cpdlp_problem* p, int32_t* ordered,
                         int64_t* order_row, int64_t* order_col) {
     NEED(h);

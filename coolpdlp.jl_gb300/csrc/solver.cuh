@@ -68,6 +68,10 @@ struct ProblemBase {
     // order (order_to_internal / order_to_user)
     bool ordered = false;
     DBuf<int32_t> order_row, order_col;
+    // what the solve's steps over each matrix run on (CPDLP_ENGINE_*), and the
+    // CTAs of the group that a resident LP runs on (0: not resident)
+    virtual int32_t engine(int side) const = 0;
+    virtual int32_t resident_ctas() const = 0;
 };
 
 void order_to_internal(const ProblemBase& P, int side, double* v, cudaStream_t s);
@@ -88,6 +92,12 @@ struct ProblemT : ProblemBase {
     // a small LP's slices for the resident kernels (rlp.cs = 0: not resident)
     ResStore<T> res;
     ResLP rlp{};
+    int32_t engine(int side) const override {
+        return rlp.cs > 0 ? CPDLP_ENGINE_RESIDENT
+             : sell[side].on ? CPDLP_ENGINE_SLICES
+             : fmt[side] == CPDLP_FMT_ELL ? CPDLP_ENGINE_ELL : CPDLP_ENGINE_TILES;
+    }
+    int32_t resident_ctas() const override { return rlp.cs; }
     // 1 ./ D1 and 1 ./ D2 in T for the KKT terms (FP32 problems keep a copy;
     // FP64 problems use invD1 / invD2 themselves)
     DBuf<T> invD1t, invD2t;

@@ -386,12 +386,26 @@ int cpdlp_solve(cpdlp_handle* h, const cpdlp_lp* lp, const cpdlp_params* params,
 int cpdlp_solve_history(const cpdlp_handle* h, int64_t* kkt_passes, cpdlp_kkt_errors* errs,
                         int64_t capacity, int64_t* count);
 
-/* The product layout the solve of this problem uses, per matrix ([0]: rows
- * of A, the dual step; [1]: rows of A', the primal step): format
- * (CPDLP_FMT_CSR or CPDLP_FMT_ELL), CSR tile size in nonzeros (0 for ELL)
- * and ELL width (0 for CSR).  Any pointer may be NULL.  EXT (measurement). */
+/* How the problem stores its matrices ([0]: rows of A, [1]: rows of A'): format
+ * (CPDLP_FMT_CSR or CPDLP_FMT_ELL), CSR tile size in nonzeros (0 for ELL) and
+ * ELL width (0 for CSR).  The KKT checks run on these; the steps where
+ * cpdlp_problem_engine gives tiles or ELL.  Any pointer may be NULL.  EXT
+ * (measurement). */
 int cpdlp_problem_layout(const cpdlp_problem* p, int32_t* format, int32_t* tile_nnz,
                          int64_t* width);
+
+/* What the solve's steps run on, per matrix (engine[0]: rows of A, the dual step;
+ * engine[1]: rows of A', the primal step). */
+enum {
+    CPDLP_ENGINE_TILES = 0,    /* warp tiles of the CSR */
+    CPDLP_ENGINE_SLICES = 1,   /* 32-row slices beside the CSR */
+    CPDLP_ENGINE_ELL = 2,      /* the ELL slabs */
+    CPDLP_ENGINE_RESIDENT = 3  /* the whole LP in the shared memory of resident_ctas CTAs */
+};
+/* *resident_ctas = 0 for an LP that is not resident.  (A batch or a job chooses
+ * per LP: this is the single-LP solve's choice.)  Either pointer may be NULL.
+ * EXT (measurement). */
+int cpdlp_problem_engine(const cpdlp_problem* p, int32_t* engine, int32_t* resident_ctas);
 
 /* Whether the solve of this problem runs in density order
  * (CPDLP_TILE_DENSITY_ORDER); *ordered = 1 or 0.  With order_row (m) and

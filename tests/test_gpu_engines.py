@@ -1,0 +1,33 @@
+"""Which engine a problem's steps run on (cpdlp_problem_engine), where the choice
+follows from the LP's sizes and row lengths alone."""
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _layout(handle, lp, **fields):
+    from coolpdlp import native, _abi as A
+    prm = A.default_params_py(A.ALGO_PDLP)
+    for k, v in fields.items():
+        setattr(prm, k, v)
+    S = native.LPStruct(lp.m, lp.n, lp.colptr, lp.rowval, lp.nzval, lp.c, lp.lv, lp.uv, lp.lc, lp.uc)
+    lay = native.Problem(handle, S, prm).layout()
+    assert lay["A"]["resident_ctas"] == lay["At"]["resident_ctas"]
+    return lay["A"]["engine"], lay["At"]["engine"], lay["A"]["resident_ctas"]
+
+
+@pytest.mark.parametrize("name,float_type,want", [
+    ("200x400x5", "F64", ("resident", "resident", 4)), ("100x200x5", "F64", ("resident", "resident", 1)),
+    ("200x400x5", "F32", ("resident", "resident", 1)), ("1000x2000x5", "F32", ("resident", "resident", 8)),
+    ("20000x40000x5", "F64", ("slices", "slices", 0)), ("20000x40000x5", "F32", ("slices", "slices", 0))])
+def test_engine_by_size(handle, name, float_type, want):
+    from coolpdlp import generators as G, _abi as A
+    m, n, k = (int(v) for v in name.split("x"))
+    assert _layout(handle, G.random_sparse_lp(m, n, k, seed=1), float_type=getattr(A, f"VAL_{float_type}")) == want
+
+
+def test_engine_by_request(handle):
+    from coolpdlp import generators as G, _abi as A
+    lp = G.random_sparse_lp(1000, 2000, 5, seed=1)
+    assert _layout(handle, lp, matrix_type=A.FMT_ELL) == ("ell", "ell", 0)
+    assert _layout(handle, lp, tile_nnz=128) == ("tiles", "tiles", 0)
