@@ -1286,8 +1286,13 @@ double spectral_norm_T(Handle& h, ProblemT<V>& P, const cpdlp_params* prm, int64
     // launches of GROUP: a launch, an event and its wait cost the host more than
     // the three kernels of a medium LP's iteration take (FP64: solve of a flow LP of
     // 63,000 nonzeros 15.5 -> 14.4 ms; power method and setup of a random LP of
-    // 1M nonzeros 7.9 -> 3.1 ms).
+    // 1M nonzeros 7.9 -> 3.1 ms).  Iterations longer than LONG_ITERATION seconds stay
+    // single, and no more than KEEP_BUSY seconds of them are queued ahead: what is
+    // queued beyond the last one runs for nothing (power-law LP of 14M nonzeros, FP32
+    // iterates, 60 iterations of 0.5 ms: state set-up 41.8 -> 32.2 ms; 4M nonzeros,
+    // 11 iterations: 3.3 -> 1.4 ms).
     constexpr int RING = 64, LAUNCHES = 16, SINGLES = 8, GROUP = 8;
+    constexpr double LONG_ITERATION = 25e-6, KEEP_BUSY = 100e-6;
     void* block = h.host_get(sizeof(PowerSlot) * RING);
     PowerSlot* ring = static_cast<PowerSlot*>(block);
     PowerSlot* dring = nullptr;
@@ -1347,9 +1352,10 @@ double spectral_norm_T(Handle& h, ProblemT<V>& P, const cpdlp_params* prm, int64
     double theta_d = 0.0;
     int64_t launched = 0, it = 0, ahead = 2, queued = 0, read = 0;
     int64_t ends[LAUNCHES];
+    double first_read = 0.0, each = 0.0;  // seconds an iteration
     for (bool stop = false; !stop;) {
         while (launched - it < ahead && launched <= maxiter) {
-            const bool many = launched >= SINGLES;
+            const bool many = launched >= SINGLES && each <= LONG_ITERATION;
             cudaGraphExec_t& exec = cleanup.exec[many];
             if (!exec) capture(many ? GROUP : 1, exec);
             CK(cudaGraphLaunch(exec, s));
@@ -1365,8 +1371,13 @@ double spectral_norm_T(Handle& h, ProblemT<V>& P, const cpdlp_params* prm, int64
             theta_d = slot.theta;
             stop = it > maxiter || slot.residual <= tol || slot.residual <= rtol * slot.theta;
         }
+        const double now = now_seconds();
+        if (first_read == 0.0) first_read = now;
+        else each = (now - first_read) / (double)(it - 1);
         ahead = std::min<int64_t>(2 * ahead, launched < SINGLES ? SINGLES : 3 * GROUP);
-        if (now_seconds() >= deadline) break;
+        if (each > LONG_ITERATION)
+            ahead = std::max<int64_t>(2, std::min<int64_t>(SINGLES, (int64_t)(KEEP_BUSY / each)));
+        if (now >= deadline) break;
     }
     if (iters_out) *iters_out = it;
     return std::sqrt(theta_d);
