@@ -167,7 +167,7 @@ void build_engines(Matrix& M, const std::vector<int32_t>& hp, const DBuf<int32_t
     SellSide<T>& L = sell_of<T>(M);
     if (M.nnz > 0) {
         L.on = build_sell<T>(L, hp, ptr.p, idx.p, val.p, M.m, 32 * items, s) &&
-               (sizeof(T) == 8 || (double)L.long_nnz <= SELL_MAX_LONG_F32 * (double)M.nnz);
+               sell_suits(L, M.m, M.nnz, false);
         if (!L.on) L.release();
     }
 }

@@ -84,7 +84,10 @@ bool build_sell(SellSide<T>& S, const std::vector<int32_t>& hp, const int32_t* p
     int32_t slot = 0, id = 0;
     for (int64_t r = 0; r < rows; r++) {
         const int32_t n = hp[(size_t)r + 1] - hp[(size_t)r];
-        if (n <= LONG_ROW) continue;
+        if (n <= LONG_ROW) {
+            S.widest = std::max(S.widest, n);
+            continue;
+        }
         S.long_nnz += n;
         const int32_t np = (n + tile - 1) / tile;
         for (int32_t p = 0; p < np; p++) longs.push_back(make_int4((int32_t)r, -(p + 1), id, slot));

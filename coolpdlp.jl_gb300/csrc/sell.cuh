@@ -30,6 +30,17 @@ constexpr int SELL_WINDOW = 256;
 // autotuner: the share of the nonzeros in rows longer than LONG_ROW
 constexpr double SELL_MAX_PADDING = 1.5;
 constexpr double SELL_MAX_LONG_F32 = 0.05;
+// FP32: a lane walks its row, so a slice takes as long as its longest row has
+// entries, while tiles have a lane an entry.  With few rows that chain is the
+// kernel: slices take at most this many entries a row, or at least this many rows.
+// us a step (tiles, slices; m x m, L entries in every row and column): L = 24: m =
+// 500 5.2, 4.5; L = 32: 500 5.3, 5.4, 2,000 6.2, 5.5; L = 48: 2,000 6.2, 7.4, 8,000
+// 9.2, 9.1; L = 64: 2,000 6.7, 8.8, 8,000 10.8, 10.3, 16,000 16.9, 14.2.  Narrow
+// storage, which reads less: L = 24: 500 4.9, 4.7; L = 32: 2,000 5.9, 5.9, 500 5.1, 5.9;
+// L = 48: 8,000 8.4, 9.3, 16,000 14.2, 12.0.  (FP64: slices at all of them: L = 64:
+// 500 16.1, 14.7, 8,000 41.5, 17.1.)
+constexpr int SELL_F32_ENTRIES = 32, SELL_PM1_ENTRIES = 24;
+constexpr int64_t SELL_F32_ROWS = 16000;
 constexpr uint8_t SELL_SKIP = 255;  // no row, or a row that the long pieces take
 
 template <class T>
@@ -38,6 +49,7 @@ struct SellSide {
     int32_t nslices = 0, nltasks = 0, npieces = 0, tile = 512;
     int64_t entries = 0;          // with padding
     int64_t long_nnz = 0;         // nonzeros of the rows that the pieces take
+    int32_t widest = 0;           // entries of the longest row in a slice
     DBuf<int32_t> off;            // per slice, units of 32 entries
     DBuf<uint8_t> len;            // per slice row
     DBuf<int32_t> perm;           // slice row -> row; empty: the identity
@@ -75,6 +87,16 @@ struct SellView {
 template <class T>
 bool build_sell(SellSide<T>& S, const std::vector<int32_t>& hp, const int32_t* ptr,
                 const int32_t* idx, const T* val, int64_t rows, int tile, cudaStream_t s);
+
+// Whether the products of a side should run on its slices, from its row lengths
+// (without the autotuner; FP64: whenever build_sell keeps them)
+template <class T>
+bool sell_suits(const SellSide<T>& S, int64_t rows, int64_t nnz, bool narrow) {
+    if (sizeof(T) == 8) return true;
+    return (double)S.long_nnz <= SELL_MAX_LONG_F32 * (double)nnz &&
+           (S.widest <= (narrow ? SELL_PM1_ENTRIES : SELL_F32_ENTRIES) ||
+            rows >= SELL_F32_ROWS);
+}
 
 template <class V, class T>
 SellView<V, T> sell_view(const SellSide<V>& S, const int32_t* ptr, const int32_t* idx, const V* val,

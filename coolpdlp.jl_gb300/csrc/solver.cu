@@ -1095,7 +1095,7 @@ ProblemBase* make_problem(Handle& h, const cpdlp_lp* lp, const cpdlp_params* prm
     // below the autotuner's sizes, with the library's own choice of engine (no
     // ELL, no pinned tile size): a small LP with valued storage runs its blocks on
     // the resident kernels, others step on the sliced engine, where its padding
-    // is small and, in FP32, few entries are in long rows (us a step, tiles and
+    // is small and, in FP32, sell_suits allows it (us a step, tiles and
     // slices: FP64 flow 63,000 nonzeros 8.9, 5.5, random 1,000,000 42.7, 20.2,
     // power-law 240,000 with a quarter in long rows 17.1, 14.7; FP32 random
     // 1,000,000 15.7, 14.2, 200,000 9.3, 7.8, power-law 240,000 10.1, 10.9)
@@ -1107,7 +1107,7 @@ ProblemBase* make_problem(Handle& h, const cpdlp_lp* lp, const cpdlp_params* prm
                                  side == 0 ? P->a_idx.p : P->at_idx.p,
                                  pm1 ? nullptr : side == 0 ? P->a_val.p : P->at_val.p,
                                  side_rows(*P, side), 32 * (side == 0 ? items_A : items_At), s) &&
-                   (sizeof(T) == 8 || (double)S.long_nnz <= SELL_MAX_LONG_F32 * (double)nnz);
+                   sell_suits(S, side_rows(*P, side), nnz, pm1);
             if (!S.on) S.release();
         }
     }

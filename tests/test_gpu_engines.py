@@ -1,5 +1,6 @@
 """Which engine a problem's steps run on (cpdlp_problem_engine), where the choice
 follows from the LP's sizes and row lengths alone."""
+import numpy as np
 import pytest
 
 pytestmark = pytest.mark.gpu
@@ -31,3 +32,29 @@ def test_engine_by_request(handle):
     lp = G.random_sparse_lp(1000, 2000, 5, seed=1)
     assert _layout(handle, lp, matrix_type=A.FMT_ELL) == ("ell", "ell", 0)
     assert _layout(handle, lp, tile_nnz=128) == ("tiles", "tiles", 0)
+
+
+def _even_rows(m, per_row):
+    """m x m with `per_row` entries in every row and every column."""
+    from coolpdlp import generators as G
+    rng = np.random.RandomState(m + per_row)
+    shifts = np.append(0, 1 + rng.choice(m - 1, per_row - 1, False))
+    cols = (np.arange(m)[:, None] + shifts[None, :]) % m
+    rows = np.repeat(np.arange(m), per_row)
+    colptr, rowval, nzval = G.csc_from_triplets(m, m, rows, cols.ravel(), rng.randn(rows.size))
+    return G.LPData(m, m, colptr, rowval, nzval, rng.rand(m), np.zeros(m), np.full(m, 10.0),
+                    np.full(m, -np.inf), np.full(m, 5.0))
+
+
+@pytest.mark.parametrize("m,per_row,narrow,want", [
+    (5000, 32, False, "slices"), (5000, 33, False, "tiles"), (15999, 64, False, "tiles"),
+    (16000, 64, False, "slices"), (2000, 24, True, "slices"), (2000, 25, True, "tiles"),
+    (15999, 33, True, "tiles"), (16000, 33, True, "slices")])
+def test_fp32_rows_of_many_entries(handle, m, per_row, narrow, want):
+    """Slices need many rows where a row has many entries (FP32): the edges of
+    the rule."""
+    from coolpdlp import _abi as A
+    lp = _even_rows(m, per_row)
+    if narrow:
+        lp.nzval = np.sign(lp.nzval)
+    assert _layout(handle, lp, float_type=A.VAL_F32) == (want, want, 0)
