@@ -485,19 +485,43 @@ void build_ell(Handle& h, ProblemT<T>& P, int side, const std::vector<int32_t>& 
     }
 }
 
-// Autotuner of one matrix's product (side 0: rows of A, side 1: rows of A'):
-// the fused step kernel that uses the matrix (the primal step for A', the dual
-// step for A) runs on scratch vectors with CSR tiles and, where allowed, ELL,
-// timed with CUDA events on the handle's stream; ELL is kept when it is at
-// least 3% faster.  The engines sum a row of at most LONG_ROW entries in the
-// same order, so the choice does not change FP32 results; the tile size would
-// (it is also the piece size of long rows), so it follows from the size alone
+// Large matrices (AUTOTUNE_MIN_NNZ nonzeros) choose their engine per side (0: rows
+// of A, the dual step; 1: rows of A', the primal step).
+// FP32, and narrow storage: by timing.  The fused step kernel runs on scratch
+// vectors with CSR tiles, ELL and slices, timed with CUDA events on the handle's
+// stream; one that is not the engine before it is kept when it is at least 3%
+// faster.  The candidates sum every row in the same order with the same roundings
+// (ELL is one only where no row is longer than LONG_ROW, which tiles and slices
+// cut into pieces alike), so the choice does not change the iterates.  The tile
+// size would (it is also the piece size), so it follows from the size alone
 // (wave_items).  Decisions are cached per matrix shape and requested format for
 // the process.  With ELL chosen the slabs stay in P.
+// FP64: by the row lengths (ell_f64), because slices and ELL fuse each product
+// into the sum and tiles do not.  The power method, in FP64 for either type, follows
+// the row lengths too (spectral_norm_T).
+// The density order, which does change the order of the sums, is timed for both
+// types.
 constexpr int64_t AUTOTUNE_MIN_NNZ = 1 << 21;
 constexpr int FMT_SELL = -1;  // the tuner's name for the sliced engine (internal)
 // ELL is a candidate when its slabs hold at most this many times the nonzeros
 constexpr int64_t ELL_MAX_PADDING = 3;
+
+// FP64 with the library's own choice of format: ELL, else slices where build_sell
+// keeps them, else tiles.  ELL (which fits, so slices are padded less) only where many
+// entries are in rows of just over LONG_ROW: slices give such a row a warp to itself,
+// a quarter to a half of whose lanes are masked (us a step, ELL and slices: 40,000
+// x 40,000, 64 entries a row and about 64 a column 38.3, 45.9; 22,000 rows of 100 37.1,
+// 43.9), until the one thread a row has too long a chain (20,000 rows of 200 90.3,
+// 61.5).  Rows of at most LONG_ROW: no difference (37 to 118 us a step, within 5%).
+bool ell_f64(const std::vector<int32_t>& hp, int64_t rows) {
+    int64_t widest = 0, in_long = 0;
+    for (int64_t r = 0; r < rows; r++) {
+        const int64_t len = hp[(size_t)r + 1] - hp[(size_t)r];
+        widest = std::max(widest, len);
+        if (len > LONG_ROW) in_long += len;
+    }
+    return widest > LONG_ROW && widest <= 2 * LONG_ROW && 20 * in_long > hp[(size_t)rows];
+}
 
 // Nonzeros per lane of a large matrix's tiles.  Four blocks of eight 512-nonzero
 // tiles are resident on an SM; between 0.95 and 1.39 such waves the last one is
@@ -508,134 +532,96 @@ int wave_items(int64_t nnz, int items, int num_sms) {
     return items == 16 && waves > 0.95 && waves < 1.39 ? 8 : items;
 }
 
-struct SideChoice {
-    int fmt;
-    int items;
-};
-
-template <class T, class Launch>
-SideChoice tune_side(Handle& h, ProblemT<T>& P, int side, const std::vector<int32_t>& hp,
-                     int heuristic, bool try_csr, bool try_ell, int which, Launch&& launch) {
-    if (!try_ell) return SideChoice{CPDLP_FMT_CSR, heuristic};
-    static std::mutex mu;
-    static std::map<std::tuple<int64_t, int64_t, int64_t, int, int, int, int>, SideChoice> cache;
-    const int64_t rows = side_rows(P, side), cols = side_rows(P, 1 - side);
-    const auto key = std::make_tuple(rows, cols, P.nnz, (int)sizeof(T), h.device, which,
-                                     (int)try_csr * 2 + (int)try_ell);
-    {
-        std::lock_guard<std::mutex> lock(mu);
-        auto it = cache.find(key);
-        if (it != cache.end()) {
-            if (it->second.fmt == CPDLP_FMT_ELL) {
-                build_ell(h, P, side, hp);
-                P.fmt[side] = CPDLP_FMT_ELL;
-            }
-            return it->second;
-        }
-    }
-    cudaStream_t s = h.stream;
-    cudaEvent_t e0, e1;
-    CK(cudaEventCreate(&e0));
-    CK(cudaEventCreate(&e1));
-    SideChoice best{try_csr ? CPDLP_FMT_CSR : CPDLP_FMT_ELL, heuristic};
-    float best_ms = INFINITY;
-    auto timed = [&](int fmt, TilePlan& pl, T* part) {
-        launch(fmt, pl, part);
-        CK(cudaEventRecord(e0, s));
-        for (int r = 0; r < 4; r++) launch(fmt, pl, part);
-        CK(cudaEventRecord(e1, s));
-        CK(cudaEventSynchronize(e1));
-        float ms = 0.f;
-        CK(cudaEventElapsedTime(&ms, e0, e1));
-        return ms;
-    };
-    try {
-        if (try_csr) {
-            TilePlan plan;
-            build_tile_plan(hp, (int32_t)rows, heuristic, plan, s);
-            DBuf<T> part((size_t)std::max(plan.npieces, 1));
-            best_ms = timed(CPDLP_FMT_CSR, plan, part.p);
-        }
-        if (try_ell) {
-            build_ell(h, P, side, hp);
-            P.fmt[side] = CPDLP_FMT_ELL;
-            TilePlan none;
-            const float ms = timed(CPDLP_FMT_ELL, none, nullptr);
-            if (!try_csr || ms < 0.97f * best_ms) {
-                best_ms = ms;
-                best = SideChoice{CPDLP_FMT_ELL, heuristic};
-            } else {
-                P.fmt[side] = CPDLP_FMT_CSR;
-                P.ell_idx[side] = DBuf<int32_t>();
-                P.ell_val[side] = DBuf<T>();
-                P.ell_width[side] = 0;
-            }
-        }
-    } catch (...) {
-        cudaEventDestroy(e0);
-        cudaEventDestroy(e1);
-        throw;
-    }
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
-    std::lock_guard<std::mutex> lock(mu);
-    cache[key] = best;
-    return best;
+// ms of a launch, after one that is not timed
+template <class F>
+float time_step(Handle& h, F&& launch) {
+    struct Events {
+        cudaEvent_t e[2] = {};
+        ~Events() { for (cudaEvent_t x : e) if (x) cudaEventDestroy(x); }
+    } ev;
+    for (cudaEvent_t& e : ev.e) CK(cudaEventCreate(&e));
+    launch();
+    CK(cudaEventRecord(ev.e[0], h.stream));
+    for (int r = 0; r < 4; r++) launch();
+    CK(cudaEventRecord(ev.e[1], h.stream));
+    CK(cudaEventSynchronize(ev.e[1]));
+    float ms = 0.f;
+    CK(cudaEventElapsedTime(&ms, ev.e[0], ev.e[1]));
+    return ms / 4;
 }
 
-// The sliced engine against the tile plan the autotuner chose for this side:
-// kept when its step kernel is 3% faster; decided once per matrix shape.
+// ELL against tiles on one side; true, and the slabs in P, when ELL is kept
 template <class T, class Launch>
-void tune_sell(Handle& h, ProblemT<T>& P, int side, const std::vector<int32_t>& hp, int items,
-               Launch&& launch) {
-    if (P.fmt[side] != CPDLP_FMT_CSR) return;
+bool tune_ell(Handle& h, ProblemT<T>& P, int side, const std::vector<int32_t>& hp, int items,
+              Launch&& launch) {
     static std::mutex mu;
-    static std::map<std::tuple<int64_t, int64_t, int64_t, int, int, int, int, bool>, bool> cache;
+    static std::map<std::tuple<int64_t, int64_t, int64_t, int, int, bool, int>, bool> cache;
     const int64_t rows = side_rows(P, side), cols = side_rows(P, 1 - side);
-    const auto key = std::make_tuple(rows, cols, P.nnz, (int)sizeof(T), h.device, side, items, P.ordered);
+    const auto key = std::make_tuple(rows, cols, P.nnz, (int)sizeof(T), h.device, P.pm1, side);
     int decided = -1;
     {
         std::lock_guard<std::mutex> lock(mu);
         auto it = cache.find(key);
         if (it != cache.end()) decided = it->second ? 1 : 0;
     }
-    if (decided == 0) return;
-    cudaStream_t s = h.stream;
-    SellSide<T>& S = P.sell[side];
-    bool keep = build_sell<T>(S, hp, side == 0 ? P.a_ptr.p : P.at_ptr.p,
-                              side == 0 ? P.a_idx.p : P.at_idx.p,
-                              side == 0 ? P.a_val.p : P.at_val.p, rows, 32 * items, s);
-    if (decided < 0 && keep) {
-        struct Events {
-            cudaEvent_t e[2] = {};
-            ~Events() { for (cudaEvent_t x : e) if (x) cudaEventDestroy(x); }
-        } ev;
-        for (cudaEvent_t& e : ev.e) CK(cudaEventCreate(&e));
-        TilePlan plan;
-        build_tile_plan(hp, (int32_t)rows, items, plan, s);
-        DBuf<T> part((size_t)std::max(plan.npieces, 1));
-        auto timed = [&](int fmt) {
-            launch(fmt, plan, part.p);
-            CK(cudaEventRecord(ev.e[0], s));
-            for (int r = 0; r < 4; r++) launch(fmt, plan, part.p);
-            CK(cudaEventRecord(ev.e[1], s));
-            CK(cudaEventSynchronize(ev.e[1]));
-            float ms = 0.f;
-            CK(cudaEventElapsedTime(&ms, ev.e[0], ev.e[1]));
-            return ms;
-        };
-        const float tiles = timed(CPDLP_FMT_CSR), slices = timed(FMT_SELL);
-        keep = slices < 0.97f * tiles;
-        if (trace_level() > 0)
-            fprintf(stderr, "[cpdlp setup]   side %d: tiles %.4f ms, slices %.4f ms (%.3f entries a nonzero)\n",
-                    side, tiles / 4, slices / 4, (double)S.entries / (double)std::max<int64_t>(P.nnz, 1));
-    }
+    if (decided == 0) return false;
+    build_ell(h, P, side, hp);
+    bool keep = true;
     if (decided < 0) {
+        TilePlan plan, none;
+        build_tile_plan(hp, (int32_t)rows, items, plan, h.stream);
+        DBuf<T> part((size_t)std::max(plan.npieces, 1));
+        const float tiles = time_step(h, [&] { launch(CPDLP_FMT_CSR, plan, part.p); }),
+                    ell = time_step(h, [&] { launch(CPDLP_FMT_ELL, none, (T*)nullptr); });
+        keep = ell < 0.97f * tiles;
         std::lock_guard<std::mutex> lock(mu);
         cache[key] = keep;
     }
-    S.on = keep;
-    if (!keep) S.release();
+    if (keep) {
+        P.fmt[side] = CPDLP_FMT_ELL;
+    } else {
+        P.ell_idx[side] = DBuf<int32_t>();
+        P.ell_val[side] = DBuf<T>();
+        P.ell_width[side] = 0;
+    }
+    return keep;
+}
+
+// Slices against the engine chosen so far; decided once per matrix shape.  They stay
+// where they are built: the power method takes them whatever the steps run on.
+template <class T, class Launch>
+void tune_sell(Handle& h, ProblemT<T>& P, int side, const std::vector<int32_t>& hp, int items,
+               Launch&& launch) {
+    static std::mutex mu;
+    static std::map<std::tuple<int64_t, int64_t, int64_t, int, int, int, int, bool>, bool> cache;
+    const int64_t rows = side_rows(P, side), cols = side_rows(P, 1 - side);
+    const bool ell = P.fmt[side] == CPDLP_FMT_ELL;
+    const auto key = std::make_tuple(rows, cols, P.nnz, (int)sizeof(T), h.device, side,
+                                     ell ? 0 : items, P.ordered);
+    SellSide<T>& S = P.sell[side];
+    if (!build_sell<T>(S, hp, side == 0 ? P.a_ptr.p : P.at_ptr.p, side == 0 ? P.a_idx.p : P.at_idx.p,
+                       side == 0 ? P.a_val.p : P.at_val.p, rows, 32 * items, h.stream))
+        return;
+    {
+        std::lock_guard<std::mutex> lock(mu);
+        auto it = cache.find(key);
+        if (it != cache.end()) {
+            S.on = it->second;
+            return;
+        }
+    }
+    TilePlan plan;
+    if (!ell) build_tile_plan(hp, (int32_t)rows, items, plan, h.stream);
+    DBuf<T> part((size_t)std::max(plan.npieces, 1));
+    const float before = time_step(h, [&] { launch(P.fmt[side], plan, part.p); }),
+                slices = time_step(h, [&] { launch(FMT_SELL, plan, part.p); });
+    S.on = slices < 0.97f * before;
+    if (trace_level() > 0)
+        fprintf(stderr, "[cpdlp setup]   side %d: %s %.4f ms, slices %.4f ms (%.3f entries a nonzero)\n",
+                side, ell ? "ELL" : "tiles", before, slices,
+                (double)S.entries / (double)std::max<int64_t>(P.nnz, 1));
+    std::lock_guard<std::mutex> lock(mu);
+    cache[key] = S.on;
 }
 
 // device reduction of (rows x q) partials into host doubles
@@ -955,10 +941,13 @@ ProblemBase* make_problem(Handle& h, const cpdlp_lp* lp, const cpdlp_params* prm
         hp2 = std::move(o.hp2);
         hp1 = std::move(o.hp1);
     }
-    auto ell_fits = [&](const std::vector<int32_t>& hp, int64_t rows) {
+    auto widest_row = [](const std::vector<int32_t>& hp) {
         int64_t w = 0;
-        for (int64_t r = 0; r < rows; r++) w = std::max<int64_t>(w, hp[r + 1] - hp[r]);
-        return rows * w <= ELL_MAX_PADDING * std::max<int64_t>(nnz, 1);
+        for (size_t r = 0; r + 1 < hp.size(); r++) w = std::max<int64_t>(w, hp[r + 1] - hp[r]);
+        return w;
+    };
+    auto ell_fits = [&](const std::vector<int32_t>& hp, int64_t rows) {
+        return rows * widest_row(hp) <= ELL_MAX_PADDING * std::max<int64_t>(nnz, 1);
     };
     const bool tune = mt == CPDLP_FMT_AUTO ? nnz >= AUTOTUNE_MIN_NNZ
                                            : (mt != CPDLP_FMT_ELL && prm->tile_nnz == 0 &&
@@ -968,7 +957,8 @@ ProblemBase* make_problem(Handle& h, const cpdlp_lp* lp, const cpdlp_params* prm
         build_ell(h, *P, 1, hp1);
         P->fmt[0] = P->fmt[1] = CPDLP_FMT_ELL;
     } else if (tune) {
-        const bool try_csr = true;
+        const bool f64 = sizeof(T) == 8;
+        P->timed = !f64;
         const bool ell_A = mt == CPDLP_FMT_AUTO && ell_fits(hp2, m);
         const bool ell_At = mt == CPDLP_FMT_AUTO && ell_fits(hp1, n);
         // scratch iterates (zeros) for the fused step kernels being timed
@@ -1015,17 +1005,24 @@ ProblemBase* make_problem(Handle& h, const cpdlp_lp* lp, const cpdlp_params* prm
                 else launch_tiles<1>(pl, V, VecSet<T, 1>{{vxb.p}}, de, s);
             }
         };
-        const SideChoice cAt = tune_side<T>(h, *P, 1, hp1, items_At, try_csr, ell_At, pm1 ? 3 : 1,
-                                            launch_At);
-        const SideChoice cA = tune_side<T>(h, *P, 0, hp2, items_A, try_csr, ell_A, pm1 ? 2 : 0,
-                                           launch_A);
-        items_A = cA.items;
-        items_At = cAt.items;
+        for (int side = 1; side >= 0; side--) {
+            const std::vector<int32_t>& hp = side == 0 ? hp2 : hp1;
+            if (!(side == 0 ? ell_A : ell_At)) continue;
+            if (f64) {
+                if (!ell_f64(hp, side_rows(*P, side))) continue;
+                build_ell(h, *P, side, hp);
+                P->fmt[side] = CPDLP_FMT_ELL;
+            } else if (widest_row(hp) <= LONG_ROW) {
+                if (side == 0) tune_ell<T>(h, *P, 0, hp, items_A, launch_A);
+                else tune_ell<T>(h, *P, 1, hp, items_At, launch_At);
+            }
+        }
         // density order as a candidate (CSR on both matrices): both step
         // kernels timed in each order, the density order kept when it is at
         // least 3% faster; decided once per matrix shape for the process
+        // (FP64 rows even enough for ELL are so for slices in any order)
         if (mt == CPDLP_FMT_AUTO && !order_on && !order_off && P->fmt[0] == CPDLP_FMT_CSR &&
-            P->fmt[1] == CPDLP_FMT_CSR) {
+            P->fmt[1] == CPDLP_FMT_CSR && !(f64 && ell_A && ell_At)) {
             static std::mutex mu;
             static std::map<std::tuple<int64_t, int64_t, int64_t, int, int, int>, bool> cache;
             const auto key = std::make_tuple(m, n, nnz, (int)sizeof(T), h.device, (int)pm1);
@@ -1085,10 +1082,19 @@ ProblemBase* make_problem(Handle& h, const cpdlp_lp* lp, const cpdlp_params* prm
             cudaEventDestroy(e0);
             cudaEventDestroy(e1);
         }
-        // the sliced engine as a candidate on each side that stayed with CSR
-        if (!pm1) {
-            tune_sell<T>(h, *P, 1, hp1, items_At, launch_At);
-            tune_sell<T>(h, *P, 0, hp2, items_A, launch_A);
+        // slices (narrow storage stays with ELL or tiles)
+        for (int side = 1; side >= 0 && !pm1; side--) {
+            const std::vector<int32_t>& hp = side == 0 ? hp2 : hp1;
+            if (!f64) {
+                if (side == 0) tune_sell<T>(h, *P, 0, hp, items_A, launch_A);
+                else tune_sell<T>(h, *P, 1, hp, items_At, launch_At);
+            } else if (P->fmt[side] == CPDLP_FMT_CSR) {
+                SellSide<T>& S = P->sell[side];
+                S.on = build_sell<T>(S, hp, side == 0 ? P->a_ptr.p : P->at_ptr.p,
+                                     side == 0 ? P->a_idx.p : P->at_idx.p,
+                                     side == 0 ? P->a_val.p : P->at_val.p, side_rows(*P, side),
+                                     32 * (side == 0 ? items_A : items_At), s);
+            }
         }
     }
     mark("formats, autotuner, density order");
@@ -1225,9 +1231,17 @@ double spectral_norm_T(Handle& h, ProblemT<V>& P, const cpdlp_params* prm, int64
     DBuf<double> scal(4);
     DBuf<int> d_it(1);
     // the second product's partials: its blocks', then its long rows'
-    const bool sell = !P.pm1 && P.sell[1].on;
-    const int64_t blocks = sell ? sell_blocks(P.sell[1]) : side_blocks(P, 1, TILE_WARPS),
-                  rows = sell ? blocks + (int64_t)P.sell[1].counters.n : side_partials(P, 1, TILE_WARPS);
+    // its engine, where that of the steps is chosen by timing: slices where they are
+    // held, else tiles, so that theta, and the step size with it, does not depend on
+    // the timing
+    auto on_slices = [&](int side) {
+        return !P.pm1 && (P.sell[side].on || (P.timed && P.sell[side].nslices > 0));
+    };
+    const bool sell0 = on_slices(0), sell = on_slices(1);
+    const int64_t plain = P.timed ? tiles_grid(P.planAt, TILE_WARPS) : side_blocks(P, 1, TILE_WARPS);
+    const int64_t blocks = sell ? sell_blocks(P.sell[1]) : plain,
+                  rows = sell ? blocks + (int64_t)P.sell[1].counters.n
+                       : P.timed ? plain + P.planAt.nlong : side_partials(P, 1, TILE_WARPS);
     DBuf<double> part((size_t)std::max<int64_t>(rows, 1) * 2);
     DBuf<unsigned> tickets(2);
     CK(cudaMemsetAsync(part.p, 0, part.bytes(), s));  // (a side without long rows has one unused counter)
@@ -1315,17 +1329,20 @@ double spectral_norm_T(Handle& h, ProblemT<V>& P, const cpdlp_params* prm, int64
     auto iteration = [&] {
         double* const blk = part.p;
         double* const lng = part.p + (size_t)blocks * 2;
+        auto product = [&](int side, const auto& view, const double* in, const auto& epi) {
+            if (P.timed) launch_tiles_w<TILE_WARPS>(side == 0 ? P.planA : P.planAt, view, VecSet<double, 1>{{in}}, epi, s);
+            else launch_side(P, side, view, VecSet<double, 1>{{in}}, epi, s);
+        };
         if (P.pm1) {
-            launch_side(P, 0, A1, VecSet<double, 1>{{xs.p}}, ScaledStoreEpi<double>{sv.p, P.D1.p}, s);
-            PowerEpi<double, true> pe{x.p, Ax.p, blk, lng, P.D2.p, tickets.p, scal.p, rows};
-            launch_side(P, 1, At1, VecSet<double, 1>{{sv.p}}, pe, s);
+            product(0, A1, xs.p, ScaledStoreEpi<double>{sv.p, P.D1.p});
+            product(1, At1, sv.p, PowerEpi<double, true>{x.p, Ax.p, blk, lng, P.D2.p, tickets.p, scal.p, rows});
         } else {
             const PowerEpi<double> pe{x.p, Ax.p, blk, lng, nullptr, tickets.p, scal.p, rows};
             const StoreEpi<double> se{sv.p};
-            if (P.sell[0].on) launch_sell(sell_view(P.sell[0], P.a_ptr.p, P.a_idx.p, P.a_val.p, pA.p), (const double*)x.p, se, s);
-            else launch_side(P, 0, A, VecSet<double, 1>{{x.p}}, se, s);
+            if (sell0) launch_sell(sell_view(P.sell[0], P.a_ptr.p, P.a_idx.p, P.a_val.p, pA.p), (const double*)x.p, se, s);
+            else product(0, A, x.p, se);
             if (sell) launch_sell(sell_view(P.sell[1], P.at_ptr.p, P.at_idx.p, P.at_val.p, pAt.p), (const double*)sv.p, pe, s);
-            else launch_side(P, 1, At, VecSet<double, 1>{{sv.p}}, pe, s);
+            else product(1, At, sv.p, pe);
         }
         launch_chained(k_power_residual, gr, (unsigned)RED_THREADS, s, x.p, (const double*)Ax.p,
                        (const double*)scal.p, n, P.red_rows.p, (const double*)(P.pm1 ? P.D2.p : nullptr),

@@ -49,6 +49,7 @@ struct ProblemBase {
     // ProblemT::ell_val; the CSR row pointer gives the row lengths)
     int32_t fmt[2] = {CPDLP_FMT_CSR, CPDLP_FMT_CSR};
     int64_t ell_width[2] = {0, 0};
+    bool timed = false;           // the steps' engines were chosen by timing
     DBuf<int32_t> ell_idx[2];
     DBuf<double> D1, D2, invD1, invD2;
     double primal_scale = 0, dual_scale = 0;

@@ -58,3 +58,44 @@ def test_fp32_rows_of_many_entries(handle, m, per_row, narrow, want):
     if narrow:
         lp.nzval = np.sign(lp.nzval)
     assert _layout(handle, lp, float_type=A.VAL_F32) == (want, want, 0)
+
+
+@pytest.mark.parametrize("m,per_row,want", [(40000, 55, "slices"), (22000, 100, "ell"), (10500, 200, "slices")])
+def test_fp64_of_large_lps_by_row_length(handle, m, per_row, want):
+    """From 2^21 nonzeros FP64 engines follow the row lengths, not a timing run
+    (their roundings differ): the iterates are those of the tiles to rounding."""
+    from coolpdlp import native, _abi as A
+    lp = _even_rows(m, per_row)
+    assert lp.nzval.size >= 1 << 21
+    assert _layout(handle, lp) == (want, want, 0)
+    S = native.LPStruct(lp.m, lp.n, lp.colptr, lp.rowval, lp.nzval, lp.c, lp.lv, lp.uv, lp.lc, lp.uc)
+    got = []
+    for tile in (0, 512):
+        prm = A.default_params_py(A.ALGO_PDLP)
+        prm.power_maxiter_override = 20
+        prm.tile_nnz = tile
+        if tile:
+            prm.matrix_type = A.FMT_CSR
+        st = native.State(native.Problem(handle, S, prm), prm)
+        st.step(20)
+        got.append(st.vectors(A.VEC_SOL))
+    for a, b in zip(*got):
+        assert np.max(np.abs(a - b)) <= 1e-9 * max(1.0, np.max(np.abs(b)))
+
+
+def test_power_method_does_not_follow_the_timing(handle):
+    """A large LP with +-1 storage steps on ELL or tiles, whichever was faster
+    when timed; its |A| is that of the tiles, bit for bit, either way."""
+    from coolpdlp import generators as G, native, _abi as A
+    lp = G.multicommodity_flow_lp(side=128, K=12, seed=2)
+    assert lp.nzval.size >= 1 << 21
+    S = native.LPStruct(lp.m, lp.n, lp.colptr, lp.rowval, lp.nzval, lp.c, lp.lv, lp.uv, lp.lc, lp.uc)
+    norms = []
+    for tile in (0, 512):
+        prm = A.default_params_py(A.ALGO_PDLP)
+        prm.float_type = A.VAL_F32
+        prm.tile_nnz = tile
+        if tile:
+            prm.matrix_type = A.FMT_CSR
+        norms.append(native.Problem(handle, S, prm).spectral_norm(prm))
+    assert norms[0] == norms[1]
