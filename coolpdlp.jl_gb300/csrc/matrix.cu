@@ -155,21 +155,22 @@ DBuf<double>& csr_vals<double>(Matrix& M) { return M.format == CPDLP_FMT_COO ? M
 template <>
 DBuf<float>& csr_vals<float>(Matrix& M) { return M.format == CPDLP_FMT_COO ? M.cf : M.vf; }
 
-// the product's engines over a CSR on the device (hp: its row pointer)
+// the product's engine over a CSR on the device (hp: its row pointer)
 template <class T>
-void build_engines(Matrix& M, const std::vector<int32_t>& hp, const DBuf<int32_t>& ptr,
+void build_engine(Matrix& M, const std::vector<int32_t>& hp, const DBuf<int32_t>& ptr,
                    const DBuf<int32_t>& idx, const DBuf<T>& val, cudaStream_t s) {
     const int items = choose_items(M.nnz, M.m, 0);
+    // slices by the rule of the solver's steps, else tiles.  It holds for the
+    // product by itself too (us a call, 14 of them the call's; tiles and slices): FP32
+    // power-law, a quarter of the entries in long rows, 0.25M nonzeros 17.5, 18.5, 3.1M
+    // 32.5, 31.7, 6.2M 42.7, 43.8, 12.4M 68.5, 71.0; FP32 64 entries in every row, 2,000
+    // rows 15.5, 16.8, 32,000 27.9, 21.5; FP64 power-law 0.24M 20.8, 22.6, 3.1M 69.3, 46.5,
+    // 12.4M 192, 111.
+    SellSide<T>& L = sell_of<T>(M);
+    L.on = M.nnz > 0 && build_sell<T>(L, hp, ptr.p, idx.p, val.p, M.m, 32 * items, false, s);
+    if (L.on) return;
     build_tile_plan(hp, (int32_t)M.m, items, M.plan, s);
     M.part.alloc((size_t)(M.plan.npieces > 0 ? M.plan.npieces : 1) * sizeof(double));
-    // the sliced engine by the rule of the solver's steps: little padding and, in
-    // FP32, few entries in long rows
-    SellSide<T>& L = sell_of<T>(M);
-    if (M.nnz > 0) {
-        L.on = build_sell<T>(L, hp, ptr.p, idx.p, val.p, M.m, 32 * items, s) &&
-               sell_suits(L, M.m, M.nnz, false);
-        if (!L.on) L.release();
-    }
 }
 
 template <class T>
@@ -189,7 +190,7 @@ void build_T(Handle& h, Matrix& M, CscPair& S) {
         M.ptr = std::move(S.ptr2);
         M.idx = std::move(S.idx2);
         vals_of<T>(M) = std::move(v2);
-        build_engines<T>(M, hp, M.ptr, M.idx, vals_of<T>(M), s);
+        build_engine<T>(M, hp, M.ptr, M.idx, vals_of<T>(M), s);
         return;
     }
     if (M.format == CPDLP_FMT_COO) {
@@ -204,7 +205,7 @@ void build_T(Handle& h, Matrix& M, CscPair& S) {
         M.cptr = std::move(S.ptr2);
         M.cidx = std::move(S.idx2);
         csr_vals<T>(M) = std::move(v2);
-        build_engines<T>(M, hp, M.cptr, M.cidx, csr_vals<T>(M), s);
+        build_engine<T>(M, hp, M.cptr, M.cidx, csr_vals<T>(M), s);
         CK(cudaStreamSynchronize(s));
         return;
     }

@@ -75,22 +75,34 @@ __global__ void k_sell_fill(const int32_t* __restrict__ ptr, const int32_t* __re
 
 template <class T>
 bool build_sell(SellSide<T>& S, const std::vector<int32_t>& hp, const int32_t* ptr,
-                const int32_t* idx, const T* val, int64_t rows, int tile, cudaStream_t s) {
+                const int32_t* idx, const T* val, int64_t rows, int tile, bool timed, cudaStream_t s) {
     S.release();
     S.tile = tile;
     if (rows <= 0) return true;
-    // rows longer than LONG_ROW
+    // what the row lengths say (a pass of its own: a matrix that does not suit, or
+    // has no long rows, is done with it)
+    const int32_t* const p = hp.data();
+    int64_t in_long = 0;
+    int32_t widest = 0;
+    for (int64_t r = 0; r < rows; r++) {
+        const int32_t n = p[r + 1] - p[r], own = n > LONG_ROW ? 0 : n;
+        in_long += n - own;
+        widest = std::max(widest, own);
+    }
+    S.long_nnz = in_long;
+    S.widest = widest;
+    if (!timed && !sell_suits(S, rows, p[rows], val == nullptr)) {
+        S.release();
+        return false;
+    }
+    // the pieces of the rows longer than LONG_ROW
     std::vector<int4> longs;
     int32_t slot = 0, id = 0;
-    for (int64_t r = 0; r < rows; r++) {
-        const int32_t n = hp[(size_t)r + 1] - hp[(size_t)r];
-        if (n <= LONG_ROW) {
-            S.widest = std::max(S.widest, n);
-            continue;
-        }
-        S.long_nnz += n;
+    for (int64_t r = 0; r < rows && in_long > 0; r++) {
+        const int32_t n = p[r + 1] - p[r];
+        if (n <= LONG_ROW) continue;
         const int32_t np = (n + tile - 1) / tile;
-        for (int32_t p = 0; p < np; p++) longs.push_back(make_int4((int32_t)r, -(p + 1), id, slot));
+        for (int32_t q = 0; q < np; q++) longs.push_back(make_int4((int32_t)r, -(q + 1), id, slot));
         id++;
         if (np > 1) slot += np;
     }
@@ -155,8 +167,8 @@ bool build_sell(SellSide<T>& S, const std::vector<int32_t>& hp, const int32_t* p
     return true;
 }
 template bool build_sell<float>(SellSide<float>&, const std::vector<int32_t>&, const int32_t*,
-                                const int32_t*, const float*, int64_t, int, cudaStream_t);
+                                const int32_t*, const float*, int64_t, int, bool, cudaStream_t);
 template bool build_sell<double>(SellSide<double>&, const std::vector<int32_t>&, const int32_t*,
-                                 const int32_t*, const double*, int64_t, int, cudaStream_t);
+                                 const int32_t*, const double*, int64_t, int, bool, cudaStream_t);
 
 }  // namespace cpdlp

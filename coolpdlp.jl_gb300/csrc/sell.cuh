@@ -79,17 +79,8 @@ struct SellView {
     const V* __restrict__ cval;
 };
 
-// The slices of a CSR (device; hp: its row pointer on the host); tile: the
-// piece size of long rows; val null: narrow storage.  False, and nothing kept, when
-// they would hold more than SELL_MAX_PADDING times the nonzeros: that is seen
-// before they are allocated (a window with one row of 64 entries and 255 empty ones
-// pads 32 times).  Leaves S.on false.
-template <class T>
-bool build_sell(SellSide<T>& S, const std::vector<int32_t>& hp, const int32_t* ptr,
-                const int32_t* idx, const T* val, int64_t rows, int tile, cudaStream_t s);
-
 // Whether the products of a side should run on its slices, from its row lengths
-// (without the autotuner; FP64: whenever build_sell keeps them)
+// (long_nnz and widest; without the autotuner).  FP64: whenever build_sell keeps them.
 template <class T>
 bool sell_suits(const SellSide<T>& S, int64_t rows, int64_t nnz, bool narrow) {
     if (sizeof(T) == 8) return true;
@@ -97,6 +88,16 @@ bool sell_suits(const SellSide<T>& S, int64_t rows, int64_t nnz, bool narrow) {
            (S.widest <= (narrow ? SELL_PM1_ENTRIES : SELL_F32_ENTRIES) ||
             rows >= SELL_F32_ROWS);
 }
+
+// The slices of a CSR (device; hp: its row pointer on the host); tile: the
+// piece size of long rows; val null: narrow storage.  False, and nothing kept, when
+// they would hold more than SELL_MAX_PADDING times the nonzeros: that is seen
+// before they are allocated (a window with one row of 64 entries and 255 empty ones
+// pads 32 times).  The same, before any work on the device, where the row lengths
+// do not suit (unless `timed`: the autotuner decides).  Leaves S.on false.
+template <class T>
+bool build_sell(SellSide<T>& S, const std::vector<int32_t>& hp, const int32_t* ptr,
+                const int32_t* idx, const T* val, int64_t rows, int tile, bool timed, cudaStream_t s);
 
 template <class V, class T>
 SellView<V, T> sell_view(const SellSide<V>& S, const int32_t* ptr, const int32_t* idx, const V* val,

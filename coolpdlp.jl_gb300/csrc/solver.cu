@@ -600,7 +600,7 @@ void tune_sell(Handle& h, ProblemT<T>& P, int side, const std::vector<int32_t>& 
                                      ell ? 0 : items, P.ordered);
     SellSide<T>& S = P.sell[side];
     if (!build_sell<T>(S, hp, side == 0 ? P.a_ptr.p : P.at_ptr.p, side == 0 ? P.a_idx.p : P.at_idx.p,
-                       side == 0 ? P.a_val.p : P.at_val.p, rows, 32 * items, h.stream))
+                       side == 0 ? P.a_val.p : P.at_val.p, rows, 32 * items, true, h.stream))
         return;
     {
         std::lock_guard<std::mutex> lock(mu);
@@ -1093,7 +1093,7 @@ ProblemBase* make_problem(Handle& h, const cpdlp_lp* lp, const cpdlp_params* prm
                 S.on = build_sell<T>(S, hp, side == 0 ? P->a_ptr.p : P->at_ptr.p,
                                      side == 0 ? P->a_idx.p : P->at_idx.p,
                                      side == 0 ? P->a_val.p : P->at_val.p, side_rows(*P, side),
-                                     32 * (side == 0 ? items_A : items_At), s);
+                                     32 * (side == 0 ? items_A : items_At), false, s);
             }
         }
     }
@@ -1112,9 +1112,7 @@ ProblemBase* make_problem(Handle& h, const cpdlp_lp* lp, const cpdlp_params* prm
             S.on = build_sell<T>(S, side == 0 ? hp2 : hp1, side == 0 ? P->a_ptr.p : P->at_ptr.p,
                                  side == 0 ? P->a_idx.p : P->at_idx.p,
                                  pm1 ? nullptr : side == 0 ? P->a_val.p : P->at_val.p,
-                                 side_rows(*P, side), 32 * (side == 0 ? items_A : items_At), s) &&
-                   sell_suits(S, side_rows(*P, side), nnz, pm1);
-            if (!S.on) S.release();
+                                 side_rows(*P, side), 32 * (side == 0 ? items_A : items_At), false, s);
         }
     }
     // the CSR plans (also kept for an ELL side: the tuner and the exports use them),
