@@ -99,3 +99,35 @@ def test_power_method_does_not_follow_the_timing(handle):
             prm.matrix_type = A.FMT_CSR
         norms.append(native.Problem(handle, S, prm).spectral_norm(prm))
     assert norms[0] == norms[1]
+
+
+@pytest.mark.parametrize("narrow", [False, True])
+def test_fp32_slices_of_wide_rows_are_the_tile_engines_bits(handle, narrow):
+    """16,400 rows of 0 to 64 entries (and a few of 65 and 300) and as many columns
+    of about 30 on slices: the iterates have the tile engine's bits."""
+    from coolpdlp import generators as G, native, _abi as A
+    rng = np.random.RandomState(12)
+    m = 16400
+    lengths = np.arange(m) % 65
+    lengths[:40], lengths[40:44] = 65, 300
+    rows = np.repeat(np.arange(m), lengths)
+    cols = np.concatenate([(i * 97 + np.sort(rng.choice(m, k, False))) % m for i, k in enumerate(lengths)])
+    vals = rng.randn(rows.size)
+    colptr, rowval, nzval = G.csc_from_triplets(m, m, rows, cols, np.sign(vals) if narrow else vals)
+    lp = G.LPData(m, m, colptr, rowval, nzval, rng.rand(m), np.zeros(m), np.full(m, 10.0),
+                  np.full(m, -np.inf), np.full(m, 5.0))
+    S = native.LPStruct(lp.m, lp.n, lp.colptr, lp.rowval, lp.nzval, lp.c, lp.lv, lp.uv, lp.lc, lp.uc)
+    prm = A.default_params_py(A.ALGO_PDLP)
+    prm.float_type = A.VAL_F32
+    got = []
+    for tile in (0, 256):
+        prm.tile_nnz = tile
+        P = native.Problem(handle, S, prm)
+        lay = P.layout()
+        assert lay["A"]["engine"] == lay["At"]["engine"] == ("tiles" if tile else "slices")
+        assert lay["A"]["tile_nnz"] == lay["At"]["tile_nnz"] == 256
+        st = native.State(P, prm, np.linspace(0, 1, m), np.linspace(-1, 1, m))
+        st.step(30)
+        got.append([v for which in (A.VEC_SOL, A.VEC_SOL_AVG) for v in st.vectors(which)])
+    for a, b in zip(*got):
+        assert np.array_equal(a, b)
