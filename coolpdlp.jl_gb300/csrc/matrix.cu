@@ -207,6 +207,12 @@ void build_T(Handle& h, Matrix& M, CscPair& S) {
         csr_vals<T>(M) = std::move(v2);
         build_engine<T>(M, hp, M.cptr, M.cidx, csr_vals<T>(M), s);
         CK(cudaStreamSynchronize(s));
+        // (slices read the CSR in the pieces of long rows alone)
+        if (sell_of<T>(M).on && sell_of<T>(M).nltasks == 0) {
+            M.cptr.release();
+            M.cidx.release();
+            csr_vals<T>(M).release();
+        }
         return;
     }
     // ELL: width d = maximum(diff(rowptr)) (mat_ell.jl:57)

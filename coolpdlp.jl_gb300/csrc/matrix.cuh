@@ -12,9 +12,9 @@ namespace cpdlp {
 //  CSR: ptr = rowptr (m+1, 0-based), idx = colval (0-based), values; tile plan
 //  ELL: idx = colval (m*width, column-major, 1-based, 0 = padding), values
 //  COO: ptr = rowval (0-based), idx = colval (0-based), values, findnz order;
-//       mul! runs over a CSR copy (cptr, cidx, cd / cf)
+//       mul! runs over a CSR copy (cptr, cidx, cd / cf; kept where the engine reads it)
 // CSR and COO products run on the sliced engine where it holds the matrix well
-// (sell), else on the tile plan.
+// (sell), else on the tile plan: a matrix has one of the two.
 struct Matrix {
     Handle* h = nullptr;
     int32_t format = CPDLP_FMT_CSR;

@@ -59,6 +59,21 @@ def test_matrix_memory(handle, fmt):
     assert 0 < b <= 1.25 * a, (a, b)
 
 
+def test_coo_holds_no_csr_beside_its_slices(handle):
+    """Triplets and slices, where a CSR matrix holds the CSR and slices: a second
+    row index an entry in place of the row pointer."""
+    import coolpdlp as cp
+    pool = Pool()
+    S = _csc(True)
+    held = {}
+    for cls in (cp.GPUSparseMatrixCSR, cp.GPUSparseMatrixCOO):
+        before = pool.get(USED_NOW)
+        A = cls(S, np.float64)
+        held[cls] = pool.get(USED_NOW) - before
+        A.close()
+    assert held[cp.GPUSparseMatrixCOO] <= held[cp.GPUSparseMatrixCSR] + 4 * S.nnz + 4096
+
+
 def test_problem_memory(handle):
     from coolpdlp import native, _abi as A
     prm = A.default_params_py(A.ALGO_PDLP)
