@@ -91,7 +91,8 @@ bool build_sell(SellSide<T>& S, const std::vector<int32_t>& hp, const int32_t* p
     }
     S.long_nnz = in_long;
     S.widest = widest;
-    if (!timed && !sell_suits(S, rows, p[rows], val == nullptr)) {
+    S.suits = sell_suits(S, rows, p[rows], val == nullptr);
+    if (!timed && !S.suits) {
         S.release();
         return false;
     }

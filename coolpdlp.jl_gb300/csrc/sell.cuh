@@ -46,6 +46,7 @@ constexpr uint8_t SELL_SKIP = 255;  // no row, or a row that the long pieces tak
 template <class T>
 struct SellSide {
     bool on = false;
+    bool suits = false;           // sell_suits, of slices that are held
     int32_t nslices = 0, nltasks = 0, npieces = 0, tile = 512;
     int64_t entries = 0;          // with padding
     int64_t long_nnz = 0;         // nonzeros of the rows that the pieces take

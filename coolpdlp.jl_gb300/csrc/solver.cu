@@ -587,8 +587,9 @@ bool tune_ell(Handle& h, ProblemT<T>& P, int side, const std::vector<int32_t>& h
     return keep;
 }
 
-// Slices against the engine chosen so far; decided once per matrix shape.  They stay
-// where they are built: the power method takes them whatever the steps run on.
+// Slices against the engine chosen so far; decided once per matrix shape.  Where the
+// row lengths suit them (sell_suits) they stay whatever the steps run on: the power
+// method takes them.
 template <class T, class Launch>
 void tune_sell(Handle& h, ProblemT<T>& P, int side, const std::vector<int32_t>& hp, int items,
                Launch&& launch) {
@@ -598,17 +599,21 @@ void tune_sell(Handle& h, ProblemT<T>& P, int side, const std::vector<int32_t>& 
     const bool ell = P.fmt[side] == CPDLP_FMT_ELL;
     const auto key = std::make_tuple(rows, cols, P.nnz, (int)sizeof(T), h.device, side,
                                      ell ? 0 : items, P.ordered);
-    SellSide<T>& S = P.sell[side];
-    if (!build_sell<T>(S, hp, side == 0 ? P.a_ptr.p : P.at_ptr.p, side == 0 ? P.a_idx.p : P.at_idx.p,
-                       side == 0 ? P.a_val.p : P.at_val.p, rows, 32 * items, true, h.stream))
-        return;
+    int decided = -1;
     {
         std::lock_guard<std::mutex> lock(mu);
         auto it = cache.find(key);
-        if (it != cache.end()) {
-            S.on = it->second;
-            return;
-        }
+        if (it != cache.end()) decided = it->second ? 1 : 0;
+    }
+    SellSide<T>& S = P.sell[side];
+    const bool held = build_sell<T>(S, hp, side == 0 ? P.a_ptr.p : P.at_ptr.p,
+                                    side == 0 ? P.a_idx.p : P.at_idx.p,
+                                    side == 0 ? P.a_val.p : P.at_val.p, rows, 32 * items,
+                                    decided != 0, h.stream);
+    if (!held) return;
+    if (decided >= 0) {
+        S.on = decided == 1;
+        return;
     }
     TilePlan plan;
     if (!ell) build_tile_plan(hp, (int32_t)rows, items, plan, h.stream);
@@ -620,8 +625,11 @@ void tune_sell(Handle& h, ProblemT<T>& P, int side, const std::vector<int32_t>& 
         fprintf(stderr, "[cpdlp setup]   side %d: %s %.4f ms, slices %.4f ms (%.3f entries a nonzero)\n",
                 side, ell ? "ELL" : "tiles", before, slices,
                 (double)S.entries / (double)std::max<int64_t>(P.nnz, 1));
-    std::lock_guard<std::mutex> lock(mu);
-    cache[key] = S.on;
+    {
+        std::lock_guard<std::mutex> lock(mu);
+        cache[key] = S.on;
+    }
+    if (!S.on && !S.suits) S.release();
 }
 
 // device reduction of (rows x q) partials into host doubles
@@ -1229,11 +1237,11 @@ double spectral_norm_T(Handle& h, ProblemT<V>& P, const cpdlp_params* prm, int64
     DBuf<double> scal(4);
     DBuf<int> d_it(1);
     // the second product's partials: its blocks', then its long rows'
-    // its engine, where that of the steps is chosen by timing: slices where they are
-    // held, else tiles, so that theta, and the step size with it, does not depend on
-    // the timing
+    // its engine, where that of the steps is chosen by timing: slices where the row
+    // lengths suit them, else tiles, so that theta, and the step size with it, does
+    // not depend on the timing
     auto on_slices = [&](int side) {
-        return !P.pm1 && (P.sell[side].on || (P.timed && P.sell[side].nslices > 0));
+        return !P.pm1 && (P.timed ? P.sell[side].suits : P.sell[side].on);
     };
     const bool sell0 = on_slices(0), sell = on_slices(1);
     const int64_t plain = P.timed ? tiles_grid(P.planAt, TILE_WARPS) : side_blocks(P, 1, TILE_WARPS);
