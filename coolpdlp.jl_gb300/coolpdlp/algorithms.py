@@ -102,12 +102,12 @@ class Algorithm:
     name: "PDLP" or "PDHG"; T: np.float64 / np.float32 (iterate precision);
     Ti: index type (the device always uses int32 indices, so only its range is
     checked); M: the matrix type of the solve's products (conversion.jl:37-55):
-    "CSR" (the CSR engines: tiles, or slices where rows are short and even),
+    "CSR" (the CSR engines: tiles or slices, by the row lengths),
     "ELL" (the reference's ELL layout, one thread per row), "COO" (solved on
     the CSR engines: the reference's COO product sums with atomics in a
     run-dependent order), a GPUSparseMatrix* class, or None / "AUTO" (default):
-    for matrices of at least 2^21 nonzeros the autotuner picks per matrix among
-    CSR tiles, CSR slices and ELL."""
+    for matrices of at least 2^21 nonzeros ELL too, picked per matrix by timing
+    (Float32) or by the row lengths (Float64, whose engines round differently)."""
 
     KEYWORDS = ("chambolle_pock_alpha", "ruiz_iter", "invnorm_scaling", "primal_weight_damping",
                 "zero_tol", "sufficient_decay", "necessary_decay", "artificial_decay",

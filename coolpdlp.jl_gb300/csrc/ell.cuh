@@ -4,8 +4,9 @@
 //
 // Layout: idx / val are rows x width, column-major (entry k of row r at
 // r + k*rows), rows left-aligned in CSR order; the row pointer gives each
-// row's length, so the padding is never read.  Consecutive threads read
-// consecutive addresses of a slab (coalesced).  A row's sum runs in its
+// row's length.  A warp reads up to its longest row's end, so the padding has to
+// hold index 0 (of any vector gathered) and value 0; it adds -0.  Consecutive threads
+// read consecutive addresses of a slab (coalesced).  A row's sum runs in its
 // column order, sequentially, like the reference's spmv_ell! loop, so every
 // FP32 row reproduces a sequential CPU sum exactly (in the CSR tile engine only
 // rows of at most LONG_ROW nonzeros do); FP64 sums are fused multiply-adds.

@@ -453,7 +453,7 @@ void launch_side4(const ProblemT<T>& P, int side, const CsrView<V, VT>& view, co
 }
 
 // the ELL slabs of a CSR (0-based; narrow storage keeps the signed index):
-// entry k of row r at r + k*rows, padding index 0 and value 0 (never read)
+// entry k of row r at r + k*rows, padding index 0 and value 0 (ell.cuh reads it)
 template <class T>
 __global__ void k_csr_to_ell(const int32_t* __restrict__ ptr, const int32_t* __restrict__ idx,
                              const T* __restrict__ val, int64_t rows, int64_t width,

@@ -151,15 +151,15 @@ typedef struct cpdlp_params {
     /* matrix_type M of Algorithm{A}(T, Ti, M) (src/components/conversion.jl:
      * 37-55, src/problems/modify.jl:80-105): the product format of the
      * single-LP solve's matrices A and A'.  CPDLP_FMT_CSR: the CSR
-     * engines (tiles, or slices of 32 rows; large matrices: the faster by
-     * timing); CPDLP_FMT_ELL: the
+     * engines (tiles, or slices of 32 rows, by the row lengths; FP32 iterates and
+     * at least 2^21 nonzeros: the faster by timing); CPDLP_FMT_ELL: the
      * reference's ELL layout (column-major, width = the longest row), one
      * thread per row, each row summed in column order; CPDLP_FMT_COO: solved
      * on the CSR engine (the reference's COO product accumulates with atomics
      * in a run-dependent order; CSR sums each row in COO's column order);
      * CPDLP_FMT_AUTO (default, EXT): for matrices of at least 2^21 nonzeros
-     * the autotuner times CSR tiles, CSR slices and ELL (when its padding is at
-     * most 3x the nonzeros) and keeps the fastest per matrix, otherwise CSR.
+     * also ELL, when its padding is at most 3x the nonzeros: FP32 iterates, rows of
+     * at most 64 nonzeros, by timing; FP64 by the row lengths.  Otherwise CSR.
      * Batched solves and jobs use the CSR engine. */
     int32_t matrix_type;
 } cpdlp_params;
@@ -335,7 +335,8 @@ int cpdlp_state_solve_blocks(cpdlp_handle* h, cpdlp_state* s, int64_t max_blocks
 
 /* EXT, measurement: mean milliseconds per launch, over `reps` launches timed
  * with CUDA events on the handle's stream, of ms[0] the fused primal step
- * kernel, ms[1] the fused dual step kernel, ms[2] the four-iterate KKT pass.
+ * kernel, ms[1] the fused dual step kernel, ms[2] the four-iterate KKT pass (of
+ * an LP on the resident kernels too, whose blocks run in one launch instead).
  * Outputs go to scratch buffers: the state is unchanged. */
 int cpdlp_state_profile(cpdlp_handle* h, cpdlp_state* s, int32_t reps, double* ms);
 
@@ -457,8 +458,11 @@ int cpdlp_spmv_csr_noalloc(cpdlp_handle* h, int64_t m, int64_t n, int64_t nnz,
  * No counterpart in the reference, which solves one LP per call: this is the
  * batched form of solve(milp, algo) (common.jl:203-209) over `count` LPs.
  * x_out[k] / y_out[k] receive LP k's solution (NULL pointers skip the copy);
- * stats[k] its ConvergenceStats.  All LPs share `params`.  One CTA solves
- * one LP, so an LP's result does not depend on the other LPs of the call.
+ * stats[k] its ConvergenceStats.  All LPs share `params`.  One CTA or
+ * thread-block cluster solves one LP, chosen from the LP alone, so an LP's result
+ * does not depend on the other LPs of the call.  An LP's time limit and
+ * time_elapsed count from its first step: its power method, which is bounded by
+ * its iteration limit, comes before.
  * With float_type CPDLP_VAL_F32, an LP that reaches termination_reltol and
  * targets a smaller refine_reltol, or whose FP32 iterates stall (error not
  * halved over 30 checks), continues in FP64 warm-started from its FP32
