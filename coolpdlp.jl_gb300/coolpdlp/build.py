@@ -38,7 +38,8 @@ def build_library(verbose: bool = False, force: bool = False, extra_flags=None) 
     os.makedirs(BUILD, exist_ok=True)
     os.makedirs(_abi.LIB_DIR, exist_ok=True)
     sources = sorted(glob.glob(os.path.join(CSRC, "*.cu")))
-    headers = glob.glob(os.path.join(CSRC, "*.cuh")) + [_abi.HEADER_PATH]
+    headers = [p for e in ("*.cuh", "*.h") for p in glob.glob(os.path.join(CSRC, e))]
+    headers.append(_abi.HEADER_PATH)
     hdr_time = _newest(headers)
     flags = NVCC_FLAGS + list(extra_flags or []) + os.environ.get("CPDLP_NVCC_EXTRA", "").split()
     exe = nvcc()

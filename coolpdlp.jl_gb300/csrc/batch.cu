@@ -7,7 +7,8 @@
 // cluster (res_plan) is solved there by k_res_pdlp; the others by tile kernels
 // over global memory, with tile partitions that never cross an LP boundary.
 // One CTA or cluster solves one LP at a time and takes the next LP from an
-// atomic counter over a largest-first order when it finishes: power method (linalg.jl:86-96), primal weight (step_size.jl:29-40), then blocks of
+// atomic counter over a largest-first order when it finishes: power method
+// (linalg.jl:86-96), primal weight (step_size.jl:29-40), then blocks of
 // check_every fused PDHG steps (pdlp.jl:96-136) with the four-iterate KKT
 // check, restart and termination logic (pdlp.jl:138-196, restart.jl:40-57,
 // termination.jl:89-101) run by the CTA itself, thread 0 taking the FP64
